@@ -23,7 +23,9 @@ CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA, "bin", "nvcc")
 EXT_SUFFIX = sysconfig.get_config_var("EXT_SUFFIX")
 
-CU_SOURCES = ["abi.cu", "convert.cu", "spmm_tc.cu", "spmm_split.cu", "spmm_mma.cu", "formats.cu",
+CU_SOURCES = ["abi.cu", "convert.cu", "spmm_direct.cu", "spmm_direct_odd.cu",
+              "spmm_direct_bf16x2.cu", "spmm_direct_split24.cu", "spmm_direct_low.cu", "spmm_umma.cu",
+              "spmm_mma.cu", "formats.cu",
               "noalloc.cu", "tune.cu",
               "relabel.cu", "tca.cu", "features.cu", "mlp.cu"]
 GEN_SOURCES = ["gen.cpp"]

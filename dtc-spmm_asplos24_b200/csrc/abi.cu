@@ -2,7 +2,6 @@
 // argument checks, status/error text, per-device state, dispatch.
 #include <mutex>
 #include <string>
-#include <cudaTypedefs.h>
 #include "impl.h"
 
 namespace dtc {
@@ -55,39 +54,6 @@ bool is_sm100() {
   return g_major[d] == 10;
 }
 
-dtc_status encode_c_map(CUtensorMap* map, float* C, int64_t M, int32_t N, int box_rows) {
-  static PFN_cuTensorMapEncodeTiled encode = nullptr;
-  static std::once_flag once;
-  static cudaError_t lookup = cudaSuccess;
-  std::call_once(once, [] {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    lookup = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q);
-    if (lookup == cudaSuccess && q == cudaDriverEntryPointSuccess)
-      encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled>(fn);
-  });
-  if (!encode) {
-    set_error("cuTensorMapEncodeTiled is not available from the driver");
-    return DTC_ERR_UNSUPPORTED;
-  }
-  if (((uintptr_t)C & 15) != 0 || N % 4 != 0 || M < 1 || N < 1) {
-    set_error("C must be 16-byte aligned with N % 4 == 0");
-    return DTC_ERR_INVALID_ARGUMENT;
-  }
-  const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M};
-  const cuuint64_t strides[1] = {(cuuint64_t)N * sizeof(float)};
-  const cuuint32_t box[2] = {32u, (cuuint32_t)box_rows};
-  const cuuint32_t estr[2] = {1u, 1u};
-  CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, C, dims, strides, box, estr,
-                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                      CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_error("cuTensorMapEncodeTiled failed for C (code " + std::to_string((int)r) + ")");
-    return DTC_ERR_CUDA;
-  }
-  return DTC_OK;
-}
-
 uint64_t* cta_timer_buffer(int32_t* capacity) {
   int d = cur_dev();
   std::lock_guard<std::mutex> lk(g_mu);
@@ -95,14 +61,13 @@ uint64_t* cta_timer_buffer(int32_t* capacity) {
   return g_timer[d];
 }
 
-// The chunk-queue region at byte `offset` of a caller workspace of `bytes`
-// bytes, or null when it does not fit (the kernels then run one CTA per chunk).
-void* queue_region(void* ws, size_t bytes, size_t offset, int64_t T, int grid) {
-  if (!ws) return nullptr;
-  const size_t need = spmm_queue_bytes(T, grid);
+float* slot_region(void* ws, size_t bytes, size_t offset, int64_t T, int32_t N, int H, int64_t* n) {
+  *n = 0;
+  if (!ws || T <= 0) return nullptr;
   char* q = (char*)ws + offset;
-  if (((uintptr_t)q & 255) != 0 || offset + need > bytes) return nullptr;
-  return q;
+  if (((uintptr_t)q & 15) != 0 || offset + direct_slots_bytes(T, N, H) > bytes) return nullptr;
+  *n = direct_chunks(T);
+  return (float*)q;
 }
 
 uint32_t* device_error_word() {
@@ -163,15 +128,30 @@ dtc_status dtc_spmm(const int32_t* d_rowWindowOffset, const uint8_t* d_tileId,
                     const float* d_tcValues, int32_t num_nodes, int32_t num_windows,
                     int64_t num_blocks, const float* d_B, int32_t N, float* d_C,
                     dtc_stream_t stream) {
+  return dtc_spmm_ws(d_rowWindowOffset, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues,
+                     num_nodes, num_windows, num_blocks, d_B, N, d_C, nullptr, 0, stream);
+}
+
+dtc_status dtc_spmm_workspace_bytes(int32_t num_nodes, int64_t num_blocks, int32_t N,
+                                    size_t* bytes) {
+  DTC_REQUIRE(bytes != nullptr, "bytes is null");
+  DTC_REQUIRE(num_nodes >= 0 && num_blocks >= 0 && N >= 1, "bad sizes");
+  *bytes = direct_slots_bytes(num_blocks, N, 16);
+  return DTC_OK;
+}
+
+dtc_status dtc_spmm_ws(const int32_t* d_rowWindowOffset, const uint8_t* d_tileId,
+                       const int32_t* d_tcblockOffset, const int32_t* d_sparseAToX,
+                       const float* d_tcValues, int32_t num_nodes, int32_t num_windows,
+                       int64_t num_blocks, const float* d_B, int32_t N, float* d_C,
+                       void* d_workspace, size_t workspace_bytes, dtc_stream_t stream) {
   DTC_REQUIRE(d_rowWindowOffset && d_tcblockOffset && d_B && d_C, "null device pointer");
   DTC_REQUIRE(num_blocks == 0 || (d_tileId && d_sparseAToX), "null device pointer");
-  if (N % 4 != 0)
-    return spmm_mma_sync_impl(d_rowWindowOffset, d_tileId, d_tcblockOffset, d_sparseAToX,
-                              d_tcValues, num_nodes, num_windows, d_B, N, d_C,
-                              (cudaStream_t)stream);
-  return spmm_tf32_impl(d_rowWindowOffset, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues,
-                        num_nodes, num_windows, num_blocks, d_B, N, d_C, 0, 0, nullptr,
-                        (cudaStream_t)stream);
+  int64_t n = 0;
+  float* slots = slot_region(d_workspace, workspace_bytes, 0, num_blocks, N, 16, &n);
+  return spmm_run(d_rowWindowOffset, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues,
+                  num_nodes, num_windows, num_blocks, DTC_B_F32, d_B, nullptr, N, DTC_PREC_TF32,
+                  d_C, (cudaStream_t)stream, Epilogue{}, 16, 8, slots, n);
 }
 
 dtc_status dtc_spmm_balance_workspace_bytes(int32_t num_nodes, int64_t num_blocks, int32_t N,
@@ -179,8 +159,8 @@ dtc_status dtc_spmm_balance_workspace_bytes(int32_t num_nodes, int64_t num_block
   DTC_REQUIRE(bytes != nullptr, "bytes is null");
   DTC_REQUIRE(num_nodes >= 0 && num_blocks >= 0 && N >= 1, "bad sizes");
   int32_t nwin = (num_nodes + 15) / 16;
-  *bytes = align_up((size_t)(nwin + 1) * 4, 256) + align_up(spmm_partials_bytes(num_blocks, N, 0), 256) +
-           spmm_queue_bytes(num_blocks, 0);
+  *bytes = align_up((size_t)(nwin + 1) * 4, 256) +
+           align_up(spmm_partials_bytes(num_blocks, N, 0), 256);
   return DTC_OK;
 }
 
@@ -203,14 +183,11 @@ dtc_status dtc_spmm_balance(const int32_t* d_tcblockRowid, const uint8_t* d_tile
   cudaStream_t st = (cudaStream_t)stream;
   int32_t* rwo = (int32_t*)d_workspace;
   float* part = (float*)((char*)d_workspace + rwo_bytes);
-  void* queue = queue_region(d_workspace, workspace_bytes, rwo_bytes + part_bytes, num_blocks, 0);
   dtc_status s = rowid_to_rwo(d_tcblockRowid, num_blocks, nwin, rwo, st);
   if (s != DTC_OK) return s;
-  if (N % 4 != 0)
-    return spmm_mma_sync_impl(rwo, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues,
-                              num_nodes, nwin, d_B, N, d_C, st);
-  return spmm_tf32_impl(rwo, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues, num_nodes,
-                        nwin, num_blocks, d_B, N, d_C, 1, 0, part, st, 0, Epilogue{}, 16, queue);
+  return spmm_run(rwo, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues, num_nodes, nwin,
+                  num_blocks, DTC_B_F32, d_B, nullptr, N, DTC_PREC_TF32, d_C, st, Epilogue{}, 16, 8,
+                  part, spmm_partials(num_blocks, 0));
 }
 
 dtc_status dtc_spmm_ex_workspace_bytes(int32_t num_nodes, int64_t num_blocks, int32_t N,
@@ -219,7 +196,7 @@ dtc_status dtc_spmm_ex_workspace_bytes(int32_t num_nodes, int64_t num_blocks, in
   DTC_REQUIRE(num_nodes >= 0 && num_blocks >= 0 && N >= 1, "bad sizes");
   DTC_REQUIRE(block_h == 16 || block_h == 32, "block_h must be 16 or 32");
   *bytes = ((mode == 1) ? align_up(spmm_partials_bytes(num_blocks, N, grid, block_h), 256) : 0) +
-           spmm_queue_bytes(num_blocks, grid);
+           direct_slots_bytes(num_blocks, N, block_h);
   return DTC_OK;
 }
 
@@ -238,19 +215,27 @@ dtc_status spmm_ex_impl(const int32_t* rwo, const uint8_t* tile, const int32_t* 
   DTC_REQUIRE(rwo && toff && p0 && C, "null device pointer");
   DTC_REQUIRE(M >= 0 && T >= 0 && N >= 1, "bad sizes");
   DTC_REQUIRE(H == 16 || H == 32, "block_h must be 16 or 32");
-  // required: the partial tiles of balance mode; optional after them: the
-  // chunk queue (persistent CTAs)
+  // required: the partial tiles of balance mode; optional after them: a slot for
+  // every chunk the kernels would like to cut (spmm_run)
   const size_t part_bytes = (mode == 1) ? align_up(spmm_partials_bytes(T, N, grid, H), 256) : 0;
   if (part_bytes > 0 && (!ws || wsb < part_bytes)) {
     set_error("spmm workspace too small (dtc_spmm_ex_workspace_bytes)");
     return DTC_ERR_WORKSPACE_TOO_SMALL;
   }
-  void* queue = queue_region(ws, wsb, part_bytes, T, grid);
+  int64_t n = mode == 1 ? spmm_partials(T, grid) : 0;
+  float* slots = mode == 1 ? (float*)ws : nullptr;
+  if (n < direct_chunks(T)) {  // the second region, where the caller gave it, holds every chunk
+    int64_t more = 0;
+    float* q = slot_region(ws, wsb, part_bytes, T, N, H, &more);
+    if (q) {
+      slots = q;
+      n = more;
+    }
+  }
   if (bformat == DTC_B_F32 && precision == DTC_PREC_TF32)
-    return spmm_tf32_impl(rwo, tile, toff, s2x, vals, M, nwin, T, (const float*)p0, N, C, mode,
-                          grid, (float*)ws, st, ntile, epi, H, queue, W);
-  return spmm_split_impl(rwo, tile, toff, s2x, vals, M, nwin, T, bformat, p0, p1, N, precision,
-                         C, mode, grid, (float*)ws, st, ntile, epi, H, queue, W);
+    DTC_REQUIRE(N % 4 == 0, "fp32 B needs N % 4 == 0 here (16-byte row segments)");
+  return spmm_run(rwo, tile, toff, s2x, vals, M, nwin, T, bformat, p0, p1, N, precision, C, st, epi,
+                  H, W, slots, n);
 }
 
 }  // namespace

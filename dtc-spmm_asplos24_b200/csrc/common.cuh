@@ -1,8 +1,7 @@
 // Shared device/host helpers for the sm_100a kernels: status handling, bounded
-// mbarrier waits, TMA stores and tcgen05 (TMEM / UMMA) wrappers.
+// mbarrier waits and tcgen05 (TMEM / UMMA) wrappers.
 #pragma once
 #include <cuda_runtime.h>
-#include <cuda.h>
 #include <stdint.h>
 #include <string>
 #include "dtc_spmm.h"
@@ -41,10 +40,6 @@ uint32_t* device_error_word();  // device address of the word (per device)
 // when off); *capacity receives its size in CTA records.
 uint64_t* cta_timer_buffer(int32_t* capacity);
 
-// The chunk-queue region at byte `offset` of a caller workspace, or null when it
-// does not fit or is not 256-byte aligned.
-void* queue_region(void* ws, size_t bytes, size_t offset, int64_t T, int grid);
-
 // Aligns a workspace carve-out.
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -76,15 +71,6 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
       : "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile(
-      "{\n\t.reg .b64 st;\n\t"
-      "mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(
-          smem_u32(bar)),
-      "r"(bytes)
-      : "memory");
-}
-
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -97,6 +83,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// try_wait that lets the hardware suspend the thread for up to about `ns`: a warp
+// that waits for long does not take issue slots from the ones it waits for.
+__device__ __forceinline__ bool mbar_try_wait_for(uint64_t* bar, uint32_t parity, uint32_t ns) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(ns)
+      : "memory");
+  return ok != 0;
+}
+
 // Waits for phase `parity` of `bar` to complete. Gives up after `limit_ns`
 // (default 2 s), records kErrWaitTimeout in *err and returns false.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* err,
@@ -104,8 +104,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   if (mbar_try_wait(bar, parity)) return true;
   uint64_t t0 = global_timer_ns();
   while (true) {
-    for (int i = 0; i < 64; ++i)
-      if (mbar_try_wait(bar, parity)) return true;
+    for (int i = 0; i < 16; ++i)
+      if (mbar_try_wait_for(bar, parity, 2000)) return true;
     if (global_timer_ns() - t0 > limit_ns) {
       atomicOr(err, kErrWaitTimeout);
       return false;
@@ -117,43 +117,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
-
-// Bulk (TMA engine) store of `bytes` (multiple of 16, both addresses 16-byte
-// aligned) from shared to global memory, tracked by this thread's bulk group.
-__device__ __forceinline__ void bulk_store_s2g(void* gdst, const void* ssrc, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst),
-               "r"(smem_u32(ssrc)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() {
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-// Waits until at most one (N = 1) / no (N = 0) committed group still reads its
-// shared-memory source.
-template <int N>
-__device__ __forceinline__ void bulk_wait_read() {
-  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
-}
-// TMA 2-D tile store: the box at (x, y) of `map` from shared memory `ssrc`
-// (128-byte aligned), tracked by this thread's bulk group. Parts of the box
-// outside the tensor are not written. x * element size must be a multiple of
-// 16 bytes and x, y must not be negative.
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* ssrc, int32_t x,
-                                             int32_t y) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(ssrc)), "r"(x), "r"(y)
-               : "memory");
-}
-
-// Waits until every committed group has completed (writes performed).
-__device__ __forceinline__ void bulk_wait_all() {
-  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-}
-// Barrier over `count` threads (multiple of 32) on hardware barrier `id` (1-15).
-__device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t count) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
-
 
 // ---- tcgen05 -------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {

@@ -134,23 +134,15 @@ std::vector<torch::Tensor> run_DTCSpMM(torch::Tensor X, torch::Tensor RowWindowO
                             TCblockoffset.data_ptr<int32_t>(), SparseAToX.data_ptr<int32_t>(), vp,
                             (int32_t)num_nodes, nwin, X.data_ptr<float>(), (int32_t)X.size(1),
                             C.data_ptr<float>(), cur_stream()), "dtc_spmm_mma_sync");
-  } else if (X.size(1) % 4 != 0) {
-    check(dtc_spmm(RowWindowOffset.data_ptr<int32_t>(), TCblocktileId.data_ptr<uint8_t>(),
-                   TCblockoffset.data_ptr<int32_t>(), SparseAToX.data_ptr<int32_t>(), vp,
-                   (int32_t)num_nodes, nwin, T, X.data_ptr<float>(), (int32_t)X.size(1),
-                   C.data_ptr<float>(), cur_stream()), "dtc_spmm");
   } else {
-    // the window-scheduled product with the chunk queue in a torch workspace
     const int32_t N = (int32_t)X.size(1);
     size_t wsb = 0;
-    check(dtc_spmm_ex_workspace_bytes((int32_t)num_nodes, T, N, 16, 0, 0, &wsb),
-          "dtc_spmm_ex_workspace_bytes");
-    auto ws = torch::empty({(int64_t)(wsb > 0 ? wsb : 1)}, X.options().dtype(torch::kUInt8));
-    check(dtc_spmm_ex(RowWindowOffset.data_ptr<int32_t>(), TCblocktileId.data_ptr<uint8_t>(),
+    check(dtc_spmm_workspace_bytes((int32_t)num_nodes, T, N, &wsb), "dtc_spmm_workspace_bytes");
+    auto ws = torch::empty({(int64_t)wsb}, X.options().dtype(torch::kUInt8));
+    check(dtc_spmm_ws(RowWindowOffset.data_ptr<int32_t>(), TCblocktileId.data_ptr<uint8_t>(),
                       TCblockoffset.data_ptr<int32_t>(), SparseAToX.data_ptr<int32_t>(), vp,
-                      (int32_t)num_nodes, nwin, T, 16, 8, DTC_B_F32, X.data_ptr<float>(), nullptr,
-                      N, DTC_PREC_TF32, C.data_ptr<float>(), 0, 0, 0, ws.data_ptr(), wsb,
-                      cur_stream()), "dtc_spmm_ex");
+                      (int32_t)num_nodes, nwin, T, X.data_ptr<float>(), N, C.data_ptr<float>(),
+                      ws.data_ptr(), wsb, cur_stream()), "dtc_spmm_ws");
   }
   return {C};
 }

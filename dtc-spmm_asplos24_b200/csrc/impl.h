@@ -12,26 +12,23 @@ struct Epilogue {
   int relu = 0;
 };
 
-dtc_status spmm_tf32_impl(const int32_t* rwo, const uint8_t* tile, const int32_t* toff,
-                          const int32_t* s2x, const float* vals, int32_t M, int32_t nwin,
-                          int64_t T, const float* B, int32_t N, float* C, int mode, int grid,
-                          float* part, cudaStream_t st, int ntile = 0, Epilogue epi = {},
-                          int H = 16, void* queue = nullptr, int W = 8);
-dtc_status spmm_split_impl(const int32_t* rwo, const uint8_t* tile, const int32_t* toff,
-                           const int32_t* s2x, const float* vals, int32_t M, int32_t nwin,
-                           int64_t T, int bformat, const void* p0, const void* p1, int32_t N,
-                           int precision, float* C, int mode, int grid, float* part,
-                           cudaStream_t st, int ntile = 0, Epilogue epi = {}, int H = 16,
-                           void* queue = nullptr, int W = 8);
-// `queue`: the optional chunk-queue region of a workspace (spmm_queue_bytes,
-// 256-byte aligned). With it the kernels run persistent CTAs that pull chunks
-// from a counter; without it, one CTA per chunk.
-// Tensor map of the row-major fp32 matrix C [M x N] with boxes of 32 columns x
-// `box_rows` rows, for TMA stores of finished row-window tiles. Needs C
-// 16-byte aligned and N % 4 == 0.
-dtc_status encode_c_map(CUtensorMap* map, float* C, int64_t M, int32_t N, int box_rows);
+// C = act(A B + bias) on ME-TCF arrays of block shape H x W. `slots`: workspace for
+// the pieces of windows that chunk boundaries cut, H x N floats for each of
+// `nslots` chunks, or null (one CTA then runs such a window's pieces in turn).
+dtc_status spmm_run(const int32_t* rwo, const uint8_t* tile, const int32_t* toff,
+                    const int32_t* s2x, const float* vals, int32_t M, int32_t nwin, int64_t T,
+                    int bformat, const void* b0, const void* b1, int32_t N, int precision, float* C,
+                    cudaStream_t st, Epilogue epi, int H, int W, float* slots, int64_t nslots);
+// Chunks spmm_run cuts T blocks into when `nslots` does not limit them, and the
+// bytes of that many slots.
+int direct_chunks(int64_t T);
+size_t direct_slots_bytes(int64_t T, int32_t N, int H);
+// The slots at byte `offset` of a caller workspace (null when they do not fit).
+float* slot_region(void* ws, size_t bytes, size_t offset, int64_t T, int32_t N, int H, int64_t* n);
+// Tiles of the partials region that strict balance requires for `grid` chunks
+// (0 = 16 per SM), and its bytes.
+int64_t spmm_partials(int64_t T, int grid);
 size_t spmm_partials_bytes(int64_t T, int32_t N, int grid, int H = 16);
-size_t spmm_queue_bytes(int64_t T, int grid);
 dtc_status rowid_to_rwo(const int32_t* rowid, int64_t T, int32_t nwin, int32_t* rwo,
                         cudaStream_t st);
 dtc_status spmm_mma_sync_impl(const int32_t* rwo, const uint8_t* tile, const int32_t* toff,

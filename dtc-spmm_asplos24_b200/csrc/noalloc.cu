@@ -86,9 +86,7 @@ extern "C" dtc_status dtc_spmm_balance_noalloc(const int32_t* d_tcblockRowid,
   float* part = (float*)((char*)base + rwo_bytes);
   s = rowid_to_rwo(d_tcblockRowid, num_blocks, nwin, rwo, st);
   if (s != DTC_OK) return s;
-  if (N % 4 != 0)
-    return spmm_mma_sync_impl(rwo, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues,
-                              num_nodes, nwin, d_B, N, d_C, st);
-  return spmm_tf32_impl(rwo, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues, num_nodes,
-                        nwin, num_blocks, d_B, N, d_C, 1, grid, part, st);
+  return spmm_run(rwo, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues, num_nodes, nwin,
+                  num_blocks, DTC_B_F32, d_B, nullptr, N, DTC_PREC_TF32, d_C, st, Epilogue{}, 16, 8,
+                  part_bytes ? part : nullptr, 2 * (int64_t)grid);
 }

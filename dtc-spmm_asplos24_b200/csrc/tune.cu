@@ -26,7 +26,6 @@ using namespace dtc;
 namespace {
 
 constexpr int kWaveChoices[] = {1, 2, 4, 8, 16, 32, 64};
-constexpr int kMaxWaves = 64;         // chunks of the queue region
 constexpr int kMaxBalanceWaves = 16;  // chunks with partial tiles (balance mode)
 
 // N-tiles per CTA when the caller does not cap them (see the kernels' dispatch).
@@ -86,7 +85,7 @@ dtc_status dtc_autotune_workspace_bytes(int32_t num_nodes, int64_t num_blocks, i
   DTC_REQUIRE(num_nodes >= 0 && num_blocks >= 0 && N >= 1, "bad sizes");
   DTC_REQUIRE(block_h == 16 || block_h == 32, "block_h must be 16 or 32");
   *bytes = align_up(spmm_partials_bytes(num_blocks, N, kMaxBalanceWaves * num_sms(), block_h), 256) +
-           spmm_queue_bytes(num_blocks, kMaxWaves * num_sms());
+           direct_slots_bytes(num_blocks, N, block_h);
   return DTC_OK;
 }
 
@@ -131,11 +130,6 @@ dtc_status dtc_autotune(const int32_t* d_rowWindowOffset, const uint8_t* d_tileI
   DTC_CUDA(cudaEventCreate(&ev.a));
   DTC_CUDA(cudaEventCreate(&ev.b));
   const int sms = num_sms();
-  // the chunk queue sits after the largest candidate's partial tiles
-  void* queue = queue_region(
-      d_workspace, workspace_bytes,
-      align_up(spmm_partials_bytes(num_blocks, N, kMaxBalanceWaves * sms, block_h), 256), num_blocks,
-      kMaxWaves * sms);
   int best_i = -1;
   for (int i = 0; i < ncand; ++i) {
     dtc_schedule& c = cand[i];
@@ -143,16 +137,10 @@ dtc_status dtc_autotune(const int32_t* d_rowWindowOffset, const uint8_t* d_tileI
     if (g > num_blocks) g = num_blocks > 0 ? num_blocks : 1;
     c.grid = (int32_t)g;
     auto run = [&]() {
-      return tf32 ? spmm_tf32_impl(d_rowWindowOffset, d_tileId, d_tcblockOffset, d_sparseAToX,
-                                   d_tcValues, num_nodes, num_windows, num_blocks,
-                                   (const float*)d_Bplane0, N, d_C, c.mode, c.grid,
-                                   (float*)d_workspace, st, c.ntile, Epilogue{}, block_h, queue,
-                                   block_w)
-                  : spmm_split_impl(d_rowWindowOffset, d_tileId, d_tcblockOffset, d_sparseAToX,
-                                    d_tcValues, num_nodes, num_windows, num_blocks, bformat,
-                                    d_Bplane0, d_Bplane1, N, precision, d_C, c.mode, c.grid,
-                                    (float*)d_workspace, st, c.ntile, Epilogue{}, block_h, queue,
-                                    block_w);
+      return dtc_spmm_ex(d_rowWindowOffset, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues,
+                         num_nodes, num_windows, num_blocks, block_h, block_w, bformat, d_Bplane0,
+                         d_Bplane1, N, precision, d_C, c.mode, c.grid, c.ntile, d_workspace,
+                         workspace_bytes, stream);
     };
     s = run();  // warm-up
     if (s != DTC_OK) return s;

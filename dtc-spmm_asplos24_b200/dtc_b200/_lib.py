@@ -31,6 +31,8 @@ SIGNATURES = {
     "dtc_bformat_bytes": [C.c_int, i64, i32, szp, szp],
     "dtc_pack_b": [C.c_int, vp, i64, i32, vp, vp, vp],
     "dtc_spmm": [vp, vp, vp, vp, vp, i32, i32, i64, vp, i32, vp, vp],
+    "dtc_spmm_workspace_bytes": [i32, i64, i32, szp],
+    "dtc_spmm_ws": [vp, vp, vp, vp, vp, i32, i32, i64, vp, i32, vp, vp, sz, vp],
     "dtc_spmm_balance_workspace_bytes": [i32, i64, i32, szp],
     "dtc_spmm_balance": [vp, vp, vp, vp, vp, i32, i64, vp, i32, vp, vp, sz, vp],
     "dtc_spmm_ex": [vp, vp, vp, vp, vp, i32, i32, i64, i32, i32, C.c_int, vp, vp, i32, C.c_int,

@@ -84,13 +84,17 @@ def convert(rowptr, col, M, H=16, W=8, values=None, device="cuda"):
 
 
 def spmm(m: METCF, B: torch.Tensor, use_values=True, out=None):
-    """Window-scheduled SpMM (one launch). A = 1 when the METCF has no values."""
+    """Window-scheduled SpMM. A = 1 when the METCF has no values."""
     B = B.contiguous()
     N = B.shape[1]
     C_ = out if out is not None else torch.empty((m.M, N), dtype=torch.float32, device=B.device)
     vals = m.TCvalues if use_values else None
-    call("dtc_spmm", _ptr(m.RowWindowOffset), _ptr(m.TCblocktileId), _ptr(m.TCblockoffset),
-         _ptr(m.SparseAToX), _ptr(vals), m.M, m.nwin, m.T, _ptr(B), N, _ptr(C_), _stream())
+    wsb = C.c_size_t()
+    call("dtc_spmm_workspace_bytes", m.M, m.T, N, C.byref(wsb))
+    ws = torch.empty(max(wsb.value, 1), dtype=torch.uint8, device=B.device)
+    call("dtc_spmm_ws", _ptr(m.RowWindowOffset), _ptr(m.TCblocktileId), _ptr(m.TCblockoffset),
+         _ptr(m.SparseAToX), _ptr(vals), m.M, m.nwin, m.T, _ptr(B), N, _ptr(C_), _ptr(ws),
+         wsb.value, _stream())
     return C_
 
 
@@ -150,28 +154,28 @@ def pack_b_into(B: torch.Tensor, fmt: int, planes):
 
 def spmm_ex_workspace_bytes(m: METCF, N, mode=0, grid=0):
     """Workspace bytes of spmm_ex for this schedule: the partial tiles of balance
-    mode (required) and the chunk-queue region after them (optional: without it
-    the kernels run one CTA per chunk instead of persistent CTAs)."""
+    mode (required) and a slot per chunk after them (optional: without them fewer
+    CTAs share a row window of many blocks)."""
     wsb = C.c_size_t()
     call("dtc_spmm_ex_workspace_bytes", m.M, m.T, N, m.H, mode, grid, C.byref(wsb))
     return wsb.value
 
 
 def spmm_ex_launches(m: METCF, mode=0, grid=0, queue=True):
-    """Kernels one spmm_ex call launches: the chunk-table kernel (when the
-    workspace holds the chunk queue), the SpMM, and the partial-tile reduction
-    in balance mode when the blocks are cut into more than one chunk."""
+    """Kernels one spmm_ex call launches: the SpMM and, when the workspace has
+    slots (always in balance mode) and the blocks are cut into more than one
+    chunk, the sum of the cut windows' pieces."""
     if m.T == 0:
         return 0
     sms = torch.cuda.get_device_properties(m.RowWindowOffset.device).multi_processor_count
-    G = min(grid if grid > 0 else 16 * sms, m.T)
-    return (1 if queue else 0) + 1 + (1 if (mode == 1 and G > 1) else 0)
+    q = min(max(m.T // (sms * 60), 8), 192)  # blocks per range, 4 ranges per chunk
+    return 1 + (1 if (queue or mode == 1) and m.T // (4 * q) > 1 else 0)
 
 
 def spmm_ex(m: METCF, planes, fmt, N, precision, mode=0, grid=0, use_values=True, out=None,
             workspace=None, ntile=0):
     """SpMM with any B storage form (planes from pack_b), precision and schedule
-    (mode 0 window / 1 balance, grid = chunks, ntile = 128-feature tiles per CTA),
+    (mode 0 window / 1 balance, grid = chunks with partial tiles in the workspace),
     on ME-TCF arrays of window height 16 or 32 and block width 8 (or 16 at height
     16)."""
     dev = planes[0].device

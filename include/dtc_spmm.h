@@ -5,17 +5,16 @@
  * the current device, every call is asynchronous on `stream` unless stated,
  * and every call returns a dtc_status (never exits the process). The library
  * allocates no device memory: callers pass a workspace sized by the matching
- * *_workspace_bytes query. The tcgen05 SpMM entry points read B and write C
- * with 16-byte accesses and TMA stores: d_B / B planes and d_C must be 16-byte
- * aligned and N a multiple of 4 (16 for the split-precision forms); other N
- * go to the legacy-ISA kernel where an entry point says so. They also read
- * d_sparseAToX in 16-byte pieces: it must be 16-byte aligned.
+ * *_workspace_bytes query. The SpMM entry points read B and write C with
+ * 16-byte accesses: d_B / B planes and d_C must be 16-byte aligned and N a
+ * multiple of 4 (16 for the split-precision forms); the entry points that say
+ * so take any N. They also need d_sparseAToX 16-byte aligned.
  *
- * Workspaces of the SpMM entry points hold the partial tiles of strict balance
- * (required) followed by a small chunk-queue region (optional): with it, one
- * CTA per SM pulls chunks of TC blocks from a device counter; with only the
- * required bytes, the kernels run one CTA per chunk. The *_workspace_bytes
- * queries return the size with the queue (workspace base 256-byte aligned).
+ * Workspaces of the SpMM entry points hold pieces of row windows that are cut
+ * between CTAs: the partial tiles of strict balance (required) and, after them,
+ * a slot for every chunk of TC blocks (optional: without it fewer CTAs share a
+ * window of many blocks). The *_workspace_bytes queries return the size with
+ * both (workspace base 256-byte aligned).
  *
  * Each entry point names the reference interface it replaces (paths relative
  * to the reference project root, HPMLL/DTC-SpMM_ASPLOS24).
@@ -214,6 +213,16 @@ dtc_status dtc_spmm(const int32_t* d_rowWindowOffset, const uint8_t* d_tileId,
                     int64_t num_blocks, const float* d_B, int32_t N, float* d_C,
                     dtc_stream_t stream);
 
+/* dtc_spmm with a workspace: a window of more blocks than one CTA's share is
+ * then multiplied by several CTAs (same bits as without). Any N. */
+dtc_status dtc_spmm_workspace_bytes(int32_t num_nodes, int64_t num_blocks, int32_t N,
+                                    size_t* bytes);
+dtc_status dtc_spmm_ws(const int32_t* d_rowWindowOffset, const uint8_t* d_tileId,
+                       const int32_t* d_tcblockOffset, const int32_t* d_sparseAToX,
+                       const float* d_tcValues, int32_t num_nodes, int32_t num_windows,
+                       int64_t num_blocks, const float* d_B, int32_t N, float* d_C,
+                       void* d_workspace, size_t workspace_bytes, dtc_stream_t stream);
+
 /* Strict-balance SpMM. Replaces run_DTCSpMM_balance /
  * spmm_balance_forward_ptx_uint8_prefetch (DTC-SpMM/DTCSpMM.cpp:163-178 ->
  * DTCSpMM_kernel.cu:1118-1199, kernels :4730-4901, :5085-5362). Every CTA gets
@@ -254,13 +263,13 @@ size_t dtc_noalloc_scratch_capacity(void);
  * schedule. block_h x block_w = the ME-TCF's block shape (the conversion's
  * blockSize_h x blockSize_w, DTC-SpMM/DTCSpMM.cpp:315-316): 16 x 8, 32 x 8 or
  * 16 x 16 (the compaction width knob; tile ids must fit a byte).
- * mode 0 = window-scheduled, 1 = strict balance. grid = chunks G of the TC-block
- * range (0 = 16 per SM); the split threshold is ceil(num_blocks / G) blocks.
- * ntile = 128-feature tiles per CTA (0 = all of N up to 4, or up to 2 for the
- * split forms at block_h 32 or block_w 16; 1 or 2 split wider N across more
- * CTAs). d_rowWindowOffset is required (build it from TCblockRowid with
+ * mode 0 = window-scheduled, 1 = strict balance. grid = chunks of the TC-block
+ * range that the required workspace has partial tiles for (0 = 16 per SM); the
+ * kernels cut the range themselves, into fewer chunks than they would like only
+ * where the workspace has fewer slots. ntile is checked and has no effect (the
+ * kernels pick their feature slices). d_rowWindowOffset is required (build it from TCblockRowid with
  * dtc_rowid_to_window_offset). Workspace: required in mode 1 (partial tiles),
- * optional chunk queue after it (see the top of this header). */
+ * optional slots after it (see the top of this header). */
 dtc_status dtc_spmm_ex(const int32_t* d_rowWindowOffset, const uint8_t* d_tileId,
                        const int32_t* d_tcblockOffset, const int32_t* d_sparseAToX,
                        const float* d_tcValues, int32_t num_nodes, int32_t num_windows,
