@@ -1,4 +1,4 @@
-// ME-TCF conversion on the GPU, fully parallel (no per-window serial loops).
+// ME-TCF conversion on the GPU, one pass over the edges per phase.
 //
 // Output semantics follow the reference conversion bit for bit
 // (DTC-SpMM/DTCSpMM_kernel.cu:107-419, DTC-SpMM/DTCSpMM.cpp:313-359):
@@ -8,16 +8,60 @@
 //   TCblocktileId entries of a block are stored in CSR edge order;
 //   SparseAToX[b*W + slot] = column (0 in unused slots).
 // The reference computes U_w and the per-block scatter with one thread per
-// window (:234-240, :309-329); here both steps are radix sorts + scans:
-//   phase 1: sort (window, col) keys -> distinct flags -> scan -> ranks;
-//   phase 2: stable sort of edges by global block id -> offsets, tile ids.
-#include <cub/cub.cuh>
+// window (:234-240, :309-329).
+//
+// A window is the unit here too, but everything that a window needs fits a CTA's shared
+// memory, so each phase reads every edge once or twice and writes it once (a global radix
+// sort moves 16 bytes per edge and pass: five passes for the ranks and three for the
+// blocks, with the passes around them 3.8 ms for R-MAT 2^20, 32 M edges, of which the
+// edges' own bytes are 0.13 ms; here 1.0 ms: ranks 0.42, places 0.51). By window:
+//   ranks, up to 512 edges: one warp sorts packed (column, edge) keys in registers
+//     (bitonic, neighbours by shuffles) and reads the ranks off the order; up to 2048 (half
+//     of both where column and edge need more than 32 bits): the same by 128 threads
+//   ranks, larger: 1024 threads mark the columns in a bitmap (2^20 columns per sweep over
+//     the window) and count the bits before each (a whole CTA per SM, the longest first)
+//   places, up to 1024 edges: one warp marks the cells of every block and counts the marks
+//     before each; larger: a warp per 128 blocks does so, which finds its part of each row
+//     by binary search
+//   places where some row's ranks do not ascend (unsorted or repeated columns), and
+//     windows of more than 32 rows: 128 threads sort by block, or beyond 1024 edges 1024
+//     threads advance a counter per block row by row
+// The lines lie where shared memory ends: a sort of 2048 keys beats clearing and counting a
+// bitmap of 2^20 columns (5 us) up to there.
+// Bound: instruction issue and the latency of dependent loads; DRAM is at a fifth.
+#include <algorithm>
 #include "common.cuh"
 
 namespace dtc {
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kGroup = 128;              // threads of a CTA: four windows, or one middle window
+constexpr int kWarpFill = 1024;          // windows up to here: places by one warp
+constexpr int kThreads = 1024;           // threads of a large window
+constexpr int kSweepCols = 1 << 20;      // columns per sweep of a large window's bitmap
+constexpr int kSweepBlocks = 1 << 14;    // blocks per sweep of a large window's counters
+constexpr int kMaxH = 256;               // rows of a window (block_h * block_w <= 256)
+constexpr int kUnitH = 32;               // rows up to which a warp takes part of a window
+
+template <typename K>
+struct Cap {
+  static constexpr int kEdges = sizeof(K) == 4 ? 2048 : 1024;
+  static constexpr int kBits = sizeof(K) == 4 ? 11 : 10;
+  static constexpr int kWarp = sizeof(K) == 4 ? 512 : 256;  // ranks by one warp (registers)
+};
+// Bytes of a group: keys, 16-bit ranks and row starts of a middle window, or four
+// warps' scratch.
+constexpr int kCells = 4160;  // bytes of a warp's cell masks (130 blocks of 256 cells)
+constexpr int kWarpBytes = kCells * 3 / 2 + (2 * kUnitH + 1) * 4 + 12;  // masks, places, rows
+template <typename K>
+constexpr int group_bytes() {
+  return std::max(Cap<K>::kEdges * ((int)sizeof(K) + 2) + (kMaxH + 1) * 4 + 60, 4 * kWarpBytes);
+}
+static_assert(Cap<uint32_t>::kWarp * 2 + (kMaxH + 1) * 4 <= kWarpBytes && kWarpBytes % 16 == 0 &&
+              kCells >= (kWarpFill / 8 + 1) * 32, "warp scratch");
+constexpr int kPer = 16;      // windows per CTA at most, by one warp each
+constexpr int kLargeBytes =
+    kSweepCols / 8 + kSweepCols / 64 * 2 + kSweepCols / 32768 * 4 + (kMaxH + 1) * 4 + 256;
 
 inline int bits_for(uint64_t n) {  // bits to represent values in [0, n)
   int b = 0;
@@ -25,256 +69,1140 @@ inline int bits_for(uint64_t n) {  // bits to represent values in [0, n)
   return b < 1 ? 1 : b;
 }
 
-inline unsigned grid_for(int64_t n, int per = kThreads) {
-  int64_t g = (n + per - 1) / per;
-  if (g < 1) g = 1;
-  if (g > (1 << 30)) g = 1 << 30;
-  return (unsigned)g;
-}
-
-// Validates CSR structure: rowptr[0] == 0, rowptr non-decreasing,
-// rowptr[M] == nnz, 0 <= col < num_cols. Sets bits in *bad.
-__global__ void k_validate(const int32_t* __restrict__ col, const int32_t* __restrict__ rowptr,
-                           int32_t M, int64_t nnz, int32_t num_cols, uint32_t* bad) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r = i; r <= M; r += stride) {
-    int32_t v = rowptr[r];
-    if (r == 0 && v != 0) atomicOr(bad, 1u);
-    if (r == M && v != nnz) atomicOr(bad, 2u);
-    if (r < M && rowptr[r + 1] < v) atomicOr(bad, 4u);
+struct Csr {
+  const int32_t* col;
+  const int32_t* rowptr;
+  int32_t M, nwin, H, W;
+  int64_t nnz;
+  int32_t shift;  // log2 W, or -1
+  __device__ __forceinline__ int32_t block(int32_t rank) const {
+    return shift >= 0 ? rank >> shift : rank / W;
   }
-  for (int64_t e = i; e < nnz; e += stride) {
-    int32_t c = col[e];
-    if (c < 0 || c >= num_cols) atomicOr(bad, 8u);
+  __device__ __forceinline__ int32_t slot(int32_t rank) const {
+    return shift >= 0 ? rank & (W - 1) : rank % W;
   }
+};
+
+__device__ __forceinline__ void window_edges(const Csr& a, int32_t w, int32_t& e0, int32_t& n) {
+  const int64_t r0 = (int64_t)w * a.H, r1 = min(r0 + a.H, (int64_t)a.M);
+  e0 = __ldg(a.rowptr + r0);
+  const int32_t e1 = __ldg(a.rowptr + r1);
+  n = e1 - e0;
+  if (e0 < 0 || e1 > a.nnz || n < 0) n = 0;  // invalid CSR: reported by k_list
 }
 
-// edgeToRow[e] = row (DTCSpMM_kernel.cu:107-120): one warp per row.
-__global__ void k_edge_to_row(const int32_t* __restrict__ rowptr, int32_t M,
-                              int32_t* __restrict__ edgeToRow) {
-  int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t r = warp; r < M; r += nwarps) {
-    int32_t e1 = rowptr[r + 1];
-    for (int32_t e = rowptr[r] + lane; e < e1; e += 32) edgeToRow[e] = (int32_t)r;
-  }
+// The i-th of the listed windows, those of more than kHuge edges first.
+constexpr int kHuge = 16384;
+__device__ __forceinline__ int32_t listed(const int32_t* count, const int32_t* list, int32_t room,
+                                          int32_t i) {
+  const int32_t huge = __ldg(count);
+  return __ldg(list + (i < huge ? i : room - 1 - (i - huge)));
+}
+__device__ __forceinline__ int32_t many_listed(const int32_t* count, int32_t room) {
+  return (int32_t)min((int64_t)__ldg(count) + __ldg(count + 1), (int64_t)room);
 }
 
-// Sort keys (window << colbits | col) and edge ids.
-template <typename K>
-__global__ void k_make_keys(const int32_t* __restrict__ col, const int32_t* __restrict__ edgeToRow,
-                            int64_t nnz, int32_t H, int colbits, K* __restrict__ keys,
-                            int32_t* __restrict__ ids) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnz; e += stride) {
-    K w = (K)(edgeToRow[e] / H);
-    keys[e] = (w << colbits) | (K)(uint32_t)col[e];
-    ids[e] = (int32_t)e;
-  }
-}
-
-// flags[i] = 1 where sorted key i starts a new (window, col) pair; flags[nnz] = 0.
-template <typename K>
-__global__ void k_distinct_flags(const K* __restrict__ keys, int64_t nnz, int32_t* __restrict__ flags) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= nnz; i += stride)
-    flags[i] = (i < nnz && (i == 0 || keys[i] != keys[i - 1])) ? 1 : 0;
-}
-
-// edgeToColumn[e] = rank of col(e) among the window's distinct columns:
-// P = exclusive scan of flags (P[nnz] = #distinct pairs); the window's sorted
-// range equals its CSR edge range, so rank(i) = P[i+1] - 1 - P[rowptr[w*H]].
-template <typename K>
-__global__ void k_ranks(const K* __restrict__ keys, const int32_t* __restrict__ ids,
-                        const int32_t* __restrict__ P, const int32_t* __restrict__ rowptr, int64_t nnz,
-                        int32_t H, int colbits, int32_t* __restrict__ edgeToColumn) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nnz; i += stride) {
-    int32_t w = (int32_t)(keys[i] >> colbits);
-    int32_t s = rowptr[(int64_t)w * H];
-    edgeToColumn[ids[i]] = P[i + 1] - 1 - P[s];
-  }
-}
-
-// blockPartition[w] = ceil(U_w / W) (0 for empty windows, :215-227).
-__global__ void k_block_partition(const int32_t* __restrict__ P, const int32_t* __restrict__ rowptr,
-                                  int32_t M, int32_t nwin, int32_t H, int32_t W,
-                                  int32_t* __restrict__ blockPartition, int32_t* __restrict__ bp_ext) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w <= nwin; w += stride) {
-    if (w == nwin) { bp_ext[w] = 0; continue; }
-    int64_t r1 = w * H + H;
-    if (r1 > M) r1 = M;
-    int32_t u = P[rowptr[r1]] - P[rowptr[w * H]];
-    int32_t nb = (u + W - 1) / W;
-    blockPartition[w] = nb;
-    bp_ext[w] = nb;
-  }
-}
-
-// TCblockRowid[b] = w (:149-173); one warp per window.
-__global__ void k_block_rowid(const int32_t* __restrict__ rwo, int32_t nwin,
-                              int32_t* __restrict__ rowid) {
-  int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t w = warp; w < nwin; w += nwarps) {
-    int32_t b1 = rwo[w + 1];
-    for (int32_t b = rwo[w] + lane; b < b1; b += 32) rowid[b] = (int32_t)w;
-  }
-}
-
-// Global block id of each edge (CSR order) for the stable sort.
-__global__ void k_edge_block(const int32_t* __restrict__ edgeToColumn,
-                             const int32_t* __restrict__ edgeToRow, const int32_t* __restrict__ rwo,
-                             int64_t nnz, int32_t H, int32_t W, uint32_t* __restrict__ blk,
-                             int32_t* __restrict__ ids) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnz; e += stride) {
-    blk[e] = (uint32_t)(rwo[edgeToRow[e] / H] + edgeToColumn[e] / W);
-    ids[e] = (int32_t)e;
-  }
-}
-
-// Per sorted position j (edges grouped by block, CSR order inside a block):
-// block offsets, tile ids (:287-300) and SparseAToX (:296).
-__global__ void k_scatter_tiles(const uint32_t* __restrict__ blk_sorted,
-                                const int32_t* __restrict__ ids_sorted,
-                                const int32_t* __restrict__ col, const int32_t* __restrict__ edgeToColumn,
-                                const int32_t* __restrict__ edgeToRow, int64_t nnz, int64_t T,
-                                int32_t H, int32_t W, int32_t* __restrict__ tcblockOffset,
-                                uint8_t* __restrict__ tileId, int32_t* __restrict__ sparseAToX) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nnz; j += stride) {
-    int32_t b = (int32_t)blk_sorted[j];
-    if (j == 0 || (int32_t)blk_sorted[j - 1] != b) {
-      // every TC block holds at least one edge, so offsets are run starts
-      int32_t prev = (j == 0) ? -1 : (int32_t)blk_sorted[j - 1];
-      for (int32_t q = prev + 1; q <= b; ++q) tcblockOffset[q] = (int32_t)j;
+// Lists the windows of more than mid_cap edges (mid_list) and of more than `cap`, those of more than kHuge from the front and
+// the others from the back (count[0], count[1]); with `bad`, checks the row pointer
+// (rowptr[0] == 0, non-decreasing, rowptr[M] == nnz) and sets its bits. With `rwo`
+// (phase 2), also lists their units of `unit` blocks: (window, first block).
+__global__ void k_list(const Csr a, int32_t cap, int32_t mid_cap, int32_t* count, int32_t* list,
+                       int32_t* mid_count, int32_t* mid_list, int32_t mid_room, uint32_t* bad,
+                       int32_t room, const int32_t* rwo, int32_t unit, int32_t* units,
+                       int2* unit_list, int64_t unit_room) {
+  const int32_t w = blockIdx.x * blockDim.x + threadIdx.x;
+  if (w < a.nwin) {
+    int32_t e0, n;
+    window_edges(a, w, e0, n);
+    if (n > cap) {
+      const int32_t at = n > kHuge ? atomicAdd(count, 1) : room - 1 - atomicAdd(count + 1, 1);
+      const bool in = at >= 0 && at < room;  // (a valid CSR cannot have more)
+      if (in) list[at] = w;
+      if (in && rwo) {
+        const int32_t nb = rwo[w + 1] - rwo[w], many = unit ? (nb + unit - 1) / unit : 0;
+        const int32_t u = atomicAdd(units, many);
+        for (int32_t i = 0; i < many && u + i < unit_room; ++i)
+          unit_list[u + i] = make_int2(w, i * unit);
+      }
+    } else if (n > mid_cap) {
+      const int32_t at = atomicAdd(mid_count, 1);
+      if (at < mid_room) mid_list[at] = w;
     }
-    if (j == nnz - 1) tcblockOffset[T] = (int32_t)nnz;
-    int32_t e = ids_sorted[j];
-    int32_t rk = edgeToColumn[e];
-    int32_t slot = rk % W;
-    tileId[j] = (uint8_t)((edgeToRow[e] % H) * W + slot);
-    sparseAToX[(int64_t)b * W + slot] = col[e];  // duplicates write the same value
+  }
+  if (bad) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t r = w; r <= a.M; r += stride) {
+      const int32_t v = a.rowptr[r];
+      if (r == 0 && v != 0) atomicOr(bad, 1u);
+      if (r == a.M && v != a.nnz) atomicOr(bad, 2u);
+      if (r < a.M && a.rowptr[r + 1] < v) atomicOr(bad, 4u);
+    }
   }
 }
 
-// Values in tile order; duplicate (row, col) of a block merged into the
-// first occurrence in CSR order (fp32 sum in CSR order), later ones 0.
-__global__ void k_tile_values(const int32_t* __restrict__ tcblockOffset,
-                              const uint8_t* __restrict__ tileId, const int32_t* __restrict__ ids_sorted,
-                              const float* __restrict__ values, int64_t T,
-                              float* __restrict__ tcValues) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < T; b += stride) {
-    uint32_t seen[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    int32_t j0 = tcblockOffset[b], j1 = tcblockOffset[b + 1];
-    for (int32_t j = j0; j < j1; ++j) {
-      uint32_t p = tileId[j];
-      float v = values[ids_sorted[j]];
-      uint32_t bit = 1u << (p & 31);
-      if (!(seen[p >> 5] & bit)) {
-        seen[p >> 5] |= bit;
-        tcValues[j] = v;
+// mixed[w] = 1 for each window of more than kWarpFill edges where the ranks of some row do
+// not ascend (unsorted or repeated columns), and *any: one pass over the edges, eight per thread.
+__global__ void k_mixed(const Csr a, const int32_t* __restrict__ e2c,
+                        const int32_t* __restrict__ e2r, uint8_t* mixed, int32_t* any) {
+  const int64_t e0 = (int64_t)blockIdx.x * blockDim.x * 8 + threadIdx.x;
+  int32_t c[8], d[8], r[8], q[8];
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    const int64_t e = e0 + v * blockDim.x;
+    const bool in = e > 0 && e < a.nnz;
+    c[v] = in ? __ldg(e2c + e - 1) : 0;
+    d[v] = in ? __ldg(e2c + e) : 1;
+    r[v] = in ? __ldg(e2r + e - 1) : 0;
+    q[v] = in ? __ldg(e2r + e) : 1;
+  }
+#pragma unroll
+  for (int v = 0; v < 8; ++v)
+    if (c[v] >= d[v] && r[v] == q[v]) {
+      mixed[q[v] / a.H] = 1;
+      *any = 1;
+    }
+}
+
+// ------------------------------------------------------------- group helpers
+// The last row r of `rows` whose start is at or before local edge i.
+__device__ __forceinline__ int row_of(const int32_t* start, int rows, int32_t i) {
+  int lo = 0, hi = rows;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (start[mid] <= i) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+// Ascending bitonic sort of key[0, n2), n2 a power of two, by one group. Pairs
+// less than 64 apart stay inside a warp's 64 keys and need no group barrier.
+template <typename K>
+__device__ __forceinline__ void bitonic(K* key, int n2, int t) {
+  for (int k = 2; k <= n2; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int i = t; i < n2 / 2; i += kGroup) {
+        const int lo = 2 * i - (i & (j - 1)), hi = lo + j;
+        const K x = key[lo], y = key[hi];
+        if ((x > y) == ((lo & k) == 0)) {
+          key[lo] = y;
+          key[hi] = x;
+        }
+      }
+      if (j > 32 || (j == 1 && k >= 64)) __syncthreads(); else __syncwarp();
+    }
+  __syncthreads();
+}
+
+// Exclusive sum of x over the group's threads (s: kGroup / 32 words); *total = sum.
+__device__ __forceinline__ int group_scan(int x, int t, int32_t* s, int* total) {
+  int v = x;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if ((t & 31) >= o) v += u;
+  }
+  if ((t & 31) == 31) s[t >> 5] = v;
+  __syncthreads();
+  int before = 0, sum = 0;
+#pragma unroll
+  for (int i = 0; i < kGroup / 32; ++i) {
+    if (i < (t >> 5)) before += s[i];
+    sum += s[i];
+  }
+  *total = sum;
+  __syncthreads();
+  return before + v - x;
+}
+
+// The same over the whole CTA (s: kThreads / 32 words).
+__device__ __forceinline__ int cta_scan(int x, int32_t* s, int* total) {
+  const int t = threadIdx.x;
+  int v = x;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if ((t & 31) >= o) v += u;
+  }
+  if ((t & 31) == 31) s[t >> 5] = v;
+  __syncthreads();
+  int before = 0, sum = 0;
+#pragma unroll
+  for (int i = 0; i < kThreads / 32; ++i) {
+    if (i < (t >> 5)) before += s[i];
+    sum += s[i];
+  }
+  *total = sum;
+  __syncthreads();
+  return before + v - x;
+}
+
+// Ascending bitonic sort of 32 E keys per warp over T threads (a warp, or the CTA):
+// thread t holds elements t E .. t E + E - 1. Distances below E are between a thread's
+// own registers, below 32 E between lanes, the others through `buf` (T E keys).
+template <typename K, int E, int T>
+__device__ __forceinline__ void reg_bitonic(K (&x)[E], int t, K* buf) {
+#pragma unroll
+  for (int k = 2; k < E; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int i = 0; i < E; ++i)
+        if ((i & j) == 0) {
+          const K lo = min(x[i], x[i | j]), hi = max(x[i], x[i | j]);
+          x[i] = (i & k) == 0 ? lo : hi;
+          x[i | j] = (i & k) == 0 ? hi : lo;
+        }
+  // (loops from here on: unrolled, the steps of all sizes are beyond the instruction
+  // cache, and the kernel took four times as long)
+#pragma unroll 1
+  for (int k = E; k <= T * E; k <<= 1) {
+    const bool up = ((t * E) & k) == 0;  // the run of k ascends
+#pragma unroll 1
+    for (int d = k / E / 2; d > 0; d >>= 1) {
+      const bool keep_min = up == ((t & d) == 0);
+      if (T > 32 && d >= 32) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < E; ++i) buf[i * T + t] = x[i];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+          const K y = buf[i * T + (t ^ d)];
+          x[i] = (x[i] < y) == keep_min ? x[i] : y;
+        }
       } else {
-        int32_t f = j0;
-        while (tileId[f] != p) ++f;
-        tcValues[f] += v;
-        tcValues[j] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+          const K y = __shfl_xor_sync(0xffffffffu, x[i], d);
+          x[i] = (x[i] < y) == keep_min ? x[i] : y;
+        }
       }
     }
+#pragma unroll
+    for (int j = E / 2; j > 0; j >>= 1)
+#pragma unroll
+      for (int i = 0; i < E; ++i)
+        if ((i & j) == 0) {
+          const K p = x[i], q = x[i | j];
+          const bool swap = (q < p) == up;  // (equal keys: none, or two paddings)
+          x[i] = swap ? q : p;
+          x[i | j] = swap ? p : q;
+        }
   }
 }
 
-struct Phase1Layout {
-  size_t keys_in, keys_out, ids_in, ids_out, flags, P, bp_ext, bad, cub_sort, cub_scan, total;
-  bool wide;
-  int colbits, endbit;
-};
-
-struct Phase2Layout {
-  size_t blk_in, blk_out, ids_in, ids_out, cub_sort, total;
-  int endbit;
-};
-
-Phase1Layout phase1_layout(int32_t M, int64_t nnz, int32_t H) {
-  Phase1Layout L{};
-  int32_t nwin = (M + H - 1) / H;
-  L.colbits = bits_for((uint64_t)(M > 0 ? M : 1));
-  int winbits = bits_for((uint64_t)(nwin > 0 ? nwin : 1));
-  L.endbit = L.colbits + winbits;
-  L.wide = L.endbit > 32;
-  size_t ks = L.wide ? 8 : 4;
-  size_t n = (size_t)(nnz > 0 ? nnz : 1);
-  size_t off = 0;
-  auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
-  L.keys_in = take(n * ks);
-  L.keys_out = take(n * ks);
-  L.ids_in = take(n * 4);
-  L.ids_out = take(n * 4);
-  L.flags = take((n + 1) * 4);
-  L.P = take((n + 1) * 4);
-  L.bp_ext = take((size_t)(nwin + 1) * 4);
-  L.bad = take(16);
-  size_t s1 = 0, s2 = 0, s3 = 0;
-  if (L.wide) {
-    cub::DeviceRadixSort::SortPairs(nullptr, s1, (uint64_t*)nullptr, (uint64_t*)nullptr,
-                                    (int32_t*)nullptr, (int32_t*)nullptr, (int64_t)n, 0, L.endbit);
-  } else {
-    cub::DeviceRadixSort::SortPairs(nullptr, s1, (uint32_t*)nullptr, (uint32_t*)nullptr,
-                                    (int32_t*)nullptr, (int32_t*)nullptr, (int64_t)n, 0, L.endbit);
+// ------------------------------------------------------------------- phase 1
+template <typename K, int E>
+__device__ __forceinline__ void count_warp(const Csr& a, int32_t w, int32_t e0, int32_t n,
+                                           uint8_t* sm, int lane, int32_t* e2c, int32_t* e2r,
+                                           int32_t* bp, uint32_t* bad) {
+  constexpr int B = 9;  // bits of an edge's place
+  uint16_t* rank = reinterpret_cast<uint16_t*>(sm);
+  int32_t* start = reinterpret_cast<int32_t*>(sm + Cap<K>::kWarp * 2);
+  const int64_t r0 = (int64_t)w * a.H;
+  const int rows = (int)min((int64_t)a.H, a.M - r0);
+  for (int r = lane; r < rows; r += 32) start[r] = __ldg(a.rowptr + r0 + r) - e0;
+  K x[E];
+#pragma unroll
+  for (int i = 0; i < E; ++i) {  // (any order will do: loaded coalesced)
+    const int e = i * 32 + lane;
+    x[i] = (K)~(K)0;
+    if (e < n) {
+      int32_t c = __ldg(a.col + e0 + e);
+      if (c < 0 || c >= a.M) {
+        atomicOr(bad, 8u);
+        c = 0;
+      }
+      x[i] = ((K)(uint32_t)c << B) | (K)e;
+    }
   }
-  cub::DeviceScan::ExclusiveSum(nullptr, s2, (int32_t*)nullptr, (int32_t*)nullptr, (int64_t)n + 1);
-  cub::DeviceScan::ExclusiveSum(nullptr, s3, (int32_t*)nullptr, (int32_t*)nullptr,
-                                (int64_t)nwin + 1);
-  L.cub_sort = take(s1);
-  L.cub_scan = take(s2 > s3 ? s2 : s3);
-  L.total = off;
-  return L;
+  reg_bitonic<K, E, 32>(x, lane, nullptr);
+  const K before = __shfl_up_sync(0xffffffffu, x[E - 1], 1);
+  int mine = 0;
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    const bool first = i == 0 && lane == 0;
+    mine += lane * E + i < n && (first || (x[i] >> B) != ((i ? x[i ? i - 1 : 0] : before) >> B));
+  }
+  int s = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, s, o);
+    if (lane >= o) s += u;
+  }
+  int r = s - mine - 1;
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    const bool first = i == 0 && lane == 0;
+    if (lane * E + i < n) {
+      r += first || (x[i] >> B) != ((i ? x[i ? i - 1 : 0] : before) >> B);
+      rank[(int)(x[i] & (K)((1 << B) - 1))] = (uint16_t)r;
+    }
+  }
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) {
+    e2c[e0 + i] = rank[i];
+    e2r[e0 + i] = (int32_t)(r0 + row_of(start, rows, i));
+  }
+  if (lane == 31) bp[w] = (s + a.W - 1) / a.W;
+  __syncwarp();
 }
 
-Phase2Layout phase2_layout(int64_t nnz, int64_t T_upper) {
-  Phase2Layout L{};
-  size_t n = (size_t)(nnz > 0 ? nnz : 1);
-  L.endbit = bits_for((uint64_t)(T_upper > 0 ? T_upper : 1));
-  size_t off = 0;
-  auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
-  L.blk_in = take(n * 4);
-  L.blk_out = take(n * 4);
-  L.ids_in = take(n * 4);
-  L.ids_out = take(n * 4);
-  size_t s1 = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, s1, (uint32_t*)nullptr, (uint32_t*)nullptr,
-                                  (int32_t*)nullptr, (int32_t*)nullptr, (int64_t)n, 0, L.endbit);
-  L.cub_sort = take(s1);
-  L.total = off;
-  return L;
+template <typename K, int E>
+__device__ __forceinline__ void count_small(const Csr& a, int32_t w, int32_t e0, int32_t n,
+                                            uint8_t* sm, int t, int32_t* e2c, int32_t* e2r,
+                                            int32_t* bp, uint32_t* bad) {
+  constexpr int B = Cap<K>::kBits;
+  static_assert(E * kGroup <= Cap<K>::kEdges, "keys fit");
+  K* key = reinterpret_cast<K*>(sm);
+  uint16_t* rank = reinterpret_cast<uint16_t*>(key + Cap<K>::kEdges);
+  int32_t* start = reinterpret_cast<int32_t*>(rank + Cap<K>::kEdges);
+  int32_t* part = start + kMaxH + 1;
+  const int64_t r0 = (int64_t)w * a.H;
+  const int rows = (int)min((int64_t)a.H, a.M - r0);
+  for (int r = t; r < rows; r += kGroup) start[r] = __ldg(a.rowptr + r0 + r) - e0;
+  K x[E];
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    const int e = i * kGroup + t;
+    x[i] = (K)~(K)0;
+    if (e < n) {
+      int32_t c = __ldg(a.col + e0 + e);
+      if (c < 0 || c >= a.M) {
+        atomicOr(bad, 8u);
+        c = 0;
+      }
+      x[i] = ((K)(uint32_t)c << B) | (K)e;
+    }
+  }
+  reg_bitonic<K, E, kGroup>(x, t, key);
+  __syncthreads();
+  key[t] = x[E - 1];  // the last key of each thread, for the next one
+  __syncthreads();
+  const K before = t ? key[t - 1] : 0;
+  int mine = 0;
+#pragma unroll
+  for (int i = 0; i < E; ++i)
+    mine += t * E + i < n &&
+            ((i == 0 && t == 0) || (x[i] >> B) != ((i ? x[i ? i - 1 : 0] : before) >> B));
+  int total;
+  int r = group_scan(mine, t, part, &total) - 1;
+#pragma unroll
+  for (int i = 0; i < E; ++i)
+    if (t * E + i < n) {
+      r += (i == 0 && t == 0) || (x[i] >> B) != ((i ? x[i ? i - 1 : 0] : before) >> B);
+      rank[(int)(x[i] & (K)((1 << B) - 1))] = (uint16_t)r;
+    }
+  __syncthreads();
+  for (int i = t; i < n; i += kGroup) {
+    e2c[e0 + i] = rank[i];
+    e2r[e0 + i] = (int32_t)(r0 + row_of(start, rows, i));
+  }
+  if (t == 0) bp[w] = (total + a.W - 1) / a.W;
+  __syncthreads();
+}
+
+__device__ void count_large(const Csr& a, int32_t w, int32_t e0, int32_t n, uint8_t* sm,
+                            int32_t* e2c, int32_t* e2r, int32_t* bp, uint32_t* bad) {
+  uint32_t* bm = reinterpret_cast<uint32_t*>(sm);                     // kSweepCols bits
+  uint16_t* pre = reinterpret_cast<uint16_t*>(bm + kSweepCols / 32);  // set bits before 64 columns,
+  int32_t* sup = reinterpret_cast<int32_t*>(pre + kSweepCols / 64);   // counted from 2^15 columns
+  int32_t* start = sup + kSweepCols / 32768;
+  int32_t* part = start + kMaxH + 1;
+  const int t = threadIdx.x;
+  const int64_t r0 = (int64_t)w * a.H;
+  const int rows = (int)min((int64_t)a.H, a.M - r0);
+  for (int r = t; r < rows; r += kThreads) start[r] = __ldg(a.rowptr + r0 + r) - e0;
+  int32_t distinct = 0;
+  for (int64_t c0 = 0; c0 < a.M; c0 += kSweepCols) {
+    const int32_t cols = (int32_t)min((int64_t)kSweepCols, a.M - c0);
+    const int words = (cols + 1023) / 1024 * 32;
+    for (int i = t; i < words / 4; i += kThreads)
+      reinterpret_cast<uint4*>(bm)[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    for (int32_t i = t; i < n; i += 8 * kThreads) {  // eight loads under way per thread
+      int32_t c[8];
+#pragma unroll
+      for (int v = 0; v < 8; ++v)
+        c[v] = i + v * kThreads < n ? __ldg(a.col + e0 + i + v * kThreads) : -1;
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        if (i + v * kThreads >= n) break;
+        if (c0 == 0 && (c[v] < 0 || c[v] >= a.M)) {
+          atomicOr(bad, 8u);
+          c[v] = 0;
+        }
+        const uint32_t x = (uint32_t)(c[v] - (int32_t)c0);
+        if (x < (uint32_t)cols) atomicOr(bm + (x >> 5), 1u << (x & 31));
+      }
+    }
+    __syncthreads();
+    // (neighbouring threads take neighbouring words: with a run of words per thread every
+    // load was a 32-way bank conflict, 35 us per window)
+    const int pairs = words / 2;
+    for (int q = t; q < pairs; q += kThreads)
+      pre[q] = (uint16_t)__popcll(reinterpret_cast<const unsigned long long*>(bm)[q]);
+    __syncthreads();
+    constexpr int V = kSweepCols / 64 / kThreads;  // counts per thread
+    static_assert(V == 16 && kThreads / 32 == kSweepCols / 32768, "a warp per 2^15 columns");
+    uint4 g[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+    if (t * V < pairs) {
+      g[0] = reinterpret_cast<const uint4*>(pre)[2 * t];
+      g[1] = reinterpret_cast<const uint4*>(pre)[2 * t + 1];
+    }
+    uint32_t* const u = reinterpret_cast<uint32_t*>(g);
+    int mine = 0;
+#pragma unroll
+    for (int v = 0; v < V / 2; ++v) mine += (u[v] & 0xffffu) + (u[v] >> 16);
+    int total;
+    int before = cta_scan(mine, part, &total);
+    const int first = __shfl_sync(0xffffffffu, before, 0);  // set bits before the warp's columns
+    if ((t & 31) == 0) sup[t >> 5] = distinct + first;
+    before -= first;  // (at most 2^15)
+#pragma unroll
+    for (int v = 0; v < V / 2; ++v) {
+      const uint32_t lo = u[v] & 0xffffu, hi = u[v] >> 16;
+      u[v] = (uint32_t)before | (uint32_t)(before + lo) << 16;
+      before += lo + hi;
+    }
+    if (t * V < pairs) {
+      reinterpret_cast<uint4*>(pre)[2 * t] = g[0];
+      reinterpret_cast<uint4*>(pre)[2 * t + 1] = g[1];
+    }
+    __syncthreads();
+    int row = 0;  // of the thread's edge: it only moves on
+    for (int32_t i = t; i < n; i += 8 * kThreads) {
+      int32_t c[8];
+#pragma unroll
+      for (int v = 0; v < 8; ++v)
+        c[v] = i + v * kThreads < n ? __ldg(a.col + e0 + i + v * kThreads) : -1;
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        const int32_t e = i + v * kThreads;
+        if (e >= n) break;
+        const uint32_t x = (uint32_t)(c[v] - (int32_t)c0);
+        if (x < (uint32_t)cols)
+          e2c[e0 + e] = sup[x >> 15] + pre[x >> 6] +
+                        __popcll(reinterpret_cast<const unsigned long long*>(bm)[x >> 6] &
+                                 ((1ull << (x & 63)) - 1));
+        if (c0 == 0) {
+          while (row + 1 < rows && start[row + 1] <= e) ++row;
+          e2r[e0 + e] = (int32_t)(r0 + row);
+        }
+      }
+    }
+    distinct += total;
+    __syncthreads();
+  }
+  if (t == 0) bp[w] = (distinct + a.W - 1) / a.W;
+}
+
+// The first mid_ctas CTAs take the listed middle windows, the others `per` windows each,
+// one per warp at a time.
+template <typename K>
+__global__ void __launch_bounds__(kGroup, 8)
+    k_count(const Csr a, const int32_t* __restrict__ mid_count,
+            const int32_t* __restrict__ mid_list, int32_t mid_room, int mid_ctas, int per,
+            int32_t* __restrict__ e2c, int32_t* __restrict__ e2r, int32_t* __restrict__ bp,
+            uint32_t* bad) {
+  __shared__ __align__(16) uint8_t sm[group_bytes<K>()];
+  __shared__ int next;
+  int32_t e0, n;
+  const int t = threadIdx.x, lane = t & 31;
+  if ((int)blockIdx.x < mid_ctas) {
+    const int32_t many = min(__ldg(mid_count), mid_room);
+    for (int32_t i = blockIdx.x; i < many; i += mid_ctas) {
+      const int32_t w = __ldg(mid_list + i);
+      window_edges(a, w, e0, n);
+      if (n <= 8 * kGroup)
+        count_small<K, 8>(a, w, e0, n, sm, t, e2c, e2r, bp, bad);
+      else if constexpr (sizeof(K) == 4)
+        count_small<K, 16>(a, w, e0, n, sm, t, e2c, e2r, bp, bad);
+    }
+    return;
+  }
+  uint8_t* const wsm = sm + (t / 32) * kWarpBytes;
+  const int64_t w0 = (int64_t)(blockIdx.x - mid_ctas) * per;
+  if (t == 0) next = kGroup / 32;
+  __syncthreads();
+  for (int v = t / 32; v < per && w0 + v < a.nwin;) {
+    const int32_t w = (int32_t)(w0 + v);
+    window_edges(a, w, e0, n);
+    if (n == 0) {
+      if (lane == 0) bp[w] = 0;
+    } else if (n <= 128) {
+      count_warp<K, 4>(a, w, e0, n, wsm, lane, e2c, e2r, bp, bad);
+    } else if (n <= 256) {
+      count_warp<K, 8>(a, w, e0, n, wsm, lane, e2c, e2r, bp, bad);
+    } else if (n <= Cap<K>::kWarp) {
+      if constexpr (sizeof(K) == 4)
+        count_warp<K, 16>(a, w, e0, n, wsm, lane, e2c, e2r, bp, bad);
+    }
+    if (lane == 0) v = atomicAdd(&next, 1);
+    v = __shfl_sync(0xffffffffu, v, 0);
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+    k_count_large(const Csr a, const int32_t* __restrict__ count, const int32_t* __restrict__ list,
+                  int32_t room, int32_t* ticket, int32_t* __restrict__ e2c,
+                  int32_t* __restrict__ e2r, int32_t* __restrict__ bp, uint32_t* bad) {
+  extern __shared__ __align__(16) uint8_t dyn[];
+  __shared__ int32_t next;
+  const int32_t many = many_listed(count, room);
+  for (int32_t i = blockIdx.x; i < many;) {
+    int32_t e0, n;
+    const int32_t w = listed(count, list, room, i);
+    window_edges(a, w, e0, n);
+    count_large(a, w, e0, n, dyn, e2c, e2r, bp, bad);
+    if (threadIdx.x == 0) next = gridDim.x + atomicAdd(ticket, 1);
+    __syncthreads();
+    i = next;
+    __syncthreads();
+  }
+}
+
+// rwo = exclusive sum of bp (rwo[nwin] = T), 8192 windows per CTA; each CTA adds up the
+// windows before its own (a few coalesced loads per thread from L2) instead of a second
+// launch. out = {T, *bad}.
+constexpr int kScan = 8192;
+__global__ void __launch_bounds__(1024) k_scan(const int32_t* __restrict__ bp, int32_t nwin,
+                                               int32_t* __restrict__ rwo, const uint32_t* bad,
+                                               int32_t* out) {
+  __shared__ int32_t sums[33], part[kScan];
+  const int t = threadIdx.x;
+  const int64_t i0 = (int64_t)blockIdx.x * kScan;
+  const int cnt = (int)min((int64_t)kScan, nwin - i0);
+  int32_t before = 0;
+#pragma unroll 8
+  for (int64_t i = t; i < i0; i += 1024) before += __ldg(bp + i);
+  for (int i = t; i < kScan; i += 1024) part[i] = i < cnt ? __ldg(bp + i0 + i) : 0;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  if (t == 0) sums[32] = 0;
+  __syncthreads();
+  if ((t & 31) == 0) atomicAdd(&sums[32], before);
+  int32_t mine = 0;  // eight consecutive windows per thread
+#pragma unroll
+  for (int v = 0; v < 8; ++v) mine += part[8 * t + v];
+  int s = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, s, o);
+    if ((t & 31) >= o) s += u;
+  }
+  if ((t & 31) == 31) sums[t >> 5] = s;
+  __syncthreads();
+  if (t < 32) {
+    int y = sums[t];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, y, o);
+      if (t >= o) y += u;
+    }
+    sums[t] = y;
+  }
+  __syncthreads();
+  int32_t at = sums[32] + s - mine + (t >= 32 ? sums[(t >> 5) - 1] : 0);
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    const int32_t x = part[8 * t + v];
+    part[8 * t + v] = at;
+    at += x;
+  }
+  __syncthreads();
+  for (int i = t; i < cnt; i += 1024) rwo[i0 + i] = part[i];
+  if (t == 1023 && i0 + kScan >= nwin) {  // (the last CTA's last thread has the whole sum)
+    rwo[nwin] = at;
+    out[0] = at;
+    out[1] = (int32_t)*bad;
+  }
+}
+
+// ------------------------------------------------------------------- phase 2
+struct Fill {
+  const int32_t *e2c, *e2r, *rwo;
+  const float* values;
+  int32_t *rowid, *toff, *s2x;
+  uint8_t* tile;
+  float* tv;
+  int64_t T;
+};
+
+// Values of one block in tile order where a (row, column) may occur twice: merged into
+// its first occurrence (fp32 sum in CSR order), later ones 0.
+__device__ void merge_block(const Fill& f, int32_t j0, int32_t j1) {
+  uint32_t seen[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int32_t j = j0; j < j1; ++j) {
+    const uint32_t p = f.tile[j], bit = 1u << (p & 31);
+    if (!(seen[p >> 5] & bit)) {
+      seen[p >> 5] |= bit;
+    } else {
+      int32_t x = j0;
+      while (f.tile[x] != p) ++x;
+      f.tv[x] += f.tv[j];
+      f.tv[j] = 0.0f;
+    }
+  }
+}
+
+__device__ __forceinline__ void zero_slots(const Csr& a, const Fill& f, int64_t b1, int32_t used,
+                                           int t, int n) {  // unused slots of the last block
+  for (int s = used % a.W + t; used % a.W && s < a.W; s += n) f.s2x[(b1 - 1) * a.W + s] = 0;
+}
+
+// Where the edges of `nb` blocks go: a bit per cell of a block (its tile id) marks the
+// edges, so that in a window without repeated columns, whose rows' columns ascend, an
+// edge's place in its block is the number of set bits below its own. `pos` holds the
+// edges before each word of 32 cells. Scratch of one warp.
+struct Marks {
+  uint32_t* cell;
+  uint16_t* pos;
+  int words;  // per block
+  __device__ Marks(const Csr& a, uint8_t* sm)
+      : cell(reinterpret_cast<uint32_t*>(sm)),
+        pos(reinterpret_cast<uint16_t*>(sm + kCells)),
+        words((a.H * a.W + 31) / 32) {}
+  __device__ __forceinline__ void clear(int nb, int lane) const {
+    for (int i = lane; i < nb * words; i += 32) cell[i] = 0;
+    __syncwarp();
+  }
+  __device__ __forceinline__ void set(int b, int id) const {
+    atomicOr(cell + b * words + (id >> 5), 1u << (id & 31));
+  }
+  // Sums up; out(b, edges before block b).
+  template <typename F>
+  __device__ __forceinline__ void sum(int nb, int lane, F out) const {
+    __syncwarp();
+    int at = 0;
+    for (int c = 0; c < nb; c += 32) {
+      const int b = c + lane;
+      int mine = 0;
+      if (b < nb)
+        for (int q = 0; q < words; ++q) mine += __popc(cell[b * words + q]);
+      int y = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, y, o);
+        if (lane >= o) y += u;
+      }
+      if (b < nb) {
+        int p = at + y - mine;
+        out(b, p);
+        for (int q = 0; q < words; ++q) {
+          pos[b * words + q] = (uint16_t)p;
+          p += __popc(cell[b * words + q]);
+        }
+      }
+      at += __shfl_sync(0xffffffffu, y, 31);
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ int place(int b, int id) const {
+    const int x = b * words + (id >> 5);
+    return pos[x] + __popc(cell[x] & ((1u << (id & 31)) - 1));
+  }
+};
+
+// One warp's window; false (nothing written) where a row's ranks do not ascend or the
+// window has too many blocks.
+__device__ __forceinline__ bool fill_warp(const Csr& a, const Fill& f, int32_t w, int32_t e0,
+                                          int32_t n, uint8_t* sm, int lane) {
+  const int32_t b0 = __ldg(f.rwo + w), nb = __ldg(f.rwo + w + 1) - b0;
+  const Marks m(a, sm);
+  if (nb * m.words * 4 > kCells) return false;
+  const int32_t r0 = w * a.H;
+  m.clear(nb, lane);
+  bool mixed = false;
+  int used = 0, last_rk = -1, last_row = -1;  // of the edge before this warp's 32
+#pragma unroll 2
+  for (int i = lane; i - lane < n; i += 32) {
+    const bool in = i < n;
+    const int rk = in ? __ldg(f.e2c + e0 + i) : 0, row = in ? __ldg(f.e2r + e0 + i) - r0 : -2;
+    int prk = __shfl_up_sync(0xffffffffu, rk, 1), prow = __shfl_up_sync(0xffffffffu, row, 1);
+    if (lane == 0) { prk = last_rk; prow = last_row; }
+    mixed |= in && prow == row && prk >= rk;
+    last_rk = __shfl_sync(0xffffffffu, rk, 31);
+    last_row = __shfl_sync(0xffffffffu, row, 31);
+    if (in) {
+      used = max(used, rk + 1);
+      m.set(a.block(rk), row * a.W + a.slot(rk));
+    }
+  }
+  if (__any_sync(0xffffffffu, mixed)) return false;
+  m.sum(nb, lane, [&](int b, int before) {
+    f.toff[b0 + b] = e0 + before;
+    f.rowid[b0 + b] = w;
+  });
+  for (int i = lane; i < n; i += 128) {
+    int rk[4], row[4], c[4];
+    float x[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const bool in = i + 32 * v < n;
+      const int32_t e = e0 + i + 32 * v;
+      rk[v] = in ? __ldg(f.e2c + e) : -1;
+      row[v] = in ? __ldg(f.e2r + e) - r0 : 0;
+      c[v] = in ? __ldg(a.col + e) : 0;
+      x[v] = in && f.values ? __ldg(f.values + e) : 0.0f;
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      if (rk[v] >= 0) {
+        const int b = a.block(rk[v]), slot = a.slot(rk[v]), id = row[v] * a.W + slot;
+        const int32_t j = e0 + m.place(b, id);
+        f.tile[j] = (uint8_t)id;
+        f.s2x[(int64_t)(b0 + b) * a.W + slot] = c[v];
+        if (f.values) f.tv[j] = x[v];
+      }
+  }
+  used = __reduce_max_sync(0xffffffffu, used);
+  zero_slots(a, f, b0 + nb, used, lane, 32);
+  __syncwarp();
+  return true;
 }
 
 template <typename K>
-dtc_status phase1_sort(const Phase1Layout& L, char* ws, const int32_t* col, const int32_t* rowptr,
-                       int32_t M, int64_t nnz, int32_t H, int32_t* edgeToRow, int32_t* edgeToColumn,
-                       cudaStream_t st) {
-  K* keys_in = (K*)(ws + L.keys_in);
-  K* keys_out = (K*)(ws + L.keys_out);
-  int32_t* ids_in = (int32_t*)(ws + L.ids_in);
-  int32_t* ids_out = (int32_t*)(ws + L.ids_out);
-  int32_t* flags = (int32_t*)(ws + L.flags);
-  int32_t* P = (int32_t*)(ws + L.P);
-  k_make_keys<K><<<grid_for(nnz), kThreads, 0, st>>>(col, edgeToRow, nnz, H, L.colbits, keys_in,
-                                                     ids_in);
-  size_t tb = L.cub_scan - L.cub_sort;
-  DTC_CUDA(cub::DeviceRadixSort::SortPairs(ws + L.cub_sort, tb, keys_in, keys_out, ids_in, ids_out,
-                                           nnz, 0, L.endbit, st));
-  k_distinct_flags<K><<<grid_for(nnz + 1), kThreads, 0, st>>>(keys_out, nnz, flags);
-  size_t sb = L.total - L.cub_scan;
-  DTC_CUDA(cub::DeviceScan::ExclusiveSum(ws + L.cub_scan, sb, flags, P, nnz + 1, st));
-  k_ranks<K><<<grid_for(nnz), kThreads, 0, st>>>(keys_out, ids_out, P, rowptr, nnz, H, L.colbits,
-                                                 edgeToColumn);
+__device__ void fill_small(const Csr& a, const Fill& f, int32_t w, int32_t e0, int32_t n,
+                           uint8_t* sm, int t) {
+  constexpr int B = Cap<K>::kBits;
+  uint32_t* key = reinterpret_cast<uint32_t*>(sm);
+  int32_t* part = reinterpret_cast<int32_t*>(sm + Cap<K>::kEdges * 4);
+  const int32_t b0 = __ldg(f.rwo + w), nb = __ldg(f.rwo + w + 1) - b0;
+  int n2 = 2;
+  while (n2 < n) n2 <<= 1;
+  int used = 0, dup = 0;
+  for (int i = t; i < n2; i += kGroup) {
+    uint32_t k = 0xffffffffu;
+    if (i < n) {
+      const int32_t rk = __ldg(f.e2c + e0 + i);
+      k = ((uint32_t)(a.block(rk)) << B) | (uint32_t)i;
+      used = max(used, rk + 1);
+      // ranks that do not ascend along a row: a repeated column is possible
+      if (i > 0 && __ldg(f.e2c + e0 + i - 1) >= rk &&
+          __ldg(f.e2r + e0 + i - 1) == __ldg(f.e2r + e0 + i))
+        dup = 1;
+    }
+    key[i] = k;
+  }
+  for (int b = t; b < nb; b += kGroup) f.rowid[b0 + b] = w;
+  __syncthreads();
+  bitonic(key, n2, t);
+  for (int j = t; j < n; j += kGroup) {
+    const uint32_t k = key[j];
+    const int32_t b = b0 + (int32_t)(k >> B), e = e0 + (int32_t)(k & ((1u << B) - 1));
+    if (j == 0 || (key[j - 1] >> B) != (k >> B)) f.toff[b] = e0 + j;
+    const int32_t slot = a.slot(__ldg(f.e2c + e));
+    f.tile[e0 + j] = (uint8_t)((__ldg(f.e2r + e) - w * a.H) * a.W + slot);
+    f.s2x[(int64_t)b * a.W + slot] = __ldg(a.col + e);  // duplicates write the same value
+    if (f.values) f.tv[e0 + j] = __ldg(f.values + e);
+  }
+  // the most columns any thread saw, and whether any saw a possible duplicate
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    used = max(used, __shfl_xor_sync(0xffffffffu, used, o));
+    dup |= __shfl_xor_sync(0xffffffffu, dup, o);
+  }
+  if ((t & 31) == 0) part[t >> 5] = used * 2 + dup;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kGroup / 32; ++i) {
+    used = max(used, part[i] >> 1);
+    dup |= part[i] & 1;
+  }
+  zero_slots(a, f, b0 + nb, used, t, kGroup);
+  if (f.values && dup) {
+    __threadfence_block();
+    __syncthreads();
+    // block boundaries once more from the sorted keys
+    for (int j = t; j < n; j += kGroup)
+      if (j == 0 || (key[j - 1] >> B) != (key[j] >> B)) {
+        int j1 = j + 1;
+        while (j1 < n && (key[j1] >> B) == (key[j] >> B)) ++j1;
+        merge_block(f, e0 + j, e0 + j1);
+      }
+  }
+}
+
+__device__ void fill_large(const Csr& a, const Fill& f, int32_t w, int32_t e0, int32_t n,
+                           uint8_t* sm) {
+  int32_t* cur = reinterpret_cast<int32_t*>(sm);  // next place of each block of the sweep
+  int32_t* start = cur + kSweepBlocks;            // row starts (local), one past the last
+  int32_t* part = start + kMaxH + 1;
+  __shared__ int32_t s_used, s_dup;
+  __shared__ uint8_t s_mixed[kMaxH];              // rows whose ranks do not ascend
+  const int t = threadIdx.x;
+  const int64_t r0 = (int64_t)w * a.H;
+  const int rows = (int)min((int64_t)a.H, a.M - r0);
+  for (int r = t; r <= rows; r += kThreads) start[r] = __ldg(a.rowptr + r0 + r) - e0;
+  for (int r = t; r < rows; r += kThreads) s_mixed[r] = 0;
+  if (t == 0) s_used = s_dup = 0;
+  const int32_t b0 = __ldg(f.rwo + w), nb = __ldg(f.rwo + w + 1) - b0;
+  for (int b = t; b < nb; b += kThreads) f.rowid[b0 + b] = w;
+  int used = 0;
+  int32_t place = 0;  // edges in the blocks of the sweeps before
+  auto put = [&](int32_t i, int32_t rk, int32_t at, int row) {
+    const int32_t slot = a.slot(rk);
+    f.tile[e0 + at] = (uint8_t)(row * a.W + slot);
+    f.s2x[(int64_t)(b0 + a.block(rk)) * a.W + slot] = __ldg(a.col + e0 + i);
+    if (f.values) f.tv[e0 + at] = __ldg(f.values + e0 + i);
+  };
+  for (int32_t p0 = 0; p0 < nb; p0 += kSweepBlocks) {
+    const int32_t np = min(kSweepBlocks, nb - p0);
+    __syncthreads();
+    for (int b = t; b < np; b += kThreads) cur[b] = 0;
+    __syncthreads();
+#pragma unroll 4
+    for (int32_t i = t; i < n; i += kThreads) {
+      const int32_t rk = __ldg(f.e2c + e0 + i);
+      const uint32_t b = (uint32_t)(a.block(rk) - p0);
+      if (b < (uint32_t)np) atomicAdd(cur + b, 1);
+      if (p0 == 0) {
+        used = max(used, rk + 1);
+        if (i > 0) {
+          const int32_t before = __ldg(f.e2c + e0 + i - 1);
+          if (before >= rk) {
+            const int r = row_of(start, rows, i);
+            if (start[r] < i) {  // inside a row
+              s_dup = 1;
+              if (before > rk) s_mixed[r] = 1;
+            }
+          }
+        }
+      }
+    }
+    if (p0 == 0) atomicMax(&s_used, used);
+    __syncthreads();
+    const int per = (np + kThreads - 1) / kThreads, q0 = min(t * per, np), q1 = min(q0 + per, np);
+    int mine = 0;
+    for (int q = q0; q < q1; ++q) mine += cur[q];
+    int total;
+    int at = place + cta_scan(mine, part, &total);
+    for (int q = q0; q < q1; ++q) {
+      const int c = cur[q];
+      cur[q] = at;
+      f.toff[b0 + p0 + q] = e0 + at;
+      at += c;
+    }
+    place += total;
+    __syncthreads();
+    for (int r = 0; r < rows; ++r) {
+      const int32_t i0 = start[r], i1 = start[r + 1];
+      if (!s_mixed[r]) {
+        // equal blocks are neighbours: an edge's place is its distance to the first of them
+#pragma unroll 2
+        for (int32_t i = i0 + t; i < i1; i += kThreads) {
+          const int32_t rk = __ldg(f.e2c + e0 + i), blk = a.block(rk);
+          const uint32_t b = (uint32_t)(blk - p0);
+          if (b >= (uint32_t)np) continue;
+          int k = 0;
+          while (i - k > i0 && a.block(__ldg(f.e2c + e0 + i - k - 1)) == blk) ++k;
+          put(i, rk, cur[b] + k, r);
+        }
+        __syncthreads();
+        for (int32_t i = i0 + t; i < i1; i += kThreads) {
+          const uint32_t b = (uint32_t)(a.block(__ldg(f.e2c + e0 + i)) - p0);
+          if (b < (uint32_t)np) atomicAdd(cur + b, 1);
+        }
+      } else if (t < 32) {  // any order: 32 edges at a time, equal blocks by lane
+        for (int32_t i = i0; i < i1; i += 32) {
+          const int32_t rk = i + t < i1 ? __ldg(f.e2c + e0 + i + t) : -1;
+          const uint32_t b = rk < 0 ? 0xffffffffu : (uint32_t)(a.block(rk) - p0);
+          const bool in = b < (uint32_t)np;
+          const uint32_t same = __match_any_sync(0xffffffffu, in ? b : 0xffffffffu);
+          const int k = __popc(same & ((1u << t) - 1));
+          if (in) put(i + t, rk, cur[b] + k, r);
+          __syncwarp();
+          if (in && k == 0) cur[b] += __popc(same);
+          __syncwarp();
+        }
+      }
+      __syncthreads();
+    }
+  }
+  zero_slots(a, f, b0 + nb, s_used, t, kThreads);
+  if (f.values && s_dup) {
+    __threadfence_block();
+    __syncthreads();
+    for (int b = t; b < nb; b += kThreads)
+      merge_block(f, f.toff[b0 + b], b + 1 < nb ? f.toff[b0 + b + 1] : e0 + n);
+  }
+  __syncthreads();
+}
+
+// Blocks [p0, p0 + unit) of a window whose ranks ascend along every row, by one warp: its
+// part of each row is a run of edges.
+__device__ __forceinline__ void fill_unit(const Csr& a, const Fill& f, int32_t w, int32_t p0,
+                                          int32_t unit, uint8_t* sm, int lane) {
+  const int32_t b0 = __ldg(f.rwo + w), nb = __ldg(f.rwo + w + 1) - b0;
+  const int np = min(unit, nb - p0);
+  const Marks m(a, sm);
+  int32_t* first = reinterpret_cast<int32_t*>(sm + kCells * 3 / 2);  // first edge by row, less
+  int32_t* pre = first + kUnitH;                                     // the edges of rows before
+  const int64_t r0 = (int64_t)w * a.H;
+  const int rows = (int)min((int64_t)a.H, a.M - r0);
+  auto lower = [&](int32_t lo, int32_t hi, int32_t rk) {
+    while (lo < hi) {
+      const int32_t mid = lo + ((hi - lo) >> 1);
+      if (__ldg(f.e2c + mid) < rk) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+  };
+  // both ends of every row's part: at once where two lanes per row suffice
+  const bool twice = rows <= 16;
+  const int r = twice ? lane & 15 : lane;
+  int32_t s = 0, lo = 0, hi = 0;
+  if (r < rows) {
+    s = __ldg(a.rowptr + r0 + r);
+    const int32_t e = __ldg(a.rowptr + r0 + r + 1);
+    lo = lower(s, e, (twice && lane >= 16 ? p0 + np : p0) * a.W);
+    if (!twice) hi = lower(lo, e, (p0 + np) * a.W);
+  }
+  if (twice) hi = __shfl_xor_sync(0xffffffffu, lo, 16);
+  if (twice && lane >= 16) s = lo = hi = 0;
+  const int32_t start = __reduce_add_sync(0xffffffffu, lo - s);  // edges of the blocks before
+  int x = hi - lo;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += u;
+  }
+  const int n = __shfl_sync(0xffffffffu, x, 31);
+  if (lane < rows) first[lane] = lo - (x - (hi - lo));
+  if (lane < rows) pre[lane + 1] = x;
+  m.clear(np, lane);
+  const int32_t e0 = __ldg(a.rowptr + r0);
+  int used = 0, row = 0;
+  // (four edges per lane at a time: their rows and places first, then all the loads)
+  for (int i = lane; i < n; i += 128) {
+    int rk[4], id[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      if (i + 32 * v < n) {
+        while (pre[row + 1] <= i + 32 * v) ++row;  // (pre[rows] = n)
+        rk[v] = first[row] + i + 32 * v;
+        id[v] = row * a.W;
+      }
+#pragma unroll
+    for (int v = 0; v < 4; ++v) rk[v] = i + 32 * v < n ? __ldg(f.e2c + rk[v]) : -1;
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      if (rk[v] >= 0) {
+        used = max(used, rk[v] + 1);
+        m.set(a.block(rk[v]) - p0, id[v] + a.slot(rk[v]));
+      }
+  }
+  m.sum(np, lane, [&](int b, int before) {
+    f.toff[b0 + p0 + b] = e0 + start + before;
+    f.rowid[b0 + p0 + b] = w;
+  });
+  row = 0;
+  for (int i = lane; i < n; i += 128) {
+    int e[4], rk[4], id[4], c[4];
+    float x[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      if (i + 32 * v < n) {
+        while (pre[row + 1] <= i + 32 * v) ++row;
+        e[v] = first[row] + i + 32 * v;
+        id[v] = row * a.W;
+      }
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const bool in = i + 32 * v < n;
+      rk[v] = in ? __ldg(f.e2c + e[v]) : -1;
+      c[v] = in ? __ldg(a.col + e[v]) : 0;
+      x[v] = in && f.values ? __ldg(f.values + e[v]) : 0.0f;
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      if (rk[v] >= 0) {
+        const int b = a.block(rk[v]), slot = a.slot(rk[v]);
+        const int32_t j = e0 + start + m.place(b - p0, id[v] + slot);
+        f.tile[j] = (uint8_t)(id[v] + slot);
+        f.s2x[(int64_t)(b0 + b) * a.W + slot] = c[v];
+        if (f.values) f.tv[j] = x[v];
+      }
+  }
+  used = __reduce_max_sync(0xffffffffu, used);
+  if (p0 + np == nb) zero_slots(a, f, b0 + nb, used, lane, 32);
+  __syncwarp();
+}
+
+// Warps first take the units of the listed windows (more than kWarpFill edges), then a
+// window each.
+template <typename K>
+__global__ void __launch_bounds__(kGroup, 8)
+    k_fill(const Csr a, const Fill f, const int32_t* __restrict__ units,
+           const int2* __restrict__ unit_list, const uint8_t* __restrict__ mixed, int unit,
+           int64_t unit_room, int unit_ctas, int per) {
+  __shared__ __align__(16) uint8_t sm[group_bytes<K>()];
+  __shared__ int next, redo;  // windows that one warp could not do
+  const int t = threadIdx.x;
+  if ((int)blockIdx.x < unit_ctas) {
+    const int32_t many = (int32_t)min((int64_t)__ldg(units), unit_room);
+    for (int32_t i = blockIdx.x * 4 + t / 32; i < many; i += unit_ctas * 4) {
+      const int2 u = __ldg(unit_list + i);
+      if (!__ldg(mixed + u.x))
+        fill_unit(a, f, u.x, u.y, unit, sm + (t / 32) * kWarpBytes, t & 31);
+    }
+    return;
+  }
+  int32_t e0, n;
+  const int64_t w0 = (int64_t)(blockIdx.x - unit_ctas) * per;
+  if (w0 == 0 && t == 0) f.toff[f.T] = (int32_t)a.nnz;
+  if (t == 0) {
+    next = kGroup / 32;
+    redo = 0;
+  }
+  __syncthreads();
+  for (int v = t / 32; v < per && w0 + v < a.nwin;) {
+    window_edges(a, (int32_t)(w0 + v), e0, n);
+    if (n > 0 && n <= kWarpFill &&
+        !fill_warp(a, f, (int32_t)(w0 + v), e0, n, sm + (t / 32) * kWarpBytes, t & 31) &&
+        (t & 31) == 0)
+      atomicOr(&redo, 1 << v);
+    if ((t & 31) == 0) v = atomicAdd(&next, 1);
+    v = __shfl_sync(0xffffffffu, v, 0);
+  }
+  __syncthreads();
+  for (uint32_t todo = (uint32_t)redo; todo; todo &= todo - 1) {
+    const int32_t w = (int32_t)(w0 + __ffs(todo) - 1);
+    window_edges(a, w, e0, n);
+    __syncthreads();
+    fill_small<K>(a, f, w, e0, n, sm, t);
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+    k_fill_mixed(const Csr a, const Fill f, const int32_t* __restrict__ count,
+                 const int32_t* __restrict__ list, const uint8_t* __restrict__ mixed,
+                 int32_t room, const int32_t* __restrict__ any) {
+  extern __shared__ __align__(16) uint8_t dyn[];
+  if (!__ldg(any)) return;
+  const int32_t many = many_listed(count, room);
+  for (int32_t i = blockIdx.x; i < many; i += gridDim.x) {
+    const int32_t w = listed(count, list, room, i);
+    if (__ldg(mixed + w)) {
+      int32_t e0, n;
+      window_edges(a, w, e0, n);
+      fill_large(a, f, w, e0, n, dyn);
+    }
+  }
+}
+
+Csr make_csr(const int32_t* col, const int32_t* rowptr, int32_t M, int32_t nwin, int32_t H,
+             int32_t W, int64_t nnz) {
+  const int32_t b = bits_for((uint64_t)W);
+  return {col, rowptr, M, nwin, H, W, nnz, W == 1 ? 0 : (1 << b) == W ? b : -1};
+}
+
+struct Layout {
+  size_t head, list, mid, mixed, units, total;  // head: see Head
+  int64_t room, mid_room, unit_room;                 // entries of the lists
+  bool wide;
+};
+
+// Words of the workspace's head, zero at the start of a phase.
+enum Head { kCount = 0, kBad = 2, kOut = 3, kUnits = 5, kTicket = 6, kMid = 7, kAny = 8, kHead = 9 };
+
+// Blocks per unit of a large window (0: none, rows beyond the warp's arrays).
+int unit_blocks(int H) { return H > kUnitH ? 0 : 128; }
+static_assert(128 * 8 * 4 <= kCells, "a unit's masks fit");
+
+Layout layout(int32_t M, int64_t nnz, int32_t H) {
+  Layout L{};
+  L.wide = bits_for((uint64_t)(M > 0 ? M : 1)) + Cap<uint32_t>::kBits > 32;
+  const size_t large = (size_t)nnz / (kWarpFill + 1) + 1;  // listed windows, at most
+  const int unit = unit_blocks(H);
+  L.room = (int64_t)large;
+  L.unit_room = unit ? nnz / unit + (int64_t)large : 0;
+  L.head = 0;
+  L.list = 256;
+  L.mid_room = nnz / (Cap<uint64_t>::kWarp + 1) + 1;
+  L.mid = align_up(L.list + large * 4, 256);
+  L.mixed = align_up(L.mid + (size_t)L.mid_room * 4, 256);
+  L.units = align_up(L.mixed + ((size_t)M + H - 1) / H, 256);
+  L.total = align_up(L.units + (size_t)L.unit_room * 8, 256);
+  return L;
+}
+
+static_assert(kSweepBlocks * 4 + (kMaxH + 1) * 4 + 256 <= kLargeBytes, "fill_large fits");
+static_assert(kWarpFill <= Cap<uint64_t>::kEdges, "fill_small takes what a warp could not");
+
+// CTAs for the windows of more than `cap` edges: no more than there can be, one per SM.
+int large_ctas(int64_t nnz, int cap) {
+  const int64_t most = nnz / (cap + 1), want = num_sms();
+  return (int)(most < want ? most : want);
+}
+
+// Windows per CTA: kPer share out uneven windows among its warps, fewer where that would
+// leave SMs idle.
+int windows_per_cta(int32_t nwin) {
+  const int64_t p = nwin / (8 * (int64_t)num_sms());
+  return p < 4 ? 4 : p > kPer ? kPer : (int)p;
+}
+static_assert(kPer <= 32, "a bit per window");
+
+template <typename K>
+dtc_status count_impl(const Csr& a, char* ws, const Layout& L, int32_t* e2c, int32_t* e2r,
+                      int32_t* bp, cudaStream_t st) {
+  int32_t* count = (int32_t*)(ws + L.head) + kCount;
+  int32_t* list = (int32_t*)(ws + L.list);
+  uint32_t* bad = (uint32_t*)(ws + L.head) + kBad;
+  int32_t* mid_count = (int32_t*)(ws + L.head) + kMid;
+  int32_t* mid_list = (int32_t*)(ws + L.mid);
+  k_list<<<(a.nwin + 255) / 256, 256, 0, st>>>(a, Cap<K>::kEdges, Cap<K>::kWarp, count, list,
+                                               mid_count, mid_list, (int32_t)L.mid_room, bad,
+                                               (int32_t)L.room, nullptr, 0, nullptr, nullptr, 0);
+  const int large = large_ctas(a.nnz, Cap<K>::kEdges);
+  if (large) {
+    DTC_CUDA(cudaFuncSetAttribute(k_count_large, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kLargeBytes));
+    k_count_large<<<large, kThreads, kLargeBytes, st>>>(a, count, list, (int32_t)L.room,
+                                                        (int32_t*)(ws + L.head) + kTicket, e2c,
+                                                        e2r, bp, bad);
+  }
+  const int64_t most = a.nnz / (Cap<K>::kWarp + 1), want = 8 * (int64_t)num_sms();
+  const int mid_ctas = (int)(most < want ? most : want), per = windows_per_cta(a.nwin);
+  k_count<K><<<(unsigned)(mid_ctas + (a.nwin + per - 1) / per), kGroup, 0, st>>>(
+      a, mid_count, mid_list, (int32_t)L.mid_room, mid_ctas, per, e2c, e2r, bp, bad);
+  return DTC_OK;
+}
+
+template <typename K>
+dtc_status fill_impl(const Csr& a, const Fill& f, char* ws, const Layout& L, cudaStream_t st) {
+  int32_t* count = (int32_t*)(ws + L.head) + kCount;
+  int32_t* list = (int32_t*)(ws + L.list);
+  const int large = large_ctas(a.nnz, kWarpFill);
+  int32_t* units = (int32_t*)(ws + L.head) + kUnits;
+  int2* unit_list = (int2*)(ws + L.units);
+  uint8_t* mixed = (uint8_t*)(ws + L.mixed);
+  const int unit = unit_blocks(a.H);
+  int unit_ctas = 0;
+  if (large) {
+    k_list<<<(a.nwin + 255) / 256, 256, 0, st>>>(a, kWarpFill, INT32_MAX, count, list, nullptr,
+                                                 nullptr, 0, nullptr,
+                                                 (int32_t)L.room, f.rwo, unit, units, unit_list,
+                                                 L.unit_room);
+    int32_t* any = (int32_t*)(ws + L.head) + kAny;
+    DTC_CUDA(cudaMemsetAsync(mixed, unit ? 0 : 1, a.nwin, st));
+    if (!unit) DTC_CUDA(cudaMemsetAsync(any, 1, 4, st));
+    if (unit) {
+      k_mixed<<<(unsigned)((a.nnz + 2047) / 2048), 256, 0, st>>>(a, f.e2c, f.e2r, mixed,
+                                                                      any);
+      // a warp per unit up to eight CTAs per SM
+      const int64_t most = (L.unit_room + 3) / 4, want = 8 * (int64_t)num_sms();
+      unit_ctas = (int)(most < want ? most : want);
+    }
+    DTC_CUDA(cudaFuncSetAttribute(k_fill_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kLargeBytes));
+    k_fill_mixed<<<large, kThreads, kLargeBytes, st>>>(a, f, count, list, mixed,
+                                                       (int32_t)L.room, any);
+  }
+  const int per = windows_per_cta(a.nwin);
+  k_fill<K><<<(unsigned)(unit_ctas + (a.nwin + per - 1) / per), kGroup, 0, st>>>(
+      a, f, units, unit_list, mixed, unit, L.unit_room, unit_ctas, per);
   return DTC_OK;
 }
 
@@ -288,11 +1216,9 @@ extern "C" dtc_status dtc_convert_workspace_bytes(int32_t num_nodes, int64_t nnz
   DTC_REQUIRE(bytes != nullptr, "bytes is null");
   DTC_REQUIRE(num_nodes >= 0 && nnz >= 0 && block_h > 0 && block_w > 0,
               "negative sizes or non-positive block shape");
-  DTC_REQUIRE(block_h * block_w <= 256, "block_h * block_w must be <= 256 (u8 tile ids)");
+  DTC_REQUIRE((int64_t)block_h * block_w <= 256, "block_h * block_w must be <= 256 (u8 tile ids)");
   DTC_REQUIRE(nnz < (int64_t)INT32_MAX, "nnz must fit in int32 (reference index type)");
-  Phase1Layout a = phase1_layout(num_nodes, nnz, block_h);
-  Phase2Layout b = phase2_layout(nnz, nnz);
-  *bytes = a.total > b.total ? a.total : b.total;
+  *bytes = layout(num_nodes, nnz, block_h).total;
   return DTC_OK;
 }
 
@@ -314,38 +1240,26 @@ extern "C" dtc_status dtc_convert_count(const int32_t* d_col, const int32_t* d_r
     return DTC_ERR_WORKSPACE_TOO_SMALL;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  int32_t nwin = (num_nodes + block_h - 1) / block_h;
-  Phase1Layout L = phase1_layout(num_nodes, nnz, block_h);
+  const int32_t nwin = (int32_t)(((int64_t)num_nodes + block_h - 1) / block_h);
+  const Layout L = layout(num_nodes, nnz, block_h);
   char* ws = (char*)d_workspace;
-  uint32_t* bad = (uint32_t*)(ws + L.bad);
-  DTC_CUDA(cudaMemsetAsync(bad, 0, 4, st));
-  k_validate<<<grid_for((nnz > num_nodes ? nnz : num_nodes) + 1), kThreads, 0, st>>>(
-      d_col, d_rowptr, num_nodes, nnz, num_nodes, bad);
-  if (nnz > 0) {
-    k_edge_to_row<<<grid_for((int64_t)num_nodes * 32), kThreads, 0, st>>>(d_rowptr, num_nodes,
-                                                                           d_edgeToRow);
-    s = L.wide ? phase1_sort<uint64_t>(L, ws, d_col, d_rowptr, num_nodes, nnz, block_h, d_edgeToRow,
-                                       d_edgeToColumn, st)
-               : phase1_sort<uint32_t>(L, ws, d_col, d_rowptr, num_nodes, nnz, block_h, d_edgeToRow,
-                                       d_edgeToColumn, st);
+  const Csr a = make_csr(d_col, d_rowptr, num_nodes, nwin, block_h, block_w, nnz);
+  DTC_CUDA(cudaMemsetAsync(ws + L.head, 0, kHead * 4, st));
+  uint32_t* bad = (uint32_t*)(ws + L.head) + kBad;
+  if (nwin > 0) {
+    s = L.wide ? count_impl<uint64_t>(a, ws, L, d_edgeToColumn, d_edgeToRow, d_blockPartition, st)
+               : count_impl<uint32_t>(a, ws, L, d_edgeToColumn, d_edgeToRow, d_blockPartition, st);
     if (s != DTC_OK) return s;
   } else {
-    DTC_CUDA(cudaMemsetAsync(ws + L.P, 0, 4, st));
+    k_list<<<1, 32, 0, st>>>(a, 0, 0, nullptr, nullptr, nullptr, nullptr, 0, bad, 0,
+                             nullptr, 0, nullptr, nullptr, 0);
   }
-  int32_t* bp_ext = (int32_t*)(ws + L.bp_ext);
-  if (nwin > 0) {
-    k_block_partition<<<grid_for((int64_t)nwin + 1), kThreads, 0, st>>>(
-        (int32_t*)(ws + L.P), d_rowptr, num_nodes, nwin, block_h, block_w, d_blockPartition,
-        bp_ext);
-    size_t sb = L.total - L.cub_scan;
-    DTC_CUDA(cub::DeviceScan::ExclusiveSum(ws + L.cub_scan, sb, bp_ext, d_rowWindowOffset,
-                                           (int64_t)nwin + 1, st));
-  } else {
-    DTC_CUDA(cudaMemsetAsync(d_rowWindowOffset, 0, 4, st));
-  }
+  int32_t* out = (int32_t*)(ws + L.head) + kOut;
+  k_scan<<<nwin ? (nwin + kScan - 1) / kScan : 1, 1024, 0, st>>>(d_blockPartition, nwin,
+                                                                 d_rowWindowOffset, bad, out);
+  DTC_CUDA(cudaGetLastError());
   int32_t hostv[2] = {0, 0};
-  DTC_CUDA(cudaMemcpyAsync(&hostv[0], d_rowWindowOffset + nwin, 4, cudaMemcpyDeviceToHost, st));
-  DTC_CUDA(cudaMemcpyAsync(&hostv[1], bad, 4, cudaMemcpyDeviceToHost, st));
+  DTC_CUDA(cudaMemcpyAsync(hostv, out, 8, cudaMemcpyDeviceToHost, st));
   DTC_CUDA(cudaStreamSynchronize(st));
   if (hostv[1] != 0) {
     set_error("invalid CSR input (flags " + std::to_string(hostv[1]) +
@@ -378,33 +1292,19 @@ extern "C" dtc_status dtc_convert_fill(const int32_t* d_col, const int32_t* d_ro
     return DTC_ERR_WORKSPACE_TOO_SMALL;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  int32_t nwin = (num_nodes + block_h - 1) / block_h;
   if (num_blocks == 0 || nnz == 0) {
     DTC_CUDA(cudaMemsetAsync(d_tcblockOffset, 0, 4, st));
     return DTC_OK;
   }
-  Phase2Layout L = phase2_layout(nnz, num_blocks);
+  const int32_t nwin = (int32_t)(((int64_t)num_nodes + block_h - 1) / block_h);
+  const Layout L = layout(num_nodes, nnz, block_h);
   char* ws = (char*)d_workspace;
-  uint32_t* blk_in = (uint32_t*)(ws + L.blk_in);
-  uint32_t* blk_out = (uint32_t*)(ws + L.blk_out);
-  int32_t* ids_in = (int32_t*)(ws + L.ids_in);
-  int32_t* ids_out = (int32_t*)(ws + L.ids_out);
-  k_block_rowid<<<grid_for((int64_t)nwin * 32), kThreads, 0, st>>>(d_rowWindowOffset, nwin,
-                                                                   d_tcblockRowid);
-  DTC_CUDA(cudaMemsetAsync(d_sparseAToX, 0, (size_t)num_blocks * block_w * 4, st));
-  k_edge_block<<<grid_for(nnz), kThreads, 0, st>>>(d_edgeToColumn, d_edgeToRow, d_rowWindowOffset,
-                                                   nnz, block_h, block_w, blk_in, ids_in);
-  size_t tb = L.total - L.cub_sort;
-  DTC_CUDA(cub::DeviceRadixSort::SortPairs(ws + L.cub_sort, tb, blk_in, blk_out, ids_in, ids_out,
-                                           nnz, 0, L.endbit, st));
-  k_scatter_tiles<<<grid_for(nnz), kThreads, 0, st>>>(blk_out, ids_out, d_col, d_edgeToColumn,
-                                                      d_edgeToRow, nnz, num_blocks, block_h,
-                                                      block_w, d_tcblockOffset, d_tileId,
-                                                      d_sparseAToX);
-  if (d_values) {
-    k_tile_values<<<grid_for(num_blocks), kThreads, 0, st>>>(d_tcblockOffset, d_tileId, ids_out,
-                                                             d_values, num_blocks, d_tcValues);
-  }
+  const Csr a = make_csr(d_col, d_rowptr, num_nodes, nwin, block_h, block_w, nnz);
+  const Fill f{d_edgeToColumn, d_edgeToRow, d_rowWindowOffset, d_values, d_tcblockRowid,
+               d_tcblockOffset, d_sparseAToX, d_tileId, d_tcValues, num_blocks};
+  DTC_CUDA(cudaMemsetAsync(ws + L.head, 0, kHead * 4, st));
+  s = L.wide ? fill_impl<uint64_t>(a, f, ws, L, st) : fill_impl<uint32_t>(a, f, ws, L, st);
+  if (s != DTC_OK) return s;
   DTC_CUDA(cudaGetLastError());
   return DTC_OK;
 }

@@ -52,17 +52,17 @@ py::tuple preprocess_gpu(torch::Tensor edgeList, torch::Tensor nodePointer, int6
   check(dtc_convert_workspace_bytes((int32_t)num_nodes, nnz, (int32_t)blockSize_h,
                                     (int32_t)blockSize_w, &wsb), "dtc_convert_workspace_bytes");
   auto ws = torch::empty({(int64_t)wsb}, u8);
-  auto rwo = torch::zeros({nwin + 1}, i32);
+  auto rwo = torch::empty({nwin + 1}, i32);
   int64_t T = 0;
   check(dtc_convert_count(edgeList.data_ptr<int32_t>(), nodePointer.data_ptr<int32_t>(),
                           (int32_t)num_nodes, nnz, (int32_t)blockSize_h, (int32_t)blockSize_w,
                           blockPartition.data_ptr<int32_t>(), edgeToColumn.data_ptr<int32_t>(),
                           edgeToRow.data_ptr<int32_t>(), rwo.data_ptr<int32_t>(), ws.data_ptr(),
                           wsb, &T, cur_stream()), "dtc_convert_count");
-  auto rowid = torch::zeros({T}, i32);
-  auto tile = torch::zeros({nnz}, u8);
-  auto toff = torch::zeros({T + 1}, i32);
-  auto s2x = torch::zeros({T * blockSize_w}, i32);
+  auto rowid = torch::empty({T}, i32);
+  auto tile = torch::empty({nnz}, u8);
+  auto toff = torch::empty({T + 1}, i32);
+  auto s2x = torch::empty({T * blockSize_w}, i32);
   torch::Tensor tv;
   const float* vptr = nullptr;
   float* tvptr = nullptr;
@@ -70,7 +70,7 @@ py::tuple preprocess_gpu(torch::Tensor edgeList, torch::Tensor nodePointer, int6
     auto v = values.value();
     CHECK_INPUT(v); CHECK_DTYPE(v, torch::kFloat32);
     TORCH_CHECK(v.numel() == nnz, "values must have nnz entries");
-    tv = torch::zeros({nnz}, v.options());
+    tv = torch::empty({nnz}, v.options());
     vptr = v.data_ptr<float>();
     tvptr = tv.data_ptr<float>();
   }

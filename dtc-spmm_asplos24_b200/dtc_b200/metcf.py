@@ -57,10 +57,10 @@ def convert(rowptr, col, M, H=16, W=8, values=None, device="cuda"):
     nnz = col.numel()
     nwin = (M + H - 1) // H
     i32 = dict(dtype=torch.int32, device=device)
-    bp = torch.zeros(nwin, **i32)
-    e2c = torch.zeros(nnz, **i32)
-    e2r = torch.zeros(nnz, **i32)
-    rwo = torch.zeros(nwin + 1, **i32)
+    bp = torch.empty(nwin, **i32)
+    e2c = torch.empty(nnz, **i32)
+    e2r = torch.empty(nnz, **i32)
+    rwo = torch.empty(nwin + 1, **i32)
     wsb = C.c_size_t()
     call("dtc_convert_workspace_bytes", M, nnz, H, W, C.byref(wsb))
     ws = torch.empty(max(wsb.value, 1), dtype=torch.uint8, device=device)
@@ -68,15 +68,15 @@ def convert(rowptr, col, M, H=16, W=8, values=None, device="cuda"):
     call("dtc_convert_count", _ptr(col), _ptr(rowptr), M, nnz, H, W, _ptr(bp), _ptr(e2c),
          _ptr(e2r), _ptr(rwo), _ptr(ws), wsb.value, C.byref(T), _stream())
     T = T.value
-    rowid = torch.zeros(T, **i32)
-    tile = torch.zeros(nnz, dtype=torch.uint8, device=device)
-    toff = torch.zeros(T + 1, **i32)
-    s2x = torch.zeros(T * W, **i32)
+    rowid = torch.empty(T, **i32)
+    tile = torch.empty(nnz, dtype=torch.uint8, device=device)
+    toff = torch.empty(T + 1, **i32)
+    s2x = torch.empty(T * W, **i32)
     tv = None
     vals = None
     if values is not None:
         vals = torch.as_tensor(values, dtype=torch.float32).to(device).contiguous()
-        tv = torch.zeros(nnz, dtype=torch.float32, device=device)
+        tv = torch.empty(nnz, dtype=torch.float32, device=device)
     call("dtc_convert_fill", _ptr(col), _ptr(rowptr), M, nnz, H, W, _ptr(e2c), _ptr(e2r),
          _ptr(rwo), T, _ptr(rowid), _ptr(tile), _ptr(toff), _ptr(s2x), _ptr(vals), _ptr(tv),
          _ptr(ws), wsb.value, _stream())

@@ -1,0 +1,47 @@
+"""ME-TCF conversion at the edges of its window classes (edges of a window sorted by one
+warp, by one CTA, ranked by a bitmap; placed by one warp, in units, row by row): bit-exact
+with the oracle, integers and merged values alike."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+COUNTS = [0, 1, 31, 33, 128, 129, 256, 257, 512, 513, 1024, 1025, 2048, 2049, 16384, 16385, 40000]
+
+
+def _matrix(M, H, order, seed=0):
+    """Windows of COUNTS edges spread over the rows, the last one on the last window."""
+    rng = np.random.default_rng(seed)
+    nwin = (M + H - 1) // H
+    deg = np.zeros(M, np.int64)
+    rows = {}
+    for i, n in enumerate(COUNTS):
+        w = (nwin - 1) * i // (len(COUNTS) - 1)
+        r0, r1 = w * H, min(w * H + H, M)
+        share = rng.multinomial(n, rng.dirichlet(np.ones(r1 - r0)))
+        for r, d in zip(range(r0, r1), share):
+            if order == "mixed" and r % 3:  # repeated and unsorted columns
+                c = rng.integers(0, max(1, M // 7), d)
+            else:
+                c = np.sort(rng.choice(M, d, replace=False)) if d else np.empty(0, np.int64)
+            rows[r], deg[r] = c, d
+    rowptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    col = np.concatenate([rows[r] for r in sorted(rows)]).astype(np.int32)
+    return rowptr, col, rng.random(col.size).astype(np.float32)
+
+
+@pytest.mark.parametrize("order", ["ascending", "mixed"])
+@pytest.mark.parametrize("M,H,W", [(60001, 16, 8), (60001, 32, 8), (60001, 16, 16), (60001, 1, 256),
+                                   (60001, 5, 7), (60001, 64, 4), (60001, 256, 1),
+                                   (2 ** 21 + 5, 16, 8)])
+def test_window_classes(cuda, M, H, W, order):
+    from dtc_b200 import metcf
+    rowptr, col, val = _matrix(M, H, order)
+    got = metcf.convert(rowptr, col, M, H=H, W=W, values=val)
+    exp = O.metcf(rowptr, col, M, H=H, W=W, values=val)
+    assert got.T == exp["T"]
+    for k in ("RowWindowOffset", "TCblockRowid", "TCblocktileId", "TCblockoffset", "SparseAToX",
+              "blockPartition", "edgeToColumn", "edgeToRow", "TCvalues"):
+        np.testing.assert_array_equal(getattr(got, k).cpu().numpy(), exp[k], err_msg=k)
