@@ -5,10 +5,18 @@
 // reorder[i_new] = i_old, d[old] = new, src' = d[src], dst' = d[dst]) and
 // rebuilds CSR with scipy (scripts/DTCSpMM/dataset.py:38-44: coo_matrix(...)
 // .tocsr(), which sorts the columns of each row and sums duplicate entries).
-// Both operations here produce that canonical CSR: every edge (r, c, v) is
-// mapped to (r', c'), pairs are radix-sorted by (r', c') with a stable sort,
-// equal pairs are merged by summing their values in input CSR order, and the
-// row pointer is rebuilt from the sorted rows.
+// Both operations here produce that canonical CSR: the edges are radix-sorted by their
+// new row and column, values carried along, and one pass over the sorted edges writes the
+// columns, the values and the row pointer. A transposition sorts by the old column only
+// (32-bit keys, three passes for 2^19 columns where row and column took five passes of
+// 64-bit keys): edges come in row order and the sort is stable. Equal pairs are merged by
+// summing their values in input CSR order; as a canonical input has none, the pass assumes
+// so, and only where it meets one a second, compacting pass follows.
+// Bound: DRAM and the sort, 24 bytes per edge and pass. R-MAT 2^19 (16.0 M edges)
+// transposed with values: 0.67 ms, of it 0.46 the sort (1.38 ms with a row search per edge,
+// 64-bit keys, values gathered through edge numbers and separate passes for flags, scan,
+// output and row pointer).
+#include <algorithm>
 #include <cub/cub.cuh>
 #include "common.cuh"
 
@@ -42,143 +50,274 @@ __global__ void k_invert(const int32_t* __restrict__ perm, int32_t M, int32_t* _
   }
 }
 
-// Checks the input CSR (rowptr[0] == 0, non-decreasing, rowptr[M] == nnz,
-// 0 <= col < K) and writes the old row of every edge. Edge-parallel: thread e
-// finds its row by binary search, the last r in [0, M) with rowptr[r] <= e
-// (for a valid CSR the row holding e; empty rows before it share its start and
-// lose to it). Neighbouring edges take the same search path, so a warp's loads
-// are mostly broadcasts of cached entries, and a hub row of tens of thousands
-// of entries costs no more than as many short rows (with a warp per row, one
-// warp would walk each hub row alone). Every probe reads rowptr[1 .. M-1], so
-// an invalid CSR stays in bounds; it sets the error bit and is rejected by the
-// host before erow is read.
-__global__ void k_rows(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
-                       int32_t M, int32_t K, int64_t nnz, int32_t* __restrict__ erow,
-                       uint32_t* bad) {
-  const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r = t0; r < M; r += stride) {
-    const int32_t e0 = __ldg(rowptr + r), e1 = __ldg(rowptr + r + 1);
-    if (e1 < e0 || (r == 0 && e0 != 0) || (r == M - 1 && e1 != nnz)) atomicOr(bad, 2u);
+// The edges in sorted order. Transposition: key = new row (the old column), `row` the old
+// row of each edge, alone or (pair) with its value; otherwise key = new row << colbits |
+// new column and `val` the values.
+template <bool kT>
+struct Sorted {
+  const uint32_t* key32;
+  const uint64_t* key64;
+  const uint32_t* row;
+  const uint2* pair;
+  const float* val;
+  int colbits;
+  __device__ __forceinline__ uint2 at(int64_t i) const {  // (new row, new column)
+    if constexpr (kT) return make_uint2(__ldg(key32 + i), pair ? __ldg(&pair[i].x) : __ldg(row + i));
+    const uint64_t k = __ldg(key64 + i);
+    return make_uint2((uint32_t)(k >> colbits), (uint32_t)(k & ((1ull << colbits) - 1)));
   }
-  for (int64_t e = t0; e < nnz; e += stride) {
-    int32_t lo = 0, hi = M;  // rowptr[lo] <= e (rowptr[0] == 0), and hi == M or rowptr[hi] > e
-    while (hi - lo > 1) {
-      const int32_t mid = lo + ((hi - lo) >> 1);
-      if (__ldg(rowptr + mid) <= e) lo = mid; else hi = mid;
+  __device__ __forceinline__ float value(int64_t i) const {
+    if constexpr (kT) return pair ? __uint_as_float(__ldg(&pair[i].y)) : 1.0f;
+    return val ? __ldg(val + i) : 1.0f;
+  }
+};
+
+// The last r in [0, M) with rowptr[r] <= e, found by a warp, 32 probes at a time. Probes
+// stay in rowptr[1, M) for any contents.
+__device__ __forceinline__ int32_t row_at(const int32_t* __restrict__ rowptr, int32_t M, int64_t e) {
+  int32_t lo = 0, hi = M;
+  while (hi - lo > 1) {
+    const int32_t step = (hi - lo) / 33 + 1;
+    const int64_t p = lo + (int64_t)(threadIdx.x % 32 + 1) * step;
+    const int before = __popc(__ballot_sync(0xffffffffu, p < hi && __ldg(rowptr + p) <= e));
+    lo += before * step;
+    hi = (int32_t)min((int64_t)hi, (int64_t)lo + step);
+  }
+  return lo;
+}
+
+// Checks the input (CSR: rowptr[0] == 0, non-decreasing, rowptr[M] == nnz; 0 <= col < K;
+// COO, mode 2: 0 <= row < M) and writes the keys and what they carry. A CTA takes 2048
+// edges: it marks the places where rows start and a maximum scan gives every edge its row
+// (a search per edge took 19 dependent loads, 211 us for R-MAT 2^19; a warp per row walks
+// each hub row alone). mode 0: permutation (inv applied to row and column), 1: transpose,
+// 2: identity. Bad inputs are clamped: they stay in bounds until the host reads the error.
+constexpr int kTile = 2048;
+__global__ void __launch_bounds__(kThreads)
+    k_expand(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+             const float* __restrict__ val, const int32_t* __restrict__ inv, int32_t M, int32_t K,
+             int64_t nnz, int mode, int colbits, uint32_t* __restrict__ key32,
+             uint64_t* __restrict__ key64, uint32_t* __restrict__ row_pay,
+             uint2* __restrict__ pair_pay, uint32_t* bad) {
+  __shared__ int32_t row[kTile], warp_max[kThreads / 32], ends[2];
+  const int t = threadIdx.x;
+  const int64_t t0 = (int64_t)blockIdx.x * kTile;
+  if (mode != 2)
+    for (int64_t r = (int64_t)blockIdx.x * kThreads + t; r < M; r += (int64_t)gridDim.x * kThreads) {
+      const int32_t e0 = __ldg(rowptr + r), e1 = __ldg(rowptr + r + 1);
+      if (e1 < e0 || (r == 0 && e0 != 0) || (r == M - 1 && e1 != nnz)) atomicOr(bad, 2u);
     }
-    erow[e] = lo;
-    const int32_t c = __ldg(col + e);
-    if (c < 0 || c >= K) atomicOr(bad, 2u);
+  if (t0 >= nnz) return;
+  const int cnt = (int)min((int64_t)kTile, nnz - t0);
+  constexpr int V = kTile / kThreads;
+  int32_t c[V], r[V];
+  float x[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) {  // (under way while the rows are found)
+    const int i = v * kThreads + t;
+    c[v] = i < cnt ? __ldg(col + t0 + i) : 0;
+    x[v] = i < cnt && pair_pay ? __ldg(val + t0 + i) : 0.0f;
+    r[v] = i < cnt && mode == 2 ? __ldg(rowptr + t0 + i) : 0;
+  }
+  if (mode != 2) {
+    if (t < 64) {
+      const int32_t r = row_at(rowptr, M, t < 32 ? t0 : t0 + cnt - 1);
+      if (t % 32 == 0) ends[t / 32] = r;
+    }
+    for (int i = t; i < kTile; i += kThreads) row[i] = 0;
+    __syncthreads();
+    const int32_t r0 = ends[0], r1 = ends[1];
+    for (int32_t r = r0 + 1 + t; r <= r1; r += kThreads) {
+      const int64_t at = __ldg(rowptr + r) - t0;
+      if (at >= 0 && at < kTile) atomicMax(row + at, r);  // (the last of rows that start here)
+    }
+    __syncthreads();
+    int32_t y[V];  // eight neighbours per thread
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      y[v] = row[t * V + v];
+      if (v) y[v] = max(y[v], y[v - 1]);
+    }
+    int32_t m = y[V - 1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int32_t u = __shfl_up_sync(0xffffffffu, m, o);
+      if ((t & 31) >= o) m = max(m, u);
+    }
+    if ((t & 31) == 31) warp_max[t >> 5] = m;
+    __syncthreads();
+    int32_t before = __shfl_up_sync(0xffffffffu, m, 1);
+    if ((t & 31) == 0) before = 0;
+    before = max(before, r0);
+    for (int i = 0; i < (t >> 5); ++i) before = max(before, warp_max[i]);
+#pragma unroll
+    for (int v = 0; v < V; ++v) row[t * V + v] = max(y[v], before);
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < V; ++v) r[v] = row[v * kThreads + t];
+  }
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    if (v * kThreads + t < cnt && (c[v] < 0 || c[v] >= K || r[v] < 0 || r[v] >= M)) {
+      atomicOr(bad, 2u);
+      c[v] = c[v] < 0 ? 0 : (c[v] >= K ? max(K - 1, 0) : c[v]);
+      r[v] = r[v] < 0 ? 0 : (r[v] >= M ? M - 1 : r[v]);
+    }
+    if (mode == 0 && v * kThreads + t < cnt) {
+      r[v] = __ldg(inv + r[v]);
+      c[v] = __ldg(inv + c[v]);
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    const int64_t e = t0 + v * kThreads + t;
+    if (e >= nnz) break;
+    if (mode != 1) {
+      key64[e] = (uint64_t)(uint32_t)r[v] << colbits | (uint32_t)c[v];
+    } else {
+      key32[e] = (uint32_t)c[v];
+      if (pair_pay) pair_pay[e] = make_uint2((uint32_t)r[v], __float_as_uint(x[v]));
+      else row_pay[e] = (uint32_t)r[v];
+    }
   }
 }
 
-// COO input: erow = src, with both coordinates checked against the shape.
-__global__ void k_coo_rows(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
-                           int32_t M, int32_t K, int64_t nnz, int32_t* __restrict__ erow,
-                           uint32_t* bad) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnz; e += stride) {
-    const int32_t r = src[e], c = dst[e];
-    if (r < 0 || r >= M || c < 0 || c >= K) atomicOr(bad, 2u);
-    erow[e] = r;
+// Writes the result where all pairs differ (out[0] = 1 where some do not): edge i is entry
+// i; the first edge of a row also fills the row pointer since the row before.
+template <bool kT>
+__global__ void __launch_bounds__(kThreads)
+    k_emit(const Sorted<kT> in, int64_t nnz, int32_t rows, int32_t* __restrict__ rowptr,
+           int32_t* __restrict__ col_out, float* __restrict__ val_out, uint32_t* equal) {
+  const int64_t t0 = (int64_t)blockIdx.x * kTile + threadIdx.x;
+  uint2 k[kTile / kThreads], p[kTile / kThreads];
+#pragma unroll
+  for (int v = 0; v < kTile / kThreads; ++v) {
+    const int64_t i = t0 + v * kThreads;
+    k[v] = i < nnz ? in.at(i) : make_uint2((uint32_t)rows, 0);
+    p[v] = i > 0 && i <= nnz ? in.at(i - 1) : make_uint2(0xffffffffu, 0);
+  }
+#pragma unroll
+  for (int v = 0; v < kTile / kThreads; ++v) {
+    const int64_t i = t0 + v * kThreads;
+    if (i > nnz) break;
+    for (uint32_t r = p[v].x + 1; r <= k[v].x; ++r) rowptr[r] = (int32_t)i;
+    if (i == nnz) break;
+    if (p[v].x == k[v].x && p[v].y == k[v].y) *equal = 1;
+    col_out[i] = (int32_t)k[v].y;
+    if (val_out) val_out[i] = in.value(i);
   }
 }
 
-// key = new_row << colbits | new_col. mode 0: permutation (inv applied to
-// row and column), mode 1: transpose, mode 2: identity (COO input).
-__global__ void k_keys(const int32_t* __restrict__ erow, const int32_t* __restrict__ col,
-                       const int32_t* __restrict__ inv, int64_t nnz, int mode, int colbits,
-                       int32_t M, int32_t K, uint64_t* __restrict__ keys,
-                       int32_t* __restrict__ ids) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnz; e += stride) {
-    int32_t r = erow[e], c = col[e];
-    r = r < 0 ? 0 : (r >= M ? M - 1 : r);   // inputs were checked; clamp keeps
-    c = c < 0 ? 0 : (c >= K ? K - 1 : c);   // a bad input in bounds until the error is read
-    uint64_t nr, nc;
-    if (mode == 0) { nr = (uint32_t)inv[r]; nc = (uint32_t)inv[c]; }
-    else if (mode == 1) { nr = (uint32_t)c; nc = (uint32_t)r; }
-    else { nr = (uint32_t)r; nc = (uint32_t)c; }
-    keys[e] = (nr << colbits) | nc;
-    ids[e] = (int32_t)e;
+template <bool kT>
+__global__ void k_flags(const Sorted<kT> in, int64_t nnz, int32_t* __restrict__ f) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= nnz; i += stride) {
+    bool first = i < nnz;
+    if (first && i > 0) {
+      const uint2 k = in.at(i), p = in.at(i - 1);
+      first = k.x != p.x || k.y != p.y;
+    }
+    f[i] = first;
   }
 }
 
-__global__ void k_flags(const uint64_t* __restrict__ keys, int64_t nnz, int32_t* __restrict__ f) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= nnz; i += stride)
-    f[i] = (i < nnz && (i == 0 || keys[i] != keys[i - 1])) ? 1 : 0;
-}
-
-// One thread per distinct pair: column, value sum (input CSR order) and row.
-__global__ void k_emit(const uint64_t* __restrict__ keys, const int32_t* __restrict__ ids,
-                       const int32_t* __restrict__ P, const float* __restrict__ val, int64_t nnz,
-                       int colbits, int32_t* __restrict__ col_out, float* __restrict__ val_out,
-                       int32_t* __restrict__ row_sorted) {
-  const uint64_t cmask = (1ull << colbits) - 1;
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nnz; i += stride) {
-    const uint64_t k = keys[i];
-    if (i > 0 && keys[i - 1] == k) continue;
+// The same with equal pairs merged: the first edge of each sums up the values (input CSR
+// order) and writes entry P[i].
+template <bool kT>
+__global__ void k_emit_merged(const Sorted<kT> in, const int32_t* __restrict__ P, int64_t nnz,
+                              int32_t rows, int32_t* __restrict__ rowptr,
+                              int32_t* __restrict__ col_out, float* __restrict__ val_out) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= nnz; i += stride) {
+    const uint2 k = i < nnz ? in.at(i) : make_uint2((uint32_t)rows, 0);
+    const uint2 p = i > 0 ? in.at(i - 1) : make_uint2(0xffffffffu, 0);
+    if (i > 0 && p.x == k.x && p.y == k.y) continue;
     const int32_t o = P[i];
-    col_out[o] = (int32_t)(k & cmask);
-    row_sorted[o] = (int32_t)(k >> colbits);
+    for (uint32_t r = p.x + 1; r <= k.x; ++r) rowptr[r] = o;
+    if (i == nnz) continue;
+    col_out[o] = (int32_t)k.y;
     if (val_out) {
-      float s = val ? val[ids[i]] : 1.0f;
-      for (int64_t j = i + 1; j < nnz && keys[j] == k; ++j) s += val ? val[ids[j]] : 1.0f;
+      float s = in.value(i);
+      for (int64_t j = i + 1; j < nnz; ++j) {
+        const uint2 q = in.at(j);
+        if (q.x != k.x || q.y != k.y) break;
+        s += in.value(j);
+      }
       val_out[o] = s;
     }
   }
 }
 
-// rowptr_out[r] = first output position of a row >= r.
-__global__ void k_rowptr(const int32_t* __restrict__ row_sorted, int64_t n, int32_t rows,
-                         int32_t* __restrict__ rowptr) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= n; i += stride) {
-    const int32_t prev = (i == 0) ? -1 : row_sorted[i - 1];
-    const int32_t cur = (i == n) ? rows : row_sorted[i];
-    for (int32_t r = prev + 1; r <= cur; ++r) rowptr[r] = (int32_t)i;
-  }
-}
-
 struct Layout {
-  size_t inv, seen, erow, keys_in, keys_out, ids_in, ids_out, flags, P, rsort, bad, sort, scan;
+  size_t inv, seen, keys_in, keys_out, pay_in, pay_out, bad, sort, scan;
   size_t total;
   int colbits, endbit;
 };
 
-Layout layout(int32_t rows_in, int32_t cols_in, int64_t nnz, int mode) {
+// Workspace of a mode; the flags and their sums of the compacting pass take the place of
+// the unsorted keys and what they carried (at least 4 bytes per edge each, and one more).
+Layout layout(int32_t rows_in, int32_t cols_in, int64_t nnz, int mode, bool with_val) {
   Layout L{};
   const int32_t rows_out = mode == 1 ? cols_in : rows_in;
   const int32_t cols_out = mode == 1 ? rows_in : cols_in;
-  L.colbits = bits_for((uint64_t)(cols_out > 0 ? cols_out : 1));
-  L.endbit = L.colbits + bits_for((uint64_t)(rows_out > 0 ? rows_out : 1));
+  const int rowbits = bits_for((uint64_t)(rows_out > 0 ? rows_out : 1));
+  L.colbits = mode == 1 ? 0 : bits_for((uint64_t)(cols_out > 0 ? cols_out : 1));
+  L.endbit = L.colbits + rowbits;
   const size_t n = (size_t)(nnz > 0 ? nnz : 1);
   const size_t m = (size_t)(rows_in > 0 ? rows_in : 1);
+  const size_t key = mode == 1 ? 4 : 8, pay = mode == 1 && with_val ? 8 : 4;
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
-  L.inv = take(m * 4);
-  L.seen = take(m * 4);
-  L.erow = take(n * 4);
-  L.keys_in = take(n * 8);
-  L.keys_out = take(n * 8);
-  L.ids_in = take(n * 4);
-  L.ids_out = take(n * 4);
-  L.flags = take((n + 1) * 4);
-  L.P = take((n + 1) * 4);
-  L.rsort = take(n * 4);
+  L.inv = take(mode == 0 ? m * 4 : 0);
+  L.seen = take(mode == 0 ? m * 4 : 0);
+  L.keys_in = take((n + 1) * key);
+  L.keys_out = take(n * key);
+  L.pay_in = take((n + 1) * pay);
+  L.pay_out = take(n * pay);
   L.bad = take(16);
   size_t s1 = 0, s2 = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, s1, (uint64_t*)nullptr, (uint64_t*)nullptr,
-                                  (int32_t*)nullptr, (int32_t*)nullptr, (int64_t)n, 0, L.endbit);
+  if (mode == 1 && with_val)
+    cub::DeviceRadixSort::SortPairs(nullptr, s1, (uint32_t*)nullptr, (uint32_t*)nullptr,
+                                    (uint64_t*)nullptr, (uint64_t*)nullptr, (int64_t)n, 0, L.endbit);
+  else if (mode == 1)
+    cub::DeviceRadixSort::SortPairs(nullptr, s1, (uint32_t*)nullptr, (uint32_t*)nullptr,
+                                    (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)n, 0, L.endbit);
+  else if (with_val)
+    cub::DeviceRadixSort::SortPairs(nullptr, s1, (uint64_t*)nullptr, (uint64_t*)nullptr,
+                                    (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)n, 0, L.endbit);
+  else
+    cub::DeviceRadixSort::SortKeys(nullptr, s1, (uint64_t*)nullptr, (uint64_t*)nullptr, (int64_t)n,
+                                   0, L.endbit);
   cub::DeviceScan::ExclusiveSum(nullptr, s2, (int32_t*)nullptr, (int32_t*)nullptr,
                                 (int64_t)n + 1);
   L.sort = take(s1);
   L.scan = take(s2);
   L.total = off;
   return L;
+}
+
+// From the sorted edges to the result; reads the input's error word on the way.
+template <bool kT>
+dtc_status emit(const Sorted<kT>& in, int64_t nnz, int32_t rows_out, int32_t* rowptr_out,
+                int32_t* col_out, float* val_out, int32_t* flags, int32_t* P, uint32_t* bad,
+                void* scan, size_t scan_bytes, uint32_t* hbad, int64_t* nnz_out, cudaStream_t st) {
+  k_emit<kT><<<(unsigned)(nnz / kTile + 1), kThreads, 0, st>>>(in, nnz, rows_out, rowptr_out,
+                                                              col_out, val_out, bad + 1);
+  DTC_CUDA(cudaGetLastError());
+  DTC_CUDA(cudaMemcpyAsync(hbad, bad, 8, cudaMemcpyDeviceToHost, st));
+  DTC_CUDA(cudaStreamSynchronize(st));
+  *nnz_out = nnz;
+  if (hbad[0] || !hbad[1]) return DTC_OK;
+  k_flags<kT><<<grid_for(nnz + 1), kThreads, 0, st>>>(in, nnz, flags);
+  DTC_CUDA(cub::DeviceScan::ExclusiveSum(scan, scan_bytes, flags, P, nnz + 1, st));
+  k_emit_merged<kT><<<grid_for(nnz + 1), kThreads, 0, st>>>(in, P, nnz, rows_out, rowptr_out,
+                                                           col_out, val_out);
+  DTC_CUDA(cudaGetLastError());
+  int32_t hn = 0;
+  DTC_CUDA(cudaMemcpyAsync(&hn, P + nnz, 4, cudaMemcpyDeviceToHost, st));
+  DTC_CUDA(cudaStreamSynchronize(st));
+  *nnz_out = hn;
+  return DTC_OK;
 }
 
 dtc_status relabel(int mode, const int32_t* rowptr, const int32_t* col, const float* val,
@@ -192,7 +331,8 @@ dtc_status relabel(int mode, const int32_t* rowptr, const int32_t* col, const fl
   DTC_REQUIRE((rowptr || (mode == 2 && nnz == 0)) && rowptr_out, "null device pointer");
   DTC_REQUIRE(nnz == 0 || (col && col_out), "null device pointer");
   DTC_REQUIRE(mode != 0 || perm || M == 0, "perm is null");
-  const Layout L = layout(M, K, nnz, mode);
+  const bool with_val = val != nullptr && val_out != nullptr;
+  const Layout L = layout(M, K, nnz, mode, with_val);
   if (!ws || wsb < L.total) {
     set_error("relabel workspace too small");
     return DTC_ERR_WORKSPACE_TOO_SMALL;
@@ -200,35 +340,61 @@ dtc_status relabel(int mode, const int32_t* rowptr, const int32_t* col, const fl
   char* w = (char*)ws;
   int32_t* inv = (int32_t*)(w + L.inv);
   int32_t* seen = (int32_t*)(w + L.seen);
-  int32_t* erow = (int32_t*)(w + L.erow);
-  uint64_t* kin = (uint64_t*)(w + L.keys_in);
-  uint64_t* kout = (uint64_t*)(w + L.keys_out);
-  int32_t* iin = (int32_t*)(w + L.ids_in);
-  int32_t* iout = (int32_t*)(w + L.ids_out);
-  int32_t* flags = (int32_t*)(w + L.flags);
-  int32_t* P = (int32_t*)(w + L.P);
-  int32_t* rsort = (int32_t*)(w + L.rsort);
-  uint32_t* bad = (uint32_t*)(w + L.bad);
+  void *kin = w + L.keys_in, *kout = w + L.keys_out, *pin = w + L.pay_in, *pout = w + L.pay_out;
+  uint32_t* bad = (uint32_t*)(w + L.bad);  // error bits; 1 where two pairs are equal
   const int32_t rows_out = mode == 1 ? K : M;
-  DTC_CUDA(cudaMemsetAsync(bad, 0, 4, st));
+  DTC_CUDA(cudaMemsetAsync(bad, 0, 8, st));
   if (mode == 0 && M > 0) {
+    DTC_CUDA(cudaMemsetAsync(inv, 0, (size_t)M * 4, st));  // (in range for a bad perm too)
     DTC_CUDA(cudaMemsetAsync(seen, 0, (size_t)M * 4, st));
     k_invert<<<grid_for(M), kThreads, 0, st>>>(perm, M, inv, seen, bad);
   }
-  if (mode == 2) {
-    if (nnz > 0) k_coo_rows<<<grid_for(nnz), kThreads, 0, st>>>(rowptr, col, M, K, nnz, erow, bad);
-  } else if (M > 0) {
-    k_rows<<<grid_for(nnz > M ? nnz : (int64_t)M), kThreads, 0, st>>>(rowptr, col, M, K, nnz, erow,
-                                                                     bad);
+  if (M > 0) {
+    const int64_t tiles = (nnz + kTile - 1) / kTile;
+    const int64_t rows = mode == 2 ? 1 : std::min<int64_t>(((int64_t)M + kThreads - 1) / kThreads, 2048);
+    k_expand<<<(unsigned)std::max(tiles, rows), kThreads, 0, st>>>(
+        rowptr, col, val, inv, M, K, nnz, mode, L.colbits, (uint32_t*)kin, (uint64_t*)kin,
+        (uint32_t*)pin, mode == 1 && with_val ? (uint2*)pin : nullptr, bad);
+    DTC_CUDA(cudaGetLastError());
   }
-  uint32_t hbad = 0;
-  DTC_CUDA(cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, st));
-  DTC_CUDA(cudaStreamSynchronize(st));
-  if (hbad & 1u) {
+  uint32_t hbad[2] = {0, 0};
+  dtc_status s = DTC_OK;
+  if (nnz == 0) {
+    DTC_CUDA(cudaMemcpyAsync(hbad, bad, 4, cudaMemcpyDeviceToHost, st));
+    DTC_CUDA(cudaStreamSynchronize(st));
+  } else {
+    size_t sb = L.scan - L.sort;
+    const size_t cb = L.total - L.scan;
+    if (mode == 1 && with_val)
+      DTC_CUDA(cub::DeviceRadixSort::SortPairs(w + L.sort, sb, (uint32_t*)kin, (uint32_t*)kout,
+                                               (uint64_t*)pin, (uint64_t*)pout, nnz, 0, L.endbit, st));
+    else if (mode == 1)
+      DTC_CUDA(cub::DeviceRadixSort::SortPairs(w + L.sort, sb, (uint32_t*)kin, (uint32_t*)kout,
+                                               (uint32_t*)pin, (uint32_t*)pout, nnz, 0, L.endbit, st));
+    else if (with_val)
+      DTC_CUDA(cub::DeviceRadixSort::SortPairs(w + L.sort, sb, (uint64_t*)kin, (uint64_t*)kout,
+                                               (const uint32_t*)val, (uint32_t*)pout, nnz, 0,
+                                               L.endbit, st));
+    else
+      DTC_CUDA(cub::DeviceRadixSort::SortKeys(w + L.sort, sb, (uint64_t*)kin, (uint64_t*)kout, nnz, 0,
+                                              L.endbit, st));
+    if (mode == 1)
+      s = emit(Sorted<true>{(uint32_t*)kout, nullptr, (uint32_t*)pout,
+                            with_val ? (uint2*)pout : nullptr, nullptr, 0},
+               nnz, rows_out, rowptr_out, col_out, val_out, (int32_t*)kin, (int32_t*)pin, bad,
+               w + L.scan, cb, hbad, nnz_out, st);
+    else
+      s = emit(Sorted<false>{nullptr, (uint64_t*)kout, nullptr, nullptr,
+                             with_val ? (float*)pout : nullptr, L.colbits},
+               nnz, rows_out, rowptr_out, col_out, val_out, (int32_t*)kin, (int32_t*)pin, bad,
+               w + L.scan, cb, hbad, nnz_out, st);
+    if (s != DTC_OK) return s;
+  }
+  if (hbad[0] & 1u) {
     set_error("perm is not a permutation of [0, num_nodes)");
     return DTC_ERR_INVALID_ARGUMENT;
   }
-  if (hbad & 2u) {
+  if (hbad[0] & 2u) {
     set_error(mode == 2 ? "invalid COO (a coordinate out of range)"
                         : "invalid CSR (rowptr not monotone from 0 to nnz, or a column out of range)");
     return DTC_ERR_INVALID_ARGUMENT;
@@ -236,23 +402,7 @@ dtc_status relabel(int mode, const int32_t* rowptr, const int32_t* col, const fl
   if (nnz == 0) {
     DTC_CUDA(cudaMemsetAsync(rowptr_out, 0, ((size_t)rows_out + 1) * 4, st));
     *nnz_out = 0;
-    return DTC_OK;
   }
-  k_keys<<<grid_for(nnz), kThreads, 0, st>>>(erow, col, inv, nnz, mode, L.colbits, M, K, kin, iin);
-  size_t sb = L.scan - L.sort;
-  DTC_CUDA(cub::DeviceRadixSort::SortPairs(w + L.sort, sb, kin, kout, iin, iout, nnz, 0, L.endbit,
-                                           st));
-  k_flags<<<grid_for(nnz + 1), kThreads, 0, st>>>(kout, nnz, flags);
-  size_t cb = L.total - L.scan;
-  DTC_CUDA(cub::DeviceScan::ExclusiveSum(w + L.scan, cb, flags, P, nnz + 1, st));
-  int32_t hn = 0;
-  DTC_CUDA(cudaMemcpyAsync(&hn, P + nnz, 4, cudaMemcpyDeviceToHost, st));
-  k_emit<<<grid_for(nnz), kThreads, 0, st>>>(kout, iout, P, val, nnz, L.colbits, col_out, val_out,
-                                             rsort);
-  DTC_CUDA(cudaStreamSynchronize(st));
-  k_rowptr<<<grid_for((int64_t)hn + 1), kThreads, 0, st>>>(rsort, hn, rows_out, rowptr_out);
-  DTC_CUDA(cudaGetLastError());
-  *nnz_out = hn;
   return DTC_OK;
 }
 
@@ -267,9 +417,10 @@ dtc_status dtc_relabel_workspace_bytes(int32_t num_rows, int32_t num_cols, int64
                                        size_t* bytes) {
   DTC_REQUIRE(bytes != nullptr, "bytes is null");
   DTC_REQUIRE(num_rows >= 0 && num_cols >= 0 && nnz >= 0, "negative sizes");
-  // modes 0 and 2 share a layout
-  const Layout a = layout(num_rows, num_cols, nnz, 0), b = layout(num_rows, num_cols, nnz, 1);
-  *bytes = a.total > b.total ? a.total : b.total;
+  *bytes = 0;
+  for (int mode = 0; mode < 2; ++mode)  // (a COO input needs no more than a permutation)
+    for (bool with_val : {false, true})
+      *bytes = std::max(*bytes, layout(num_rows, num_cols, nnz, mode, with_val).total);
   return DTC_OK;
 }
 
