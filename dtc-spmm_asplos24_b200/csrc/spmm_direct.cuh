@@ -156,29 +156,64 @@ __device__ __forceinline__ void chunk_cuts(const DirectParams& p, int32_t k, int
   }
 }
 
-// Adds the pieces of every window that chunk boundaries cut to the first piece
-// (in C), in chunk order, and applies the epilogue: one CTA per boundary.
-__global__ void k_add_slots(const DirectParams p) {
-  const int32_t k = blockIdx.x + 1, lane = threadIdx.x & 31;
-  const int32_t c = chunk_start(p, k);
-  const int2 i = search2(p.rwo, 0, p.nwin, c + 1, 0, 0, 0, lane);
-  const Cut b = cut_at(p, c, i.x - 1, p.lmax);
-  if (!b.open) return;
-  const int32_t ws = __ldg(p.rwo + b.win), we = __ldg(p.rwo + b.win + 1);
-  if (k > 1 && chunk_start(p, k - 1) > ws) return;  // an earlier boundary owns the window
-  int32_t last = k;
-  while (last + 1 < p.G && chunk_start(p, last + 1) < we) ++last;
-  const int64_t row0 = (int64_t)b.win * p.H;
-  const int32_t rows = (int32_t)min((int64_t)p.H, p.M - row0);
-  const size_t tile = (size_t)p.H * p.N;
-  float* C = p.C + row0 * p.N;
-  for (int32_t x = threadIdx.x; x < rows * p.N; x += blockDim.x) {
-    float acc = C[x];
-    const float* s = p.slots + (size_t)k * tile + x;
-    for (int32_t j = k; j <= last; ++j, s += tile) acc += *s;
-    C[x] = finish(p, acc, x % p.N);
+// Adds the pieces of every window that chunk boundaries cut to the first piece (in C), in
+// chunk order, and applies the epilogue. A CTA looks at kAddCuts boundaries, a warp each
+// (most cut no window, and finding that out is a chain of dependent loads: with a CTA per
+// boundary it took 90 us for the 7615 of R-MAT 2^20 in 32-row windows, now 28), then all
+// its threads add up the windows found.
+constexpr int kAddThreads = 256, kAddCuts = 4;
+__global__ void __launch_bounds__(kAddThreads) k_add_slots(const DirectParams p) {
+  __shared__ int3 found[kAddCuts];  // window, first and last chunk; -1: none
+  const int32_t lane = threadIdx.x & 31, wr = threadIdx.x >> 5;
+  if (wr < kAddCuts) {
+    const int32_t k = blockIdx.x * kAddCuts + wr + 1;
+    int3 f = make_int3(-1, 0, 0);
+    if (k < p.G) {
+      const int32_t c = chunk_start(p, k);
+      const int2 i = search2(p.rwo, 0, p.nwin, c + 1, 0, 0, 0, lane);
+      const Cut b = cut_at(p, c, i.x - 1, p.lmax);
+      const int32_t ws = __ldg(p.rwo + b.win), we = __ldg(p.rwo + b.win + 1);
+      if (b.open && !(k > 1 && chunk_start(p, k - 1) > ws)) {  // else an earlier one has it
+        f = make_int3(b.win, k, k);
+        while (f.z + 1 < p.G && chunk_start(p, f.z + 1) < we) ++f.z;
+      }
+    }
+    if (lane == 0) found[wr] = f;
+  }
+  __syncthreads();
+  const int64_t tile = (int64_t)p.H * p.N;
+  const bool vec = p.N % 4 == 0 && (((uintptr_t)p.slots | (uintptr_t)p.C) & 15) == 0;
+  for (int u = 0; u < kAddCuts; ++u) {
+    const int3 f = found[u];
+    if (f.x < 0) continue;
+    const int64_t row0 = (int64_t)f.x * p.H;
+    const int32_t n = (int32_t)min((int64_t)p.H, p.M - row0) * p.N;
+    float* const C = p.C + row0 * p.N;
+    const float* const s = p.slots + f.y * tile;
+    if (vec) {
+      for (int32_t x = threadIdx.x * 4; x < n; x += kAddThreads * 4) {
+        float4 acc = *reinterpret_cast<const float4*>(C + x);
+#pragma unroll 4
+        for (int32_t j = 0; j <= f.z - f.y; ++j) {
+          const float4 v = __ldcs(reinterpret_cast<const float4*>(s + j * tile + x));
+          acc = make_float4(acc.x + v.x, acc.y + v.y, acc.z + v.z, acc.w + v.w);
+        }
+        const int32_t c = x % p.N;
+        *reinterpret_cast<float4*>(C + x) =
+            make_float4(finish(p, acc.x, c), finish(p, acc.y, c + 1), finish(p, acc.z, c + 2),
+                        finish(p, acc.w, c + 3));
+      }
+    } else {
+      for (int32_t x = threadIdx.x; x < n; x += kAddThreads) {
+        float acc = C[x];
+#pragma unroll 4
+        for (int32_t j = 0; j <= f.z - f.y; ++j) acc += __ldcs(s + j * tile + x);
+        C[x] = finish(p, acc, x % p.N);
+      }
+    }
   }
 }
+inline unsigned add_ctas(const DirectParams& p) { return (p.G - 1 + kAddCuts - 1) / kAddCuts; }
 
 // -------------------------------------------------------------- instructions
 // Copies to shared memory; `none`: zeros instead, the source is not read.
@@ -953,7 +988,7 @@ dtc_status launch(DirectParams& p, cudaStream_t st) {
   fn<<<grid, kNW * 32, smem, st>>>(p);
   DTC_CUDA(cudaGetLastError());
   if (p.slots && p.G > 1) {
-    k_add_slots<<<p.G - 1, 256, 0, st>>>(p);
+    k_add_slots<<<add_ctas(p), kAddThreads, 0, st>>>(p);
     DTC_CUDA(cudaGetLastError());
   }
   return DTC_OK;

@@ -487,7 +487,7 @@ dtc_status launch_umma(DirectParams& p, cudaStream_t st) {
   fn<<<grid, kUmmaThreads, S::kSmem, st>>>(p);
   DTC_CUDA(cudaGetLastError());
   if (p.slots && p.G > 1) {
-    k_add_slots<<<p.G - 1, 256, 0, st>>>(p);
+    k_add_slots<<<add_ctas(p), kAddThreads, 0, st>>>(p);
     DTC_CUDA(cudaGetLastError());
   }
   return DTC_OK;
