@@ -421,7 +421,7 @@ def run_batched(args):
     tune_s = time.perf_counter() - t0
     bs.capture()
     one_ms = timed(bs.run, args.steps, args.warmup)
-    # the same launch with one CTA per chunk (hardware block scheduler, no queue)
+    # the same launch without slots (a cut window's pieces all by its first CTA)
     bs.queue = False
     bs._alloc_ws()
     bs.capture()
@@ -457,8 +457,8 @@ def run_batched(args):
 # ----------------------------------------------------------- balance report
 def run_balance_report(args):
     """Per-CTA busy times (dtc_set_cta_timer) of one SpMM launch per schedule:
-    window mode vs strict balance, persistent CTAs on the chunk queue vs one
-    CTA per chunk; plain TF32 and the BF16X2 split form at window height 32."""
+    window mode vs strict balance, with a workspace slot per chunk and without;
+    plain TF32 and the BF16X2 split form at window height 32."""
     import torch
     from dtc_b200 import balance, metcf, tune, B_F32, B_BF16X2, PREC_TF32, PREC_SPLIT3
     torch.cuda.set_device(0)
@@ -481,15 +481,15 @@ def run_balance_report(args):
                                            out=out, workspace=ws if wsb else None)
                 for _ in range(3):
                     fn()
-                r = balance.cta_report(fn, capacity=max(grid, sms) + 8, device=dev)
-                rows[f"{form}_h32_mode{mode}_{'persistent' if queue else 'one-cta-per-chunk'}"] = r
+                r = balance.cta_report(fn, capacity=max(grid, sms, m.T // 400) + 8, device=dev)
+                rows[f"{form}_h32_mode{mode}_{'slots' if queue else 'no-slots'}"] = r
     line = {"metric": "per-CTA busy time of one SpMM launch (us)", "workload": name,
             "nnz": A.nnz, "T": m.T, "chunks": min(16 * sms, m.T), "schedules": rows}
     print(json.dumps(line), flush=True)
 
 
 def _queue_bytes(m, grid):
-    """Bytes of the chunk-queue region spmm_ex_workspace_bytes includes."""
+    """Bytes of the chunk slots spmm_ex_workspace_bytes includes."""
     from dtc_b200 import metcf
     return metcf.spmm_ex_workspace_bytes(m, 128, 0, grid)
 

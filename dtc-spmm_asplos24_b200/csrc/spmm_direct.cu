@@ -1,5 +1,6 @@
 // Host side of the TC-block SpMM (kernels in spmm_direct.cuh): argument checks,
 // chunk counts, workspace sizes, and the fp32 forms' kernels.
+#include <algorithm>
 #include "spmm_direct.cuh"
 
 namespace dtc {
@@ -51,20 +52,24 @@ dtc_status rowid_to_rwo(const int32_t* rowid, int64_t T, int32_t nwin, int32_t* 
   return DTC_OK;
 }
 
-// Chunks of the TC-block range when no workspace limits them: ranges of 8 to 192
-// blocks for each of kNW warps, about five rounds of resident CTAs. Where a chunk is
-// long (64 blocks per warp and more, 40 us), the last quarter of the blocks is cut four
-// times finer, so that the last CTAs to start are short: R-MAT 2^19, N = 128 on tcgen05
-// 1.10 -> 0.87 ms; at shorter chunks the extra boundaries cost more than they give
-// (clustered 2^17, N = 128: 0.19 -> 0.23 ms).
+// Chunks of the TC-block range when no workspace limits them, from the blocks per warp of
+// a CTA (q): three chunks per SM, one wave, until a chunk has kNW * 80 blocks, then that
+// size until there are 15 per SM, then up to kNW * 192 blocks. The last quarter of the
+// blocks is cut four times finer, so that the last CTAs to start are short (R-MAT 2^19,
+// N = 128 on tcgen05: 1.10 -> 0.87 ms), except in the smallest products. A chunk costs its
+// pipeline's start and, where it cuts a window, a piece in the workspace; too few leave SMs
+// idle. us with 15 alike per SM / this: 27-point stencil 40^3, BF16, 32-row windows 117 /
+// 69, uniform 23438 x 47 116 / 89 (16-row windows 116 / 75), R-MAT 2^15 133 / 94; R-MAT
+// 2^18 with the 15 per SM that it keeps 502, with 3 580.
 struct Chunks {
   int64_t g, g1;  // all chunks; those of the first three quarters (0: all alike)
 };
 Chunks chunks_of(int64_t T) {
-  int64_t q = T / ((int64_t)num_sms() * 12 * 5);
+  const int64_t sms = num_sms();
+  int64_t q = std::max(std::min<int64_t>(T / (sms * 12), 80), T / (sms * 60));
   q = q < 8 ? 8 : q > 192 ? 192 : q;
   const int64_t g = T / (q * kNW);
-  if (q < 64) return {g < 1 ? 1 : g, 0};
+  if (q < 16) return {g < 1 ? 1 : g, 0};
   return {g * 3 / 4 + g, g * 3 / 4};
 }
 int direct_chunks(int64_t T) { return (int)chunks_of(T).g; }

@@ -2,21 +2,19 @@
 //
 // The reference picks its schedule from a hand-written table per dataset and
 // N (scripts/DTCSpMM/run_DTC_SpMM.py:10-30: balance or not, vector width,
-// N split). Here the schedule knobs of the tcgen05 kernels are measured
-// instead, on the caller's own ME-TCF arrays and B:
-//   mode   0 = window-scheduled (windows never split), 1 = strict balance
-//          (windows longer than the per-CTA chunk are split; the chunk,
-//          ceil(T / grid) blocks, is the split threshold)
-//   waves  chunks = waves x SMs, pulled by one persistent CTA per SM from a
-//          device counter (more chunks even out skew at the price of more
-//          chunk boundaries); window mode also tries 32 and 64, balance mode,
-//          whose cut windows need partial tiles per chunk, stops at 16
-//   ntile  128-feature tiles per CTA (fewer tiles spread wide N over more CTAs)
+// N split). Here the schedules that a caller can name are measured instead, on
+// the caller's own ME-TCF arrays and B:
+//   mode   0 = window-scheduled, 1 = strict balance
+//   waves  the workspace's partial tiles, waves x SMs (balance mode stops at 16)
+//   ntile  128-feature tiles per CTA
+// The kernels cut the blocks into chunks of their own (spmm_run): with the whole
+// workspace the candidates run alike and differ by noise; with balance mode's
+// required bytes alone, `waves` bounds the chunks.
 // Each candidate runs once untimed and `reps` times between CUDA events on the
 // caller's stream; the mean is its time. Candidates change neither the B form
 // nor the product precision, only how fp32 partial sums are grouped; each
-// candidate's result is bitwise reproducible (window mode writes every C
-// element once, balance mode reduces its partial tiles in fixed order).
+// candidate's result is bitwise reproducible (the pieces of a cut window are
+// added in a fixed order).
 #include <vector>
 #include "impl.h"
 

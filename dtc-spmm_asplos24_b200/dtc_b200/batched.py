@@ -5,12 +5,12 @@ whole number of 16-row windows, so no row window mixes two matrices and the
 ME-TCF of the stack is exactly the union of the per-matrix ME-TCFs. One
 conversion covers the whole batch, and one launch multiplies every matrix
 with its own dense operand: the batch's TC blocks are cut into chunks
-(contiguous block ranges, snapped to row windows in window mode) and one CTA
-per SM pulls chunk ids from a device counter, the global work queue, until
-the batch is done (queue=False runs one CTA per chunk instead, handed out by
-the hardware block scheduler). The launch (plus its small chunk-table kernel
-and, in balance mode, its partial-tile reduction) can be captured in a CUDA
-graph and replayed.
+(contiguous block ranges, cut inside a row window only where one is longer
+than a chunk), one CTA each, handed out by the hardware block scheduler.
+The pieces of cut windows go to the workspace and a small kernel adds them
+(queue=False leaves that workspace out: the CTA of a window's first piece runs
+its other pieces too; the bits are the same). Both launches can be captured in
+a CUDA graph and replayed.
 
 There is no counterpart in the reference, which multiplies one matrix per
 call (DTC-SpMM/DTCSpMM.cpp:117-178).
@@ -95,7 +95,7 @@ class BatchedSpMM:
 
     def _alloc_ws(self):
         """Workspace of the current schedule: partial tiles (balance mode) and,
-        with queue=True, the chunk-queue region after them."""
+        with queue=True, a slot per chunk after them."""
         full = _m.spmm_ex_workspace_bytes(self.m, self.N, self.mode, self.grid)
         q = _m.spmm_ex_workspace_bytes(self.m, self.N, 0, self.grid)
         wsb = full if self.queue else full - q
@@ -104,8 +104,8 @@ class BatchedSpMM:
     def autotune(self, heights=(16, 32), reps=3):
         """Exhaustive schedule search for this batch (dtc_autotune): window height
         (16 or 32; a 32-row window may span two stacked matrices, which only adds
-        distinct columns to it), strict balance or window mode, the CTA count
-        (which sets the split threshold, blocks per CTA) and the N-tiles per CTA.
+        distinct columns to it), strict balance or window mode, the chunk count
+        and the N-tiles (hints: the kernels cut by the block count alone).
         Keeps the fastest and returns {height: best Schedule}."""
         from . import tune
         from ._lib import B_F32

@@ -168,7 +168,8 @@ def spmm_ex_launches(m: METCF, mode=0, grid=0, queue=True):
     if m.T == 0:
         return 0
     sms = torch.cuda.get_device_properties(m.RowWindowOffset.device).multi_processor_count
-    q = min(max(m.T // (sms * 60), 8), 192)  # blocks per range, 4 ranges per chunk
+    # blocks per range, 4 ranges per chunk (chunks_of in spmm_direct.cu)
+    q = min(max(min(m.T // (sms * 12), 80), m.T // (sms * 60), 8), 192)
     return 1 + (1 if (queue or mode == 1) and m.T // (4 * q) > 1 else 0)
 
 
