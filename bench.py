@@ -773,7 +773,11 @@ def main():
         tuned_fn()
         torch.cuda.synchronize()
         errs[tuned] = accuracy_vs_fp64(At, Bt.cpu().numpy(), N, out_t.cpu().numpy())
-        errs["e2e"] = accuracy_vs_fp64(A, Bh, N, Cpin.numpy())
+        C_e2e = Cpin.numpy()
+        if perm is not None:  # the pipeline's C has the reordered rows
+            C_e2e = np.empty_like(C_e2e)
+            C_e2e[perm.cpu().numpy()] = Cpin.numpy()
+        errs["e2e"] = accuracy_vs_fp64(A, Bh, N, C_e2e)
 
     if rank == 0:
         dtype = {"tf32": "tf32", "split24x4": "bf16 split, 4-term (SPLIT24 B), fp32 accumulate",

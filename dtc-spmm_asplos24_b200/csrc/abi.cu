@@ -65,8 +65,14 @@ float* slot_region(void* ws, size_t bytes, size_t offset, int64_t T, int32_t N, 
   *n = 0;
   if (!ws || T <= 0) return nullptr;
   char* q = (char*)ws + offset;
-  if (((uintptr_t)q & 15) != 0 || offset + direct_slots_bytes(T, N, H) > bytes) return nullptr;
-  *n = direct_chunks(T);
+  if (((uintptr_t)q & 15) != 0 || offset >= bytes) return nullptr;
+  // fewer slots than chunks: as many chunks as there are slots (spmm_run), from one per SM
+  // on. R-MAT 2^20, N = 128, a workspace for 32 tiles per SM: 1.5 ms, 8.7 without slots (the
+  // CTA of a long window's first piece runs all the others).
+  const int64_t fit = (int64_t)((bytes - offset) / ((size_t)H * N * sizeof(float)));
+  const int64_t want = direct_chunks(T);
+  if (fit < want && fit < num_sms()) return nullptr;
+  *n = fit < want ? fit : want;
   return (float*)q;
 }
 
@@ -227,7 +233,7 @@ dtc_status spmm_ex_impl(const int32_t* rwo, const uint8_t* tile, const int32_t* 
   if (n < direct_chunks(T)) {  // the second region, where the caller gave it, holds every chunk
     int64_t more = 0;
     float* q = slot_region(ws, wsb, part_bytes, T, N, H, &more);
-    if (q) {
+    if (more > n) {
       slots = q;
       n = more;
     }

@@ -23,7 +23,8 @@ dtc_status spmm_run(const int32_t* rwo, const uint8_t* tile, const int32_t* toff
 // bytes of that many slots.
 int direct_chunks(int64_t T);
 size_t direct_slots_bytes(int64_t T, int32_t N, int H);
-// The slots at byte `offset` of a caller workspace (null when they do not fit).
+// The slots at byte `offset` of a caller workspace: `n` of them, a slot per chunk or, from
+// one per SM on, as many as fit; null when those do not fit.
 float* slot_region(void* ws, size_t bytes, size_t offset, int64_t T, int32_t N, int H, int64_t* n);
 // Tiles of the partials region that strict balance requires for `grid` chunks
 // (0 = 16 per SM), and its bytes.

@@ -25,6 +25,11 @@ def test_chunk_rule(cuda, rows, N):
     one = metcf.spmm_ex(m, [Bd], B_F32, N, PREC_TF32, workspace=ws)
     two = metcf.spmm_ex(m, [Bd], B_F32, N, PREC_TF32, workspace=ws[:1])
     assert torch.equal(one, two)
+    slot = 16 * N * 4  # (fewer slots: fewer chunks; less than one per SM: none)
+    few = [metcf.spmm_ex(m, [Bd], B_F32, N, PREC_TF32, workspace=ws[:n * slot])
+           for n in (sms - 1, sms, sms)]
+    assert torch.equal(one, few[0]) and torch.equal(few[1], few[2])
     ref = O.spmm_f64(A.rowptr, A.col, A.val, A.M, B)
     bound = O.spmm_absbound_f64(A.rowptr, A.col, A.val, A.M, B)
-    assert (np.abs(one.cpu().numpy() - ref) <= 2.0 ** -9 * bound + 1e-6).all()
+    for C in (one, few[1]):
+        assert (np.abs(C.cpu().numpy() - ref) <= 2.0 ** -9 * bound + 1e-6).all()
