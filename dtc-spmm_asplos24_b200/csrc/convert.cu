@@ -102,7 +102,8 @@ __device__ __forceinline__ int32_t many_listed(const int32_t* count, int32_t roo
   return (int32_t)min((int64_t)__ldg(count) + __ldg(count + 1), (int64_t)room);
 }
 
-// Lists the windows of more than mid_cap edges (mid_list) and of more than `cap`, those of more than kHuge from the front and
+// Lists the windows of more than mid_cap edges (mid_list) and of more than `cap`, those of
+// more than kHuge from the front and
 // the others from the back (count[0], count[1]); with `bad`, checks the row pointer
 // (rowptr[0] == 0, non-decreasing, rowptr[M] == nnz) and sets its bits. With `rwo`
 // (phase 2), also lists their units of `unit` blocks: (window, first block).
