@@ -11,7 +11,9 @@ constexpr int kWavesPerSm = 16;  // chunks per SM of the required partials regio
 // rwo[w] = first block of window w, from the sorted window id of every block.
 // Ids come from the caller: an id outside [0, nwin) or a descending pair is
 // reported through kErrBadIndex, and the written range is clamped to the
-// (nwin + 1)-entry table, so a bad id never writes outside it.
+// (nwin + 1)-entry table, so a bad id never writes outside it. The table starts at 0
+// and ends at T whatever the ids are: the kernels rely on it to find a window that
+// holds a given block (cut_at).
 __global__ void k_rowid_to_rwo(const int32_t* __restrict__ rowid, int64_t T, int32_t nwin,
                                int32_t* __restrict__ rwo, uint32_t* err) {
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -22,7 +24,9 @@ __global__ void k_rowid_to_rwo(const int32_t* __restrict__ rowid, int64_t T, int
     if (bad) atomicOr(err, kErrBadIndex);
     const int32_t lo = prev < -1 ? -1 : (prev > nwin ? nwin : prev);
     const int32_t hi = cur < -1 ? -1 : (cur > nwin ? nwin : cur);
-    for (int32_t w = lo + 1; w <= hi; ++w) rwo[w] = (int32_t)b;
+    for (int32_t w = max(lo + 1, 1); w <= min(hi, nwin - 1); ++w) rwo[w] = (int32_t)b;
+    if (b == 0) rwo[0] = 0;
+    if (b == T) rwo[nwin] = (int32_t)T;
   }
 }
 

@@ -123,8 +123,12 @@ struct Cut {
   bool open;
 };
 
-__device__ __forceinline__ Cut cut_at(const DirectParams& p, int32_t c, int32_t w, int32_t most) {
-  // (offsets made from a caller's invalid window ids stay inside the arrays)
+// The cut of block c, where `i` is the answer of a search for c + 1. A table that starts at 0
+// and ends at T holds c in window i - 1 even where it is not ascending (made from a caller's
+// invalid window ids): the search has seen rwo[i - 1] <= c < rwo[i]. The clamps are for a table
+// that the caller made.
+__device__ __forceinline__ Cut cut_at(const DirectParams& p, int32_t c, int32_t i, int32_t most) {
+  const int32_t w = max(i - 1, 0);
   const int32_t ws = min(max(__ldg(p.rwo + w), 0), p.T), we = __ldg(p.rwo + w + 1);
   Cut b;
   b.win = w;
@@ -146,13 +150,13 @@ __device__ __forceinline__ void chunk_cuts(const DirectParams& p, int32_t k, int
                                            Cut& b1) {
   const int32_t x0 = chunk_start(p, k), x1 = chunk_start(p, k + 1);
   const int2 i = search2(p.rwo, 0, p.nwin, x0 + 1, 0, p.nwin, min(x1, p.T - 1) + 1, lane);
-  b0 = cut_at(p, x0, i.x - 1, p.lmax);
+  b0 = cut_at(p, x0, i.x, p.lmax);
   if (x1 >= p.T) {
     b1.pos = p.T;
-    b1.win = i.y - 1;
+    b1.win = max(i.y - 1, 0);
     b1.open = false;
   } else {
-    b1 = cut_at(p, x1, i.y - 1, p.lmax);
+    b1 = cut_at(p, x1, i.y, p.lmax);
   }
 }
 
@@ -171,7 +175,7 @@ __global__ void __launch_bounds__(kAddThreads) k_add_slots(const DirectParams p)
     if (k < p.G) {
       const int32_t c = chunk_start(p, k);
       const int2 i = search2(p.rwo, 0, p.nwin, c + 1, 0, 0, 0, lane);
-      const Cut b = cut_at(p, c, i.x - 1, p.lmax);
+      const Cut b = cut_at(p, c, i.x, p.lmax);
       const int32_t ws = __ldg(p.rwo + b.win), we = __ldg(p.rwo + b.win + 1);
       if (b.open && !(k > 1 && chunk_start(p, k - 1) > ws)) {  // else an earlier one has it
         f = make_int3(b.win, k, k);
@@ -485,7 +489,8 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
     chunk_cuts(p, k, lane, c0, c1);
     if (seq && k == (int32_t)blockIdx.x && c0.open) break;  // an earlier CTA runs this piece
     const uint32_t mark = (uint32_t)(k - (int32_t)blockIdx.x) + 1;
-    const int32_t len = c1.pos - c0.pos;
+    // (c1.win < c0.win: only with invalid window ids)
+    const int32_t len = c1.win < c0.win ? 0 : c1.pos - c0.pos;
     const int nr = min(nranges, max(1, len >> 2));  // ranges of at least 4 blocks
     if (len > 0 && wr < nr && col0 < p.N) {
       // this warp's range
@@ -494,8 +499,8 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
       const int32_t most = max(len / nr / 2, 1);
       const int32_t wtop = min(c1.win + 1, p.nwin);
       const int2 si = search2(p.rwo, c0.win, wtop, x0 + 1, c0.win, wtop, min(x1, p.T - 1) + 1, lane);
-      const Cut r0 = wr == 0 ? c0 : cut_at(p, x0, si.x - 1, most);
-      const Cut r1 = wr == nr - 1 ? c1 : cut_at(p, x1, si.y - 1, most);
+      const Cut r0 = wr == 0 ? c0 : cut_at(p, x0, si.x, most);
+      const Cut r1 = wr == nr - 1 ? c1 : cut_at(p, x1, si.y, most);
       const int32_t nblk = r1.pos - r0.pos;
       if (nblk > 0) {
         const int32_t nst = nblk * SUB;
@@ -831,22 +836,22 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
             case 0:
               step(std::integral_constant<int, 0>{});
               phase = 1;
-              if (st == run) break;
+              if (st >= run) break;
               [[fallthrough]];
             case 1:
               step(std::integral_constant<int, 1>{});
               phase = 2;
-              if (st == run) break;
+              if (st >= run) break;
               [[fallthrough]];
             case 2:
               step(std::integral_constant<int, 2>{});
               phase = 3;
-              if (st == run) break;
+              if (st >= run) break;
               [[fallthrough]];
             default:
               step(std::integral_constant<int, 3>{});
               phase = 0;
-              if (st != run) continue;
+              if (st < run) continue;
           }
           if (wend > nblk) break;
           {  // the window is complete
@@ -947,6 +952,10 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
           }
         }
       }
+      // a warp that handed nothing over: its left neighbour waits for it all the same where
+      // invalid window ids make a window run on into a range that does not start inside it
+      __syncwarp();
+      if (lane == 0) flags[warp] = mark;
     }
     if (!seq || !c1.open) break;
     __syncthreads();  // the next piece adds to what this one wrote

@@ -72,7 +72,7 @@ struct WindowWalk {
       : p(p_), lane(lane_), w(w0), wb(w0), base(base_), nblk(nblk_) {
     ends = load(wb);
     ends_n = load(wb + 32);
-    end = __shfl_sync(0xffffffffu, ends, 0) - base;
+    end = max(__shfl_sync(0xffffffffu, ends, 0) - base, 1);  // (less: only with invalid offsets)
   }
   // On to the next window with blocks; `empty` is called for each one without.
   template <typename F>
