@@ -61,11 +61,19 @@ uint64_t* cta_timer_buffer(int32_t* capacity) {
   return g_timer[d];
 }
 
+float* aligned_tiles(void* region, int32_t N, int64_t* n) {
+  const uintptr_t a = (uintptr_t)region;
+  if (N % 4 != 0 || (a & 15) == 0) return (float*)region;
+  --*n;
+  return *n > 0 ? (float*)((a + 15) & ~(uintptr_t)15) : nullptr;
+}
+
 float* slot_region(void* ws, size_t bytes, size_t offset, int64_t T, int32_t N, int H, int64_t* n) {
   *n = 0;
   if (!ws || T <= 0) return nullptr;
+  offset += (size_t)(-((intptr_t)ws + (intptr_t)offset) & 15);
+  if (offset >= bytes) return nullptr;
   char* q = (char*)ws + offset;
-  if (((uintptr_t)q & 15) != 0 || offset >= bytes) return nullptr;
   // fewer slots than chunks: as many chunks as there are slots (spmm_run), from one per SM
   // on. R-MAT 2^20, N = 128, a workspace for 32 tiles per SM: 1.5 ms, 8.7 without slots (the
   // CTA of a long window's first piece runs all the others).
@@ -186,14 +194,16 @@ dtc_status dtc_spmm_balance(const int32_t* d_tcblockRowid, const uint8_t* d_tile
     set_error("balance workspace too small (dtc_spmm_balance_workspace_bytes)");
     return DTC_ERR_WORKSPACE_TOO_SMALL;
   }
+  DTC_REQUIRE(((uintptr_t)d_workspace & 3) == 0, "the workspace must be 4-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
   int32_t* rwo = (int32_t*)d_workspace;
-  float* part = (float*)((char*)d_workspace + rwo_bytes);
+  int64_t tiles = spmm_partials(num_blocks, 0);
+  float* part = aligned_tiles((char*)d_workspace + rwo_bytes, N, &tiles);
   dtc_status s = rowid_to_rwo(d_tcblockRowid, num_blocks, nwin, rwo, st);
   if (s != DTC_OK) return s;
   return spmm_run(rwo, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues, num_nodes, nwin,
                   num_blocks, DTC_B_F32, d_B, nullptr, N, DTC_PREC_TF32, d_C, st, Epilogue{}, 16, 8,
-                  part, spmm_partials(num_blocks, 0));
+                  part, tiles);
 }
 
 dtc_status dtc_spmm_ex_workspace_bytes(int32_t num_nodes, int64_t num_blocks, int32_t N,
@@ -229,7 +239,8 @@ dtc_status spmm_ex_impl(const int32_t* rwo, const uint8_t* tile, const int32_t* 
     return DTC_ERR_WORKSPACE_TOO_SMALL;
   }
   int64_t n = mode == 1 ? spmm_partials(T, grid) : 0;
-  float* slots = mode == 1 ? (float*)ws : nullptr;
+  DTC_REQUIRE(mode == 0 || ((uintptr_t)ws & 3) == 0, "the workspace must be 4-byte aligned");
+  float* slots = mode == 1 ? aligned_tiles(ws, N, &n) : nullptr;
   if (n < direct_chunks(T)) {  // the second region, where the caller gave it, holds every chunk
     int64_t more = 0;
     float* q = slot_region(ws, wsb, part_bytes, T, N, H, &more);

@@ -23,6 +23,9 @@ dtc_status spmm_run(const int32_t* rwo, const uint8_t* tile, const int32_t* toff
 // bytes of that many slots.
 int direct_chunks(int64_t T);
 size_t direct_slots_bytes(int64_t T, int32_t N, int H);
+// The tiles of a required region of `n` of them from its first 16-byte boundary on (the widths
+// that are multiples of 4 are written 8 and 16 bytes at a time): one less off that boundary.
+float* aligned_tiles(void* region, int32_t N, int64_t* n);
 // The slots at byte `offset` of a caller workspace: `n` of them, a slot per chunk or, from
 // one per SM on, as many as fit; null when those do not fit.
 float* slot_region(void* ws, size_t bytes, size_t offset, int64_t T, int32_t N, int H, int64_t* n);
