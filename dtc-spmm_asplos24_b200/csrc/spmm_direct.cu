@@ -30,6 +30,12 @@ __global__ void k_rowid_to_rwo(const int32_t* __restrict__ rowid, int64_t T, int
   }
 }
 
+// C of a matrix without blocks: the epilogue of 0, a warp per row.
+__global__ void __launch_bounds__(256) k_no_blocks(const DirectParams p) {
+  for (int64_t r = blockIdx.x * 8ll + threadIdx.x / 32; r < p.M; r += gridDim.x * 8ll)
+    for (int f = threadIdx.x % 32; f < p.N; f += 32) p.C[r * p.N + f] = finish(p, 0.0f, f);
+}
+
 }  // namespace
 
 dtc_status direct_f32(DirectParams& p, int W, cudaStream_t st) {
@@ -115,17 +121,22 @@ dtc_status spmm_run(const int32_t* rwo, const uint8_t* tile, const int32_t* toff
     return DTC_ERR_UNSUPPORTED;
   }
   if (M == 0) return DTC_OK;
-  if (T == 0) {
-    DTC_CUDA(cudaMemsetAsync(C, 0, (size_t)M * N * sizeof(float), st));
-    return DTC_OK;
-  }
-  if (N % 4 == 0) DTC_REQUIRE(((uintptr_t)C & 15) == 0, "C must be 16-byte aligned");
   DirectParams p{};
   p.rwo = rwo; p.toff = toff; p.s2x = s2x; p.tile = tile; p.vals = vals;
   p.b0 = b0; p.b1 = b1; p.C = C; p.err = device_error_word();
   p.stamps = cta_timer_buffer(&p.stamp_cap);
   p.bias = epi.bias; p.relu = epi.relu;
   p.M = M; p.nwin = nwin; p.N = N; p.H = H; p.T = (int32_t)T;
+  if (T == 0) {
+    if (epi.bias) {
+      k_no_blocks<<<(unsigned)std::min<int64_t>(((int64_t)M + 7) / 8, 8 * num_sms()), 256, 0, st>>>(p);
+      DTC_CUDA(cudaGetLastError());
+    } else {  // (ReLU of 0 is 0)
+      DTC_CUDA(cudaMemsetAsync(C, 0, (size_t)M * N * sizeof(float), st));
+    }
+    return DTC_OK;
+  }
+  if (N % 4 == 0) DTC_REQUIRE(((uintptr_t)C & 15) == 0, "C must be 16-byte aligned");
   const Chunks c = chunks_of(T);
   const bool limited = slots && c.g > nslots;
   p.slots = slots;
