@@ -182,12 +182,14 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// Writes the result where all pairs differ (out[0] = 1 where some do not): edge i is entry
-// i; the first edge of a row also fills the row pointer since the row before.
+// Writes the result where all pairs differ (bad[1] = 1 where some do not): edge i is entry
+// i; the first edge of a row also fills the row pointer since the row before. Writes nothing
+// for an invalid input (bad[0]), whose call leaves the outputs as they are.
 template <bool kT>
 __global__ void __launch_bounds__(kThreads)
     k_emit(const Sorted<kT> in, int64_t nnz, int32_t rows, int32_t* __restrict__ rowptr,
-           int32_t* __restrict__ col_out, float* __restrict__ val_out, uint32_t* equal) {
+           int32_t* __restrict__ col_out, float* __restrict__ val_out, uint32_t* bad) {
+  if (bad[0]) return;
   const int64_t t0 = (int64_t)blockIdx.x * kTile + threadIdx.x;
   uint2 k[kTile / kThreads], p[kTile / kThreads];
 #pragma unroll
@@ -202,7 +204,7 @@ __global__ void __launch_bounds__(kThreads)
     if (i > nnz) break;
     for (uint32_t r = p[v].x + 1; r <= k[v].x; ++r) rowptr[r] = (int32_t)i;
     if (i == nnz) break;
-    if (p[v].x == k[v].x && p[v].y == k[v].y) *equal = 1;
+    if (p[v].x == k[v].x && p[v].y == k[v].y) bad[1] = 1;
     col_out[i] = (int32_t)k[v].y;
     if (val_out) val_out[i] = in.value(i);
   }
@@ -302,12 +304,13 @@ dtc_status emit(const Sorted<kT>& in, int64_t nnz, int32_t rows_out, int32_t* ro
                 int32_t* col_out, float* val_out, int32_t* flags, int32_t* P, uint32_t* bad,
                 void* scan, size_t scan_bytes, uint32_t* hbad, int64_t* nnz_out, cudaStream_t st) {
   k_emit<kT><<<(unsigned)(nnz / kTile + 1), kThreads, 0, st>>>(in, nnz, rows_out, rowptr_out,
-                                                              col_out, val_out, bad + 1);
+                                                              col_out, val_out, bad);
   DTC_CUDA(cudaGetLastError());
   DTC_CUDA(cudaMemcpyAsync(hbad, bad, 8, cudaMemcpyDeviceToHost, st));
   DTC_CUDA(cudaStreamSynchronize(st));
+  if (hbad[0]) return DTC_OK;  // (the caller reports it)
   *nnz_out = nnz;
-  if (hbad[0] || !hbad[1]) return DTC_OK;
+  if (!hbad[1]) return DTC_OK;
   k_flags<kT><<<grid_for(nnz + 1), kThreads, 0, st>>>(in, nnz, flags);
   DTC_CUDA(cub::DeviceScan::ExclusiveSum(scan, scan_bytes, flags, P, nnz + 1, st));
   k_emit_merged<kT><<<grid_for(nnz + 1), kThreads, 0, st>>>(in, P, nnz, rows_out, rowptr_out,

@@ -46,3 +46,43 @@ def test_tiles(cuda, M, nnz, with_values, equal):
     square = np.concatenate([rowptr, np.full(K - M, nnz, np.int32)])
     perm = np.random.default_rng(2).permutation(K).astype(np.int32)
     same(metcf.permute_csr(g(square), g(c), g(v), g(perm)), O.permute_csr(square, c, v, perm))
+
+
+@pytest.mark.parametrize("fault", ["perm", "rowptr", "col", "row", "col_coo"])
+def test_outputs_of_a_refused_call_stay_as_they_are(cuda, fault):
+    import ctypes as C
+    import torch
+    from dtc_b200 import _lib
+    from dtc_b200.metcf import _ptr, _stream
+    M, nnz = 3000, 20000
+    rowptr, r, c, val = _csr(M, M, nnz, False, seed=4)
+    perm = np.arange(M, dtype=np.int32)
+    if fault == "perm":
+        perm[5] = perm[6]
+    elif fault == "rowptr":
+        rowptr[M // 2] = nnz + 1
+    elif fault == "row":
+        r[77] = M
+    else:
+        c[nnz - 1] = -1
+    g = lambda x: torch.from_numpy(x).cuda()
+    L = _lib.lib()
+    b = C.c_size_t()
+    assert L.dtc_relabel_workspace_bytes(M, M, nnz, C.byref(b)) == 0
+    ws = torch.empty(b.value, dtype=torch.uint8, device="cuda")
+    rp = torch.full((M + 1,), -5, dtype=torch.int32, device="cuda")
+    co = torch.full((nnz,), -5, dtype=torch.int32, device="cuda")
+    vo = torch.full((nnz,), -5.0, device="cuda")
+    n = C.c_int64(-5)
+    inputs = [g(rowptr), g(c), g(val), g(perm), g(r)]
+    p = [_ptr(t) for t in inputs]
+    outs = [_ptr(rp), _ptr(co), _ptr(vo), C.byref(n), _ptr(ws), b.value, _stream()]
+    calls = {"perm": lambda: L.dtc_permute_csr(*p[:3], M, nnz, p[3], *outs),
+             "csr": lambda: L.dtc_transpose_csr(*p[:3], M, M, nnz, *outs),
+             "coo": lambda: L.dtc_coo_to_csr(p[4], p[1], p[2], M, M, nnz, *outs)}
+    for name in {"perm": ["perm"], "rowptr": ["perm", "csr"], "col": ["perm", "csr"], "row": ["coo"],
+                 "col_coo": ["coo"]}[fault]:
+        assert calls[name]() == 1
+        assert n.value == -5
+        for t in (rp, co, vo):
+            assert (t == -5).all()
