@@ -54,7 +54,7 @@ def test_outputs_of_a_refused_call_stay_as_they_are(cuda, fault):
     import torch
     from dtc_b200 import _lib
     from dtc_b200.metcf import _ptr, _stream
-    M, nnz = 3000, 20000
+    M, nnz = 30000, 20000
     rowptr, r, c, val = _csr(M, M, nnz, False, seed=4)
     perm = np.arange(M, dtype=np.int32)
     if fault == "perm":
