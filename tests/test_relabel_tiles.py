@@ -86,3 +86,31 @@ def test_outputs_of_a_refused_call_stay_as_they_are(cuda, fault):
         assert n.value == -5
         for t in (rp, co, vo):
             assert (t == -5).all()
+
+
+@pytest.mark.parametrize("equal", [False, True])
+@pytest.mark.parametrize("first,gap,last", [(0, 33, 0), (5, 32, 1), (1, 5000, 300), (70000, 1, 70000)])
+def test_long_runs_of_empty_rows(cuda, first, gap, last, equal):
+    import torch
+    from dtc_b200 import dataset, metcf
+    # 3000 entries in two groups of rows, with runs of empty rows before, between and after them
+    rng = np.random.default_rng(gap)
+    rows = 600 + first + gap + last
+    r = first + rng.integers(0, 300, 3000)
+    r[1500:] += 300 + gap
+    c = rng.integers(0, 40 if equal else 1 << 20, 3000)
+    if not equal:
+        c = (c // 3000 * 3000 + np.arange(3000)).astype(np.int64)
+    val = rng.standard_normal(3000).astype(np.float32)
+    got = dataset.coo_to_csr(r.astype(np.int32), c.astype(np.int32), rows, 1 << 21, val=val)
+    exp = O._coo_to_csr(r.astype(np.int32), c.astype(np.int32), val, rows, 1 << 21)
+    for a, b in zip(got, exp):
+        np.testing.assert_array_equal(a.cpu().numpy(), b)
+    # the same rows as the columns of a matrix to transpose
+    o = np.argsort(c, kind="stable")
+    rp = np.searchsorted(c[o], np.arange((1 << 21) + 1)).astype(np.int32)
+    g = lambda x: torch.from_numpy(x).cuda()
+    got = metcf.transpose_csr(g(rp), g(r[o].astype(np.int32)), g(val[o]), rows)
+    exp = O.transpose_csr(rp, r[o].astype(np.int32), val[o], rows)
+    for a, b in zip(got, exp):
+        np.testing.assert_array_equal(a.cpu().numpy(), b)
