@@ -11,7 +11,7 @@
 // (32-bit keys, three passes for 2^19 columns where row and column took five passes of
 // 64-bit keys): edges come in row order and the sort is stable. Equal pairs are merged by
 // summing their values in input CSR order; as a canonical input has none, the pass assumes
-// so, and only where it meets one a second, compacting pass follows.
+// so, and only where it meets one a second, merging pass follows.
 // Bound: DRAM and the sort, 24 bytes per edge and pass. R-MAT 2^19 (16.0 M edges)
 // transposed with values: 0.67 ms, of it 0.46 the sort (1.38 ms with a row search per edge,
 // 64-bit keys, values gathered through edge numbers and separate passes for flags, scan,
@@ -65,6 +65,14 @@ struct Sorted {
     if constexpr (kT) return make_uint2(__ldg(key32 + i), pair ? __ldg(&pair[i].x) : __ldg(row + i));
     const uint64_t k = __ldg(key64 + i);
     return make_uint2((uint32_t)(k >> colbits), (uint32_t)(k & ((1ull << colbits) - 1)));
+  }
+  __device__ __forceinline__ uint2 at(int64_t i, float& x) const {  // and, of pairs, the value
+    if constexpr (kT) {
+      const uint2 v = pair ? __ldg(pair + i) : make_uint2(__ldg(row + i), __float_as_uint(1.0f));
+      x = __uint_as_float(v.y);
+      return make_uint2(__ldg(key32 + i), v.x);
+    }
+    return at(i);
   }
   __device__ __forceinline__ float value(int64_t i) const {
     if constexpr (kT) return pair ? __uint_as_float(__ldg(&pair[i].y)) : 1.0f;
@@ -182,96 +190,128 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// rowptr[first .. last] = value by one thread, or by all of the CTA's where some thread has a
-// long run (rows without entries): called by all threads, `any` their vote. A thread alone
-// wrote 8 M rows in 30 to 160 ms, 256 write them in 0.2.
-constexpr uint32_t kRun = 32;
-struct Runs {
-  int32_t many;
-  struct { uint32_t first, end; int32_t value; } run[kThreads];
-};
+// rowptr[first .. end) = value by each thread of a warp; long runs (rows without entries) by all
+// of its lanes, one after the other. A thread alone wrote 8 M rows in 30 to 160 ms.
 __device__ __forceinline__ void fill_rows(int32_t* __restrict__ rowptr, uint32_t first,
-                                          uint32_t end, int32_t value, bool any, Runs& s) {
-  const bool mine = end > first, far = mine && any && end - first > kRun;
-  if (mine && !far)
+                                          uint32_t end, int32_t value) {
+  const bool far = end > first && end - first > 32;
+  if (!far)
     for (uint32_t r = first; r < end; ++r) rowptr[r] = value;
-  if (!any) return;
-  if (threadIdx.x == 0) s.many = 0;
-  __syncthreads();
-  if (far) s.run[atomicAdd(&s.many, 1)] = {first, end, value};
-  __syncthreads();
-  for (int i = 0; i < s.many; ++i)
-    for (int64_t r = (int64_t)s.run[i].first + threadIdx.x; r < s.run[i].end; r += kThreads)
-      rowptr[r] = s.run[i].value;
-  __syncthreads();
+  for (uint32_t m = __ballot_sync(0xffffffffu, far); m; m &= m - 1) {
+    const int src = __ffs(m) - 1;
+    const uint32_t r1 = __shfl_sync(0xffffffffu, end, src);
+    const int32_t x = __shfl_sync(0xffffffffu, value, src);
+    for (int64_t r = (int64_t)__shfl_sync(0xffffffffu, first, src) + threadIdx.x % 32; r < r1; r += 32)
+      rowptr[r] = x;
+  }
 }
 
 // Writes the result where all pairs differ (bad[1] = 1 where some do not): edge i is entry
 // i; the first edge of a row also fills the row pointer since the row before. Writes nothing
-// for an invalid input (bad[0]), whose call leaves the outputs as they are.
+// for an invalid input (bad[0]), whose call leaves the outputs as they are; once an equal pair
+// was met, the rest is left to the merging pass, which writes all of it again.
 template <bool kT>
 __global__ void __launch_bounds__(kThreads)
     k_emit(const Sorted<kT> in, int64_t nnz, int32_t rows, int32_t* __restrict__ rowptr,
            int32_t* __restrict__ col_out, float* __restrict__ val_out, uint32_t* bad) {
-  if (bad[0]) return;
-  __shared__ Runs runs;
+  constexpr int V = kTile / kThreads;
   const int64_t t0 = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  uint2 k[kTile / kThreads], p[kTile / kThreads];
-  bool far = false;
+  uint2 k[V], p[V];
+  float x[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    const int64_t i = t0 + v * kThreads;
+    k[v] = i < nnz ? in.at(i, x[v]) : make_uint2((uint32_t)rows, 0);
+    p[v] = i > 0 && i <= nnz ? in.at(i - 1) : make_uint2(i > nnz ? (uint32_t)rows : 0xffffffffu, 0);
+  }
+  // (one thread asks: the words are one place in L2, 16 requests per CTA took 0.1 ms)
+  if (__syncthreads_or(threadIdx.x == 0 && *(volatile uint64_t*)bad != 0)) return;
+  bool equal = false;
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    const int64_t i = t0 + v * kThreads;
+    fill_rows(rowptr, p[v].x + 1, k[v].x + 1, (int32_t)i);
+    if (i >= nnz) continue;
+    equal |= p[v].x == k[v].x && p[v].y == k[v].y;
+    col_out[i] = (int32_t)k[v].y;
+    if (val_out) val_out[i] = kT ? x[v] : in.value(i);
+  }
+  if (__any_sync(0xffffffffu, equal) && threadIdx.x % 32 == 0) bad[1] = 1;  // (a store per pair: 0.15 ms)
+}
+
+// counts[b] = first edges of equal pairs among the edges of tile b; 0 past the last one.
+template <bool kT>
+__global__ void __launch_bounds__(kThreads)
+    k_firsts(const Sorted<kT> in, int64_t nnz, int32_t* __restrict__ counts) {
+  __shared__ int32_t sum;
+  const int64_t t0 = (int64_t)blockIdx.x * kTile + threadIdx.x;
+  if (threadIdx.x == 0) sum = 0;
+  int mine = 0;
 #pragma unroll
   for (int v = 0; v < kTile / kThreads; ++v) {
+    const int64_t i = t0 + v * kThreads;
+    if (i >= nnz) continue;
+    const uint2 k = in.at(i), p = i > 0 ? in.at(i - 1) : make_uint2(0xffffffffu, 0);
+    mine += k.x != p.x || k.y != p.y;
+  }
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  __syncthreads();
+  if (threadIdx.x % 32 == 0) atomicAdd(&sum, mine);
+  __syncthreads();
+  if (threadIdx.x == 0) counts[blockIdx.x] = sum;
+}
+
+// The result with equal pairs merged: the first edge of each sums up the values (input CSR
+// order) and writes its entry, the number of first edges before it: `before` its tile
+// (k_firsts, summed up), and in it by a scan over the CTA. A flag and a sum per edge in memory
+// instead cost 16 bytes per edge more.
+template <bool kT>
+__global__ void __launch_bounds__(kThreads)
+    k_emit_merged(const Sorted<kT> in, const int32_t* __restrict__ before, int64_t nnz,
+                  int32_t rows, int32_t* __restrict__ rowptr, int32_t* __restrict__ col_out,
+                  float* __restrict__ val_out) {
+  __shared__ int32_t part[kTile / 32];
+  constexpr int V = kTile / kThreads;
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  const int64_t t0 = (int64_t)blockIdx.x * kTile + threadIdx.x;
+  uint2 k[V], p[V];
+  uint32_t firsts[V];  // of the 32 edges of this warp's v-th load
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
     const int64_t i = t0 + v * kThreads;
     k[v] = i < nnz ? in.at(i) : make_uint2((uint32_t)rows, 0);
     p[v] = i > 0 && i <= nnz ? in.at(i - 1) : make_uint2(i > nnz ? (uint32_t)rows : 0xffffffffu, 0);
-    far |= k[v].x - p[v].x > kRun;  // (rows p.x + 1 .. k.x)
+    firsts[v] = __ballot_sync(0xffffffffu, i < nnz && (k[v].x != p[v].x || k[v].y != p[v].y));
+    if (lane == 0) part[v * (kThreads / 32) + warp] = __popc(firsts[v]);
   }
-  const bool any = __syncthreads_or(far);
+  __syncthreads();
+  if (warp == 0) {  // sums before each 32 edges, two per lane
+    static_assert(kTile / 32 == 64, "two per lane");
+    const int a = part[2 * lane], b = part[2 * lane + 1];
+    int y = a + b;
 #pragma unroll
-  for (int v = 0; v < kTile / kThreads; ++v) {
-    const int64_t i = t0 + v * kThreads;
-    fill_rows(rowptr, p[v].x + 1, k[v].x + 1, (int32_t)i, any, runs);
-    if (i >= nnz) continue;
-    if (p[v].x == k[v].x && p[v].y == k[v].y) bad[1] = 1;
-    col_out[i] = (int32_t)k[v].y;
-    if (val_out) val_out[i] = in.value(i);
-  }
-}
-
-template <bool kT>
-__global__ void k_flags(const Sorted<kT> in, int64_t nnz, int32_t* __restrict__ f) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= nnz; i += stride) {
-    bool first = i < nnz;
-    if (first && i > 0) {
-      const uint2 k = in.at(i), p = in.at(i - 1);
-      first = k.x != p.x || k.y != p.y;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, y, o);
+      if (lane >= o) y += u;
     }
-    f[i] = first;
+    part[2 * lane] = y - a - b;
+    part[2 * lane + 1] = y - b;
   }
-}
-
-// The same with equal pairs merged: the first edge of each sums up the values (input CSR
-// order) and writes entry P[i].
-template <bool kT>
-__global__ void k_emit_merged(const Sorted<kT> in, const int32_t* __restrict__ P, int64_t nnz,
-                              int32_t rows, int32_t* __restrict__ rowptr,
-                              int32_t* __restrict__ col_out, float* __restrict__ val_out) {
-  __shared__ Runs runs;
-  const int64_t stride = (int64_t)gridDim.x * kThreads;
-  for (int64_t i0 = blockIdx.x * (int64_t)kThreads; i0 <= nnz; i0 += stride) {
-    const int64_t i = i0 + threadIdx.x;
-    const uint2 k = i < nnz ? in.at(i) : make_uint2((uint32_t)rows, 0);
-    const uint2 p = i > nnz ? k : i > 0 ? in.at(i - 1) : make_uint2(0xffffffffu, 0);
-    const int32_t o = i <= nnz ? P[i] : 0;
-    const bool any = __syncthreads_or(k.x - p.x > kRun);
-    fill_rows(rowptr, p.x + 1, k.x + 1, o, any, runs);
-    if (i >= nnz || (i > 0 && p.x == k.x && p.y == k.y)) continue;
-    col_out[o] = (int32_t)k.y;
+  __syncthreads();
+  const int32_t base = before[blockIdx.x];
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    const int64_t i = t0 + v * kThreads;
+    const int32_t o =
+        base + part[v * (kThreads / 32) + warp] + __popc(firsts[v] & ((1u << lane) - 1));
+    fill_rows(rowptr, p[v].x + 1, k[v].x + 1, o);
+    if (!(firsts[v] >> lane & 1)) continue;
+    col_out[o] = (int32_t)k[v].y;
     if (val_out) {
       float s = in.value(i);
       for (int64_t j = i + 1; j < nnz; ++j) {
         const uint2 q = in.at(j);
-        if (q.x != k.x || q.y != k.y) break;
+        if (q.x != k[v].x || q.y != k[v].y) break;
         s += in.value(j);
       }
       val_out[o] = s;
@@ -285,7 +325,7 @@ struct Layout {
   int colbits, endbit;
 };
 
-// Workspace of a mode; the flags and their sums of the compacting pass take the place of
+// Workspace of a mode; the merging pass's counts per tile and their sums take the place of
 // the unsorted keys and what they carried (at least 4 bytes per edge each, and one more).
 Layout layout(int32_t rows_in, int32_t cols_in, int64_t nnz, int mode, bool with_val) {
   Layout L{};
@@ -320,7 +360,7 @@ Layout layout(int32_t rows_in, int32_t cols_in, int64_t nnz, int mode, bool with
     cub::DeviceRadixSort::SortKeys(nullptr, s1, (uint64_t*)nullptr, (uint64_t*)nullptr, (int64_t)n,
                                    0, L.endbit);
   cub::DeviceScan::ExclusiveSum(nullptr, s2, (int32_t*)nullptr, (int32_t*)nullptr,
-                                (int64_t)n + 1);
+                                (int64_t)n / kTile + 2);
   L.sort = take(s1);
   L.scan = take(s2);
   L.total = off;
@@ -330,7 +370,7 @@ Layout layout(int32_t rows_in, int32_t cols_in, int64_t nnz, int mode, bool with
 // From the sorted edges to the result; reads the input's error word on the way.
 template <bool kT>
 dtc_status emit(const Sorted<kT>& in, int64_t nnz, int32_t rows_out, int32_t* rowptr_out,
-                int32_t* col_out, float* val_out, int32_t* flags, int32_t* P, uint32_t* bad,
+                int32_t* col_out, float* val_out, int32_t* counts, int32_t* before, uint32_t* bad,
                 void* scan, size_t scan_bytes, uint32_t* hbad, int64_t* nnz_out, cudaStream_t st) {
   k_emit<kT><<<(unsigned)(nnz / kTile + 1), kThreads, 0, st>>>(in, nnz, rows_out, rowptr_out,
                                                               col_out, val_out, bad);
@@ -340,13 +380,16 @@ dtc_status emit(const Sorted<kT>& in, int64_t nnz, int32_t rows_out, int32_t* ro
   if (hbad[0]) return DTC_OK;  // (the caller reports it)
   *nnz_out = nnz;
   if (!hbad[1]) return DTC_OK;
-  k_flags<kT><<<grid_for(nnz + 1), kThreads, 0, st>>>(in, nnz, flags);
-  DTC_CUDA(cub::DeviceScan::ExclusiveSum(scan, scan_bytes, flags, P, nnz + 1, st));
-  k_emit_merged<kT><<<grid_for(nnz + 1), kThreads, 0, st>>>(in, P, nnz, rows_out, rowptr_out,
-                                                           col_out, val_out);
+  const int64_t tiles = nnz / kTile + 1;  // (the last one has the end of the row pointer)
+  k_firsts<kT><<<(unsigned)tiles, kThreads, 0, st>>>(in, nnz, counts);
+  // (the sums of one tile more: the last is the number of entries)
+  DTC_CUDA(cudaMemsetAsync(counts + tiles, 0, 4, st));
+  DTC_CUDA(cub::DeviceScan::ExclusiveSum(scan, scan_bytes, counts, before, tiles + 1, st));
+  k_emit_merged<kT><<<(unsigned)tiles, kThreads, 0, st>>>(in, before, nnz, rows_out, rowptr_out,
+                                                         col_out, val_out);
   DTC_CUDA(cudaGetLastError());
   int32_t hn = 0;
-  DTC_CUDA(cudaMemcpyAsync(&hn, P + nnz, 4, cudaMemcpyDeviceToHost, st));
+  DTC_CUDA(cudaMemcpyAsync(&hn, before + tiles, 4, cudaMemcpyDeviceToHost, st));
   DTC_CUDA(cudaStreamSynchronize(st));
   *nnz_out = hn;
   return DTC_OK;
