@@ -60,6 +60,11 @@ constexpr int group_bytes() {
 static_assert(Cap<uint32_t>::kWarp * 2 + (kMaxH + 1) * 4 <= kWarpBytes && kWarpBytes % 16 == 0 &&
               kCells >= (kWarpFill / 8 + 1) * 32, "warp scratch");
 constexpr int kPer = 16;      // windows per CTA at most, by one warp each
+// Up to kLane edges per window on average, a lane takes a window of up to kLane edges: a warp
+// per window waits for memory most of the time. Whole conversion of 2^24 rows of 4 edges, a
+// warp / a lane per window: one row per window 33 / 1.9 ms, two 17 / 1.8, four 8.8 / 2.2.
+constexpr int kLane = 16;
+inline bool tiny_windows(int64_t nnz, int32_t nwin) { return nnz <= (int64_t)kLane * nwin; }
 constexpr int kLargeBytes =
     kSweepCols / 8 + kSweepCols / 64 * 2 + kSweepCols / 32768 * 4 + (kMaxH + 1) * 4 + 256;
 
@@ -498,6 +503,73 @@ __device__ void count_large(const Csr& a, int32_t w, int32_t e0, int32_t n, uint
   if (t == 0) bp[w] = (distinct + a.W - 1) / a.W;
 }
 
+// A window of at most kLane edges by one lane: an edge's rank is the number of distinct
+// columns below its own, counted over the registers. `most`: edges of the warp's longest.
+__device__ __forceinline__ void count_lane(const Csr& a, int32_t w, int32_t e0, int32_t n,
+                                           int32_t most, int32_t* e2c, int32_t* e2r, int32_t* bp,
+                                           uint32_t* bad) {
+  int32_t c[kLane];
+  uint32_t firsts = 0;  // edges whose column none before has
+#pragma unroll
+  for (int j = 0; j < kLane; ++j) {
+    c[j] = INT32_MAX;
+    if (j < most && j < n) {
+      c[j] = __ldg(a.col + e0 + j);
+      if (c[j] < 0 || c[j] >= a.M) {
+        atomicOr(bad, 8u);
+        c[j] = 0;
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kLane; ++j)
+    if (j < most) {
+      bool first = j < n;
+#pragma unroll
+      for (int i = 0; i < j; ++i) first &= c[i] != c[j];
+      firsts |= (uint32_t)first << j;
+    }
+  const int64_t r0 = (int64_t)w * a.H;
+  const int rows = (int)min((int64_t)a.H, a.M - r0);
+  int32_t row = -1, end = e0;  // end of that row
+#pragma unroll
+  for (int j = 0; j < kLane; ++j)
+    if (j < most && j < n) {
+      int rank = 0;
+#pragma unroll
+      for (int i = 0; i < kLane; ++i) rank += (firsts >> i & 1) && c[i] < c[j];
+      e2c[e0 + j] = rank;
+      while (end <= e0 + j && row + 1 < rows) end = __ldg(a.rowptr + r0 + ++row + 1);
+      e2r[e0 + j] = (int32_t)(r0 + row);
+    }
+  bp[w] = (__popc(firsts) + a.W - 1) / a.W;
+}
+
+// Matrices of few edges per window: 32 windows per warp, those of more than kLane edges one
+// after the other by all its lanes.
+template <typename K>
+__global__ void __launch_bounds__(kGroup, 6)
+    k_count_tiny(const Csr a, int32_t* __restrict__ e2c, int32_t* __restrict__ e2r,
+                 int32_t* __restrict__ bp, uint32_t* bad) {
+  __shared__ __align__(16) uint8_t sm[4 * kWarpBytes];
+  const int lane = threadIdx.x & 31;
+  uint8_t* const wsm = sm + (threadIdx.x / 32) * kWarpBytes;
+  const int64_t w = (int64_t)blockIdx.x * kGroup + threadIdx.x;
+  int32_t e0 = 0, n = 0;
+  if (w < a.nwin) window_edges(a, (int32_t)w, e0, n);
+  const int32_t most = __reduce_max_sync(0xffffffffu, n <= kLane ? n : 0);
+  if (w < a.nwin && n <= kLane) count_lane(a, (int32_t)w, e0, n, most, e2c, e2r, bp, bad);
+  for (uint32_t m = __ballot_sync(0xffffffffu, n > kLane && n <= Cap<K>::kWarp); m; m &= m - 1) {
+    const int src = __ffs(m) - 1;
+    const int32_t ws = (int32_t)(w - lane + src), es = __shfl_sync(0xffffffffu, e0, src),
+                  ns = __shfl_sync(0xffffffffu, n, src);
+    if (ns <= 128) count_warp<K, 4>(a, ws, es, ns, wsm, lane, e2c, e2r, bp, bad);
+    else if (ns <= 256) count_warp<K, 8>(a, ws, es, ns, wsm, lane, e2c, e2r, bp, bad);
+    else if constexpr (sizeof(K) == 4)
+      count_warp<K, 16>(a, ws, es, ns, wsm, lane, e2c, e2r, bp, bad);
+  }
+}
+
 // The first mid_ctas CTAs take the listed middle windows, the others `per` windows each,
 // one per warp at a time.
 template <typename K>
@@ -565,9 +637,30 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // rwo = exclusive sum of bp (rwo[nwin] = T), 8192 windows per CTA; each CTA adds up the
 // windows before its own (a few coalesced loads per thread from L2) instead of a second
-// launch. out = {T, *bad}.
-constexpr int kScan = 8192;
+// launch. From kManyWindows on that sum is the longer part (it grows with the square), and it
+// is taken over the sums of the CTAs before (k_sums): 2^24 windows 36.6 -> 33.3 ms for the
+// whole conversion. out = {T, *bad}.
+constexpr int kScan = 8192, kManyWindows = 32 * kScan;
+__global__ void __launch_bounds__(1024) k_sums(const int32_t* __restrict__ bp, int32_t nwin,
+                                               int32_t* __restrict__ sums) {
+  __shared__ int32_t part[32];
+  const int64_t i0 = (int64_t)blockIdx.x * kScan;
+  int32_t s = 0;
+#pragma unroll
+  for (int v = 0; v < kScan / 1024; ++v) {
+    const int64_t i = i0 + v * 1024 + threadIdx.x;
+    s += i < nwin ? __ldg(bp + i) : 0;
+  }
+  s = __reduce_add_sync(0xffffffffu, s);
+  if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = __reduce_add_sync(0xffffffffu, part[threadIdx.x]);
+    if (threadIdx.x == 0) sums[blockIdx.x] = s;
+  }
+}
 __global__ void __launch_bounds__(1024) k_scan(const int32_t* __restrict__ bp, int32_t nwin,
+                                               const int32_t* __restrict__ cta_sums,
                                                int32_t* __restrict__ rwo, const uint32_t* bad,
                                                int32_t* out) {
   __shared__ int32_t sums[33], part[kScan];
@@ -575,8 +668,10 @@ __global__ void __launch_bounds__(1024) k_scan(const int32_t* __restrict__ bp, i
   const int64_t i0 = (int64_t)blockIdx.x * kScan;
   const int cnt = (int)min((int64_t)kScan, nwin - i0);
   int32_t before = 0;
+  const int32_t* const earlier = cta_sums ? cta_sums : bp;
+  const int64_t many = cta_sums ? (int64_t)blockIdx.x : i0;
 #pragma unroll 8
-  for (int64_t i = t; i < i0; i += 1024) before += __ldg(bp + i);
+  for (int64_t i = t; i < many; i += 1024) before += __ldg(earlier + i);
   for (int i = t; i < kScan; i += 1024) part[i] = i < cnt ? __ldg(bp + i0 + i) : 0;
 #pragma unroll
   for (int o = 16; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
@@ -1030,6 +1125,81 @@ __device__ __forceinline__ void fill_unit(const Csr& a, const Fill& f, int32_t w
   __syncwarp();
 }
 
+// A window of at most kLane edges by one lane; `most` as in count_lane.
+__device__ __forceinline__ void fill_lane(const Csr& a, const Fill& f, int32_t w, int32_t e0,
+                                          int32_t n, int32_t most) {
+  const int32_t b0 = __ldg(f.rwo + w), nb = __ldg(f.rwo + w + 1) - b0;
+  int32_t id[kLane];  // block << 16 | rank << 8 | row (past the last edge: beyond every block)
+  float x[kLane];
+  int used = 0;
+#pragma unroll
+  for (int j = 0; j < kLane; ++j) {
+    id[j] = INT32_MAX;
+    x[j] = 0.0f;
+    if (j < most && j < n) {
+      const int32_t rk = __ldg(f.e2c + e0 + j);
+      id[j] = a.block(rk) << 16 | rk << 8 | (__ldg(f.e2r + e0 + j) - w * a.H);
+      used = max(used, rk + 1);
+      if (f.values) x[j] = __ldg(f.values + e0 + j);
+    }
+  }
+  for (int b = 0; b < nb; ++b) {
+    int before = 0;
+#pragma unroll
+    for (int j = 0; j < kLane; ++j) before += id[j] >> 16 < b;
+    f.toff[b0 + b] = e0 + before;
+    f.rowid[b0 + b] = w;
+  }
+#pragma unroll
+  for (int j = 0; j < kLane; ++j)
+    if (j < most && j < n) {
+      const int b = id[j] >> 16, slot = a.slot(id[j] >> 8 & 0xff);
+      int place = 0;
+      bool again = false;  // a repeated (row, column): its value goes to the first one
+      float s = x[j];
+#pragma unroll
+      for (int i = 0; i < kLane; ++i) {
+        place += id[i] >> 16 < b || (i < j && id[i] >> 16 == b);
+        again |= i < j && id[i] == id[j];
+        if (i > j && id[i] == id[j]) s += x[i];
+      }
+      f.tile[e0 + place] = (uint8_t)((id[j] & 0xff) * a.W + slot);
+      f.s2x[(int64_t)(b0 + b) * a.W + slot] = __ldg(a.col + e0 + j);
+      if (f.values) f.tv[e0 + place] = again ? 0.0f : s;
+    }
+  zero_slots(a, f, b0 + nb, used, 0, 1);
+}
+
+// Matrices of few edges per window: as k_count_tiny.
+template <typename K>
+__global__ void __launch_bounds__(kGroup, 5) k_fill_tiny(const Csr a, const Fill f) {
+  __shared__ __align__(16) uint8_t sm[group_bytes<K>()];
+  __shared__ uint32_t redo[kGroup / 32];  // windows that one warp could not do
+  const int t = threadIdx.x, lane = t & 31;
+  const int64_t w = (int64_t)blockIdx.x * kGroup + t;
+  int32_t e0 = 0, n = 0;
+  if (w < a.nwin) window_edges(a, (int32_t)w, e0, n);
+  if (w == 0) f.toff[f.T] = (int32_t)a.nnz;
+  const int32_t most = __reduce_max_sync(0xffffffffu, n <= kLane ? n : 0);
+  if (n > 0 && n <= kLane) fill_lane(a, f, (int32_t)w, e0, n, most);
+  uint32_t todo = 0;
+  for (uint32_t m = __ballot_sync(0xffffffffu, n > kLane && n <= kWarpFill); m; m &= m - 1) {
+    const int src = __ffs(m) - 1;
+    if (!fill_warp(a, f, (int32_t)(w - lane + src), __shfl_sync(0xffffffffu, e0, src),
+                   __shfl_sync(0xffffffffu, n, src), sm + (t / 32) * kWarpBytes, lane))
+      todo |= 1u << src;
+  }
+  if (lane == 0) redo[t / 32] = todo;
+  __syncthreads();
+  for (int i = 0; i < kGroup / 32; ++i)
+    for (uint32_t m = redo[i]; m; m &= m - 1) {
+      const int32_t v = (int32_t)((int64_t)blockIdx.x * kGroup + 32 * i + __ffs(m) - 1);
+      window_edges(a, v, e0, n);
+      __syncthreads();
+      fill_small<K>(a, f, v, e0, n, sm, t);
+    }
+}
+
 // Warps first take the units of the listed windows (more than kWarpFill edges), then a
 // window each.
 template <typename K>
@@ -1099,7 +1269,7 @@ Csr make_csr(const int32_t* col, const int32_t* rowptr, int32_t M, int32_t nwin,
 }
 
 struct Layout {
-  size_t head, list, mid, mixed, units, total;  // head: see Head
+  size_t head, list, mid, mixed, units, sums, total;  // head: see Head
   int64_t room, mid_room, unit_room;                 // entries of the lists
   bool wide;
 };
@@ -1124,7 +1294,8 @@ Layout layout(int32_t M, int64_t nnz, int32_t H) {
   L.mid = align_up(L.list + large * 4, 256);
   L.mixed = align_up(L.mid + (size_t)L.mid_room * 4, 256);
   L.units = align_up(L.mixed + ((size_t)M + H - 1) / H, 256);
-  L.total = align_up(L.units + (size_t)L.unit_room * 8, 256);
+  L.sums = align_up(L.units + (size_t)L.unit_room * 8, 256);
+  L.total = align_up(L.sums + (((size_t)M + H - 1) / H / kScan + 1) * 4, 256);
   return L;
 }
 
@@ -1166,8 +1337,14 @@ dtc_status count_impl(const Csr& a, char* ws, const Layout& L, int32_t* e2c, int
   }
   const int64_t most = a.nnz / (Cap<K>::kWarp + 1), want = 8 * (int64_t)num_sms();
   const int mid_ctas = (int)(most < want ? most : want), per = windows_per_cta(a.nwin);
-  k_count<K><<<(unsigned)(mid_ctas + (a.nwin + per - 1) / per), kGroup, 0, st>>>(
-      a, mid_count, mid_list, (int32_t)L.mid_room, mid_ctas, per, e2c, e2r, bp, bad);
+  const bool tiny = tiny_windows(a.nnz, a.nwin);
+  const int64_t ctas = tiny ? 0 : ((int64_t)a.nwin + per - 1) / per;
+  if (mid_ctas + ctas)
+    k_count<K><<<(unsigned)(mid_ctas + ctas), kGroup, 0, st>>>(
+        a, mid_count, mid_list, (int32_t)L.mid_room, mid_ctas, per, e2c, e2r, bp, bad);
+  if (tiny)
+    k_count_tiny<K><<<(unsigned)(((int64_t)a.nwin + kGroup - 1) / kGroup), kGroup, 0, st>>>(
+        a, e2c, e2r, bp, bad);
   return DTC_OK;
 }
 
@@ -1202,8 +1379,13 @@ dtc_status fill_impl(const Csr& a, const Fill& f, char* ws, const Layout& L, cud
                                                        (int32_t)L.room, any);
   }
   const int per = windows_per_cta(a.nwin);
-  k_fill<K><<<(unsigned)(unit_ctas + (a.nwin + per - 1) / per), kGroup, 0, st>>>(
-      a, f, units, unit_list, mixed, unit, L.unit_room, unit_ctas, per);
+  const bool tiny = tiny_windows(a.nnz, a.nwin);
+  const int64_t ctas = tiny ? 0 : ((int64_t)a.nwin + per - 1) / per;
+  if (unit_ctas + ctas)
+    k_fill<K><<<(unsigned)(unit_ctas + ctas), kGroup, 0, st>>>(
+        a, f, units, unit_list, mixed, unit, L.unit_room, unit_ctas, per);
+  if (tiny)
+    k_fill_tiny<K><<<(unsigned)(((int64_t)a.nwin + kGroup - 1) / kGroup), kGroup, 0, st>>>(a, f);
   return DTC_OK;
 }
 
@@ -1256,8 +1438,10 @@ extern "C" dtc_status dtc_convert_count(const int32_t* d_col, const int32_t* d_r
                              nullptr, 0, nullptr, nullptr, 0);
   }
   int32_t* out = (int32_t*)(ws + L.head) + kOut;
-  k_scan<<<nwin ? (nwin + kScan - 1) / kScan : 1, 1024, 0, st>>>(d_blockPartition, nwin,
-                                                                 d_rowWindowOffset, bad, out);
+  const int32_t ctas = nwin ? (int32_t)(((int64_t)nwin + kScan - 1) / kScan) : 1;
+  int32_t* sums = nwin > kManyWindows ? (int32_t*)(ws + L.sums) : nullptr;
+  if (sums) k_sums<<<ctas, 1024, 0, st>>>(d_blockPartition, nwin, sums);
+  k_scan<<<ctas, 1024, 0, st>>>(d_blockPartition, nwin, sums, d_rowWindowOffset, bad, out);
   DTC_CUDA(cudaGetLastError());
   int32_t hostv[2] = {0, 0};
   DTC_CUDA(cudaMemcpyAsync(hostv, out, 8, cudaMemcpyDeviceToHost, st));

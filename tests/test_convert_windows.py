@@ -45,3 +45,40 @@ def test_window_classes(cuda, M, H, W, order):
     for k in ("RowWindowOffset", "TCblockRowid", "TCblocktileId", "TCblockoffset", "SparseAToX",
               "blockPartition", "edgeToColumn", "edgeToRow", "TCvalues"):
         np.testing.assert_array_equal(getattr(got, k).cpu().numpy(), exp[k], err_msg=k)
+
+
+@pytest.mark.parametrize("order", ["ascending", "mixed"])
+@pytest.mark.parametrize("M,H,W", [(70001, 1, 8), (70001, 2, 8), (70001, 16, 8), (70001, 16, 16),
+                                   (70001, 7, 5), (70001, 32, 8), (300001, 256, 1),
+                                   (2 ** 22 + 3, 3, 8), (2 ** 19 + 7, 1, 256)])
+def test_few_edges_per_window(cuda, M, H, W, order):
+    """At most 16 edges per window on average: windows of up to 16 edges by one lane, the others
+    as in other matrices; the last matrix has windows enough for the two-level scan."""
+    from dtc_b200 import metcf
+    rng = np.random.default_rng(M + H)
+    nwin = (M + H - 1) // H
+    n = rng.integers(0, 18, nwin)
+    n[:4] = 16, 17, 1, 0
+    n[rng.choice(nwin, 3, replace=False)] = 300
+    n[-1] = 15
+    if nwin > 1200:
+        n[nwin // 2], n[nwin // 3] = 1100, 2500
+    n = np.minimum(n, 8 * M // nwin + 9)
+    w = np.repeat(np.arange(nwin), n)
+    row = np.minimum(w * H + rng.integers(0, H, w.size), M - 1)
+    few = rng.random(w.size) < 0.3
+    col = np.where(few, rng.integers(0, 9, w.size), rng.integers(0, M, w.size))
+    o = np.lexsort((col if order == "ascending" else rng.random(w.size), row))
+    row, col = row[o], col[o]
+    if order == "ascending":  # distinct
+        keep = np.r_[True, (row[1:] != row[:-1]) | (col[1:] != col[:-1])]
+        row, col = row[keep], col[keep]
+    rowptr = np.searchsorted(row, np.arange(M + 1)).astype(np.int32)
+    assert col.size <= 16 * nwin
+    col, val = col.astype(np.int32), rng.random(col.size).astype(np.float32)
+    got = metcf.convert(rowptr, col, M, H=H, W=W, values=val)
+    exp = O.metcf(rowptr, col, M, H=H, W=W, values=val)
+    assert got.T == exp["T"]
+    for k in ("RowWindowOffset", "TCblockRowid", "TCblocktileId", "TCblockoffset", "SparseAToX",
+              "blockPartition", "edgeToColumn", "edgeToRow", "TCvalues"):
+        np.testing.assert_array_equal(getattr(got, k).cpu().numpy(), exp[k], err_msg=k)
