@@ -23,13 +23,15 @@
 //   places, up to 1024 edges: one warp marks the cells of every block and counts the marks
 //     before each; larger: a warp per 128 blocks does so, which finds its part of each row
 //     by binary search
-//   places where some row's ranks do not ascend (unsorted or repeated columns), and
-//     windows of more than 32 rows: 128 threads sort by block, or beyond 1024 edges 1024
-//     threads advance a counter per block row by row
+//   places where some row's ranks do not ascend (unsorted or repeated columns): the window's
+//     edges sorted by (block, edge), by one warp up to 1024, 1024 threads up to 16384, several
+//     such CTAs that share out the blocks beyond
+//   places in windows of more than 32 rows: a global radix sort
 // The lines lie where shared memory ends: a sort of 2048 keys beats clearing and counting a
 // bitmap of 2^20 columns (5 us) up to there.
 // Bound: instruction issue and the latency of dependent loads; DRAM is at a fifth.
 #include <algorithm>
+#include <cub/cub.cuh>
 #include "common.cuh"
 
 namespace dtc {
@@ -37,9 +39,13 @@ namespace {
 
 constexpr int kGroup = 128;              // threads of a CTA: four windows, or one middle window
 constexpr int kWarpFill = 1024;          // windows up to here: places by one warp
+constexpr int kLeftBytes = kWarpFill * 5;  // of a warp that sorts such a window: keys, tile ids
 constexpr int kThreads = 1024;           // threads of a large window
 constexpr int kSweepCols = 1 << 20;      // columns per sweep of a large window's bitmap
-constexpr int kSweepBlocks = 1 << 14;    // blocks per sweep of a large window's counters
+constexpr int kSortBits = 14, kSortEdges = 1 << kSortBits;  // edges that a large CTA sorts
+constexpr int kMergeWarps = 16;          // of a large CTA that merge
+constexpr int kPartBlocks = 8192;        // blocks of a part of a huge window, at most
+constexpr int kPartSort = 8192, kPartEdges = 6144;  // edges of a part: sorted at a time, on average
 constexpr int kMaxH = 256;               // rows of a window (block_h * block_w <= 256)
 constexpr int kUnitH = 32;               // rows up to which a warp takes part of a window
 
@@ -68,6 +74,7 @@ inline bool tiny_windows(int64_t nnz, int32_t nwin) { return nnz <= (int64_t)kLa
 constexpr int kLargeBytes =
     kSweepCols / 8 + kSweepCols / 64 * 2 + kSweepCols / 32768 * 4 + (kMaxH + 1) * 4 + 256;
 
+constexpr int log2_of(int n) { return n > 1 ? 1 + log2_of(n / 2) : 0; }
 inline int bits_for(uint64_t n) {  // bits to represent values in [0, n)
   int b = 0;
   while (b < 63 && (1ull << b) < n) ++b;
@@ -108,16 +115,17 @@ __device__ __forceinline__ int32_t many_listed(const int32_t* count, int32_t roo
 }
 
 // Lists the windows of more than mid_cap edges (mid_list) and of more than `cap`, those of
-// more than kHuge from the front and
-// the others from the back (count[0], count[1]); with `bad`, checks the row pointer
-// (rowptr[0] == 0, non-decreasing, rowptr[M] == nnz) and sets its bits. With `rwo`
-// (phase 2), also lists their units of `unit` blocks: (window, first block).
+// more than kHuge from the front and the others from the back (count[0], count[1]); with `bad`,
+// checks the row pointer (rowptr[0] == 0, non-decreasing, rowptr[M] == nnz) and sets its bits.
+// In phase 2 (`rwo`) also lists their units of `unit` blocks, (window, first block), and clears
+// `mixed`.
 __global__ void k_list(const Csr a, int32_t cap, int32_t mid_cap, int32_t* count, int32_t* list,
                        int32_t* mid_count, int32_t* mid_list, int32_t mid_room, uint32_t* bad,
                        int32_t room, const int32_t* rwo, int32_t unit, int32_t* units,
-                       int2* unit_list, int64_t unit_room) {
+                       int2* unit_list, int64_t unit_room, uint8_t* mixed) {
   const int32_t w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w < a.nwin) {
+    if (mixed) mixed[w] = 0;
     int32_t e0, n;
     window_edges(a, w, e0, n);
     if (n > cap) {
@@ -178,25 +186,6 @@ __device__ __forceinline__ int row_of(const int32_t* start, int rows, int32_t i)
     if (start[mid] <= i) lo = mid; else hi = mid;
   }
   return lo;
-}
-
-// Ascending bitonic sort of key[0, n2), n2 a power of two, by one group. Pairs
-// less than 64 apart stay inside a warp's 64 keys and need no group barrier.
-template <typename K>
-__device__ __forceinline__ void bitonic(K* key, int n2, int t) {
-  for (int k = 2; k <= n2; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = t; i < n2 / 2; i += kGroup) {
-        const int lo = 2 * i - (i & (j - 1)), hi = lo + j;
-        const K x = key[lo], y = key[hi];
-        if ((x > y) == ((lo & k) == 0)) {
-          key[lo] = y;
-          key[hi] = x;
-        }
-      }
-      if (j > 32 || (j == 1 && k >= 64)) __syncthreads(); else __syncwarp();
-    }
-  __syncthreads();
 }
 
 // Exclusive sum of x over the group's threads (s: kGroup / 32 words); *total = sum.
@@ -726,19 +715,89 @@ struct Fill {
 };
 
 // Values of one block in tile order where a (row, column) may occur twice: merged into
-// its first occurrence (fp32 sum in CSR order), later ones 0.
-__device__ void merge_block(const Fill& f, int32_t j0, int32_t j1) {
+// its first occurrence (fp32 sum in CSR order), later ones 0. By one thread. `tile`: the tile
+// ids, f.tile or a copy in shared memory (of edge j in [j]).
+__device__ void merge_block(const Fill& f, const uint8_t* tile, int32_t j0, int32_t j1) {
   uint32_t seen[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   for (int32_t j = j0; j < j1; ++j) {
-    const uint32_t p = f.tile[j], bit = 1u << (p & 31);
+    const uint32_t p = tile[j], bit = 1u << (p & 31);
     if (!(seen[p >> 5] & bit)) {
       seen[p >> 5] |= bit;
     } else {
       int32_t x = j0;
-      while (f.tile[x] != p) ++x;
+      while (tile[x] != p) ++x;
       f.tv[x] += f.tv[j];
       f.tv[j] = 0.0f;
     }
+  }
+}
+
+// The same by one warp, 32 edges at a time: the first lane of each cell adds up its peers.
+struct MergeScratch {
+  float sum[256], val[32];
+  int32_t first[256];  // edge of each cell that comes first, or -1
+};
+__device__ void merge_block(const Fill& f, const uint8_t* tile, int32_t j0, int32_t j1,
+                            MergeScratch& s, int lane) {
+  for (int c = lane; c < 256; c += 32) s.first[c] = -1;
+  for (int32_t j = j0 + lane; j - lane < j1; j += 32) {
+    const bool in = j < j1;
+    const uint32_t p = in ? tile[j] : 256u;
+    s.val[lane] = in ? f.tv[j] : 0.0f;
+    uint32_t peers = __match_any_sync(0xffffffffu, p);
+    __syncwarp();
+    if (in && lane == __ffs(peers) - 1) {
+      float x;
+      if (s.first[p] < 0) {
+        s.first[p] = j;
+        x = s.val[lane];
+        peers &= peers - 1;
+      } else {
+        x = s.sum[p];
+      }
+      for (; peers; peers &= peers - 1) x += s.val[__ffs(peers) - 1];
+      s.sum[p] = x;
+    }
+    __syncwarp();
+    if (in && s.first[p] != j) f.tv[j] = 0.0f;
+  }
+  for (int c = lane; c < 256; c += 32)
+    if (s.first[c] >= 0) f.tv[s.first[c]] = s.sum[c];
+  __syncwarp();
+}
+
+// Whether a cell occurs twice among the edges of a block.
+__device__ bool has_repeats(const uint8_t* tile, int32_t j0, int32_t j1) {
+  uint32_t seen[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int32_t j = j0; j < j1; ++j) {
+    const uint32_t p = tile[j], bit = 1u << (p & 31);
+    uint32_t old = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (p >> 5 == q) {
+        old = seen[q];
+        seen[q] |= bit;
+      }
+    if (old & bit) return true;
+  }
+  return false;
+}
+
+// All blocks b0 .. b0 + nb - 1, whose edges end at `last`, by `warps` warps: a lane looks
+// through a block; one that repeats a cell is merged by the lane up to 24 edges (a warp's
+// blocks wait for memory together), by the warp beyond (a lane takes a step per edge and a
+// search per repeated one).
+__device__ void merge_blocks(const Fill& f, const uint8_t* tile, int32_t b0, int32_t nb,
+                             int32_t last, int warp, int warps, MergeScratch& s, int lane) {
+  for (int32_t c = warp * 32; c < nb; c += warps * 32) {
+    const int32_t b = c + lane;
+    const int32_t j0 = b < nb ? f.toff[b0 + b] : 0, j1 = b + 1 < nb ? f.toff[b0 + b + 1] : last;
+    const bool any = b < nb && has_repeats(tile, j0, j1);
+    if (any && j1 - j0 <= 24) merge_block(f, tile, j0, j1);
+    __syncwarp();
+    for (uint32_t m = __ballot_sync(0xffffffffu, any && j1 - j0 > 24); m; m &= m - 1)
+      merge_block(f, tile, __shfl_sync(0xffffffffu, j0, __ffs(m) - 1),
+                  __shfl_sync(0xffffffffu, j1, __ffs(m) - 1), s, lane);
   }
 }
 
@@ -800,8 +859,190 @@ struct Marks {
   }
 };
 
+// Whether edge e's rank is not above that of the edge before it in its row: a repeated column
+// is possible (unsorted ones are too).
+__device__ __forceinline__ bool repeats(const Fill& f, int32_t e0, int32_t e, int32_t rk) {
+  const int32_t q = e > e0 ? e - 1 : e;  // (no branch: all loads under way together)
+  return (e > e0) & (__ldg(f.e2c + q) >= rk) & (__ldg(f.e2r + q) == __ldg(f.e2r + e));
+}
+
+// Stable sort of key[0, m), one per edge, by the `bits` bits from kSortBits on, by a whole
+// CTA: 7 bits per pass, a run of keys per warp, which counts and places 32 at a time by
+// matching their digits (by a ballot per bit: match.any took 45 cycles of the SM for 32 keys).
+// Returns where the keys end up (key or other). 16384 keys by two passes 35 us; a window of that
+// many edges 65 us in all (105 with the columns and values gathered in sorted order).
+constexpr int kDigits = 128, kHist = kDigits * 33;  // (a padded row of a word per warp and digit)
+__device__ __forceinline__ uint32_t same_digit(uint32_t d, bool in) {
+  uint32_t peers = __ballot_sync(0xffffffffu, in);
+#pragma unroll
+  for (int b = 0; b < 7; ++b) {
+    const uint32_t m = __ballot_sync(0xffffffffu, d >> b & 1);
+    peers &= d >> b & 1 ? m : ~m;
+  }
+  return peers;
+}
+__device__ __forceinline__ uint32_t* cta_sort(uint32_t* key, uint32_t* other, int32_t* hist,
+                                              int32_t* part, int m, int bits) {
+  static_assert(kThreads == 1024, "32 warps, four counters per thread");
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int seg = (m + kThreads - 1) / kThreads * 32, j0 = warp * seg, j1 = min(j0 + seg, m);
+  for (int shift = kSortBits; shift < kSortBits + bits; shift += 7) {
+    for (int i = t; i < kHist; i += kThreads) hist[i] = 0;
+    __syncthreads();
+    for (int j = j0 + lane; j - lane < j1; j += 32) {
+      const uint32_t d = j < j1 ? key[j] >> shift & (kDigits - 1) : 0;
+      const uint32_t peers = same_digit(d, j < j1);
+      if (j < j1 && lane == __ffs(peers) - 1) hist[d * 33 + warp] += __popc(peers);
+      __syncwarp();
+    }
+    __syncthreads();
+    int32_t* const h = hist + t / 8 * 33 + t % 8 * 4;  // four warps of a digit
+    const int c[4] = {h[0], h[1], h[2], h[3]};
+    int total;
+    int at = cta_scan(c[0] + c[1] + c[2] + c[3], part, &total);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      h[v] = at;
+      at += c[v];
+    }
+    __syncthreads();
+    for (int j = j0 + lane; j - lane < j1; j += 32) {
+      const uint32_t k = j < j1 ? key[j] : 0, d = k >> shift & (kDigits - 1);
+      const uint32_t peers = same_digit(d, j < j1);
+      const int to = j < j1 ? hist[d * 33 + warp] + __popc(peers & ((1u << lane) - 1)) : 0;
+      __syncwarp();
+      if (j < j1) {
+        other[to] = k;
+        if (lane == __ffs(peers) - 1) hist[d * 33 + warp] += __popc(peers);
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    uint32_t* const x = key;
+    key = other;
+    other = x;
+  }
+  return key;
+}
+
+// The most columns and whether an edge may repeat another, over the T threads of a warp or CTA.
+template <int T>
+__device__ __forceinline__ void vote(int& used, bool& dup, int t) {
+  used = __reduce_max_sync(0xffffffffu, used);
+  if constexpr (T == 32) {
+    dup = __any_sync(0xffffffffu, dup);
+  } else {
+    __shared__ int32_t s_used[T / 32];
+    if (t % 32 == 0) s_used[t / 32] = used;
+    dup = __syncthreads_or(dup);
+#pragma unroll
+    for (int i = 0; i < T / 32; ++i) used = max(used, s_used[i]);
+  }
+}
+
+// A window of up to 32 E edges in any order by a warp: its edges sorted by (block, edge), in
+// registers, are in their places.
+template <int E>
+__device__ __forceinline__ void fill_sorted(const Csr& a, const Fill& f, int32_t w, int32_t e0,
+                                            int32_t n, uint8_t* sm, int lane) {
+  constexpr int B = log2_of(32 * E);
+  static_assert((1 << B) == 32 * E && 2 * B <= 32, "block and edge in a key");
+  uint32_t* const key = reinterpret_cast<uint32_t*>(sm);
+  uint8_t* const ids = sm + kLeftBytes - kWarpFill;
+  const int32_t b0 = __ldg(f.rwo + w), nb = __ldg(f.rwo + w + 1) - b0;
+  uint32_t x[E];
+  int used = 0;
+  bool dup = false;
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    const int e = i * 32 + lane;
+    x[i] = 0xffffffffu;
+    if (e < n) {
+      const int32_t rk = __ldg(f.e2c + e0 + e);
+      x[i] = (uint32_t)a.block(rk) << B | (uint32_t)e;
+      used = max(used, rk + 1);
+      if (f.values) dup |= repeats(f, e0, e0 + e, rk);
+    }
+  }
+  reg_bitonic<uint32_t, E, 32>(x, lane, nullptr);
+#pragma unroll
+  for (int i = 0; i < E; ++i) key[lane * E + i] = x[i];
+  vote<32>(used, dup, lane);
+  __syncwarp();
+  for (int b = lane; b < nb; b += 32) f.rowid[b0 + b] = w;
+#pragma unroll 4
+  for (int j = lane; j < n; j += 32) {
+    const uint32_t k = key[j];
+    const int32_t b = b0 + (int32_t)(k >> B), e = e0 + (int32_t)(k & ((1u << B) - 1));
+    if (j == 0 || key[j - 1] >> B != k >> B) f.toff[b] = e0 + j;
+    const int32_t slot = a.slot(__ldg(f.e2c + e));
+    ids[j] = (uint8_t)((__ldg(f.e2r + e) - w * a.H) * a.W + slot);
+    f.tile[e0 + j] = ids[j];
+    f.s2x[(int64_t)b * a.W + slot] = __ldg(a.col + e);  // duplicates write the same value
+    if (f.values) f.tv[e0 + j] = __ldg(f.values + e);
+  }
+  zero_slots(a, f, b0 + nb, used, lane, 32);
+  __threadfence_block();
+  __syncwarp();
+  if (dup)  // (the keys are done with)
+    merge_blocks(f, ids - e0, b0, nb, e0 + n, 0, 1, *reinterpret_cast<MergeScratch*>(sm), lane);
+  __syncwarp();
+}
+
+// A window of up to kSortEdges edges in any order by a whole CTA. Columns and values go through
+// shared memory too: read in the sorted order from memory, a sector each, they took longer than
+// the sort.
+__device__ void fill_cta(const Csr& a, const Fill& f, int32_t w, int32_t e0, int32_t n, uint8_t* sm) {
+  uint32_t* key = reinterpret_cast<uint32_t*>(sm);
+  uint32_t* other = key + kSortEdges;
+  uint8_t* const sorted_ids = reinterpret_cast<uint8_t*>(other + kSortEdges);
+  int32_t* const hist = reinterpret_cast<int32_t*>(sorted_ids + kSortEdges);
+  uint8_t* const ids = reinterpret_cast<uint8_t*>(hist + kHist + 64);
+  const int t = threadIdx.x;
+  const int32_t b0 = __ldg(f.rwo + w), nb = __ldg(f.rwo + w + 1) - b0;
+  int used = 0;
+  bool dup = false;
+#pragma unroll 4
+  for (int j = t; j < n; j += kThreads) {
+    const int32_t rk = __ldg(f.e2c + e0 + j), row = __ldg(f.e2r + e0 + j) - w * a.H;
+    key[j] = (uint32_t)a.block(rk) << kSortBits | (uint32_t)j;
+    ids[j] = (uint8_t)(row * a.W + a.slot(rk));
+    used = max(used, rk + 1);
+    if (f.values) dup |= repeats(f, e0, e0 + j, rk);
+  }
+  vote<kThreads>(used, dup, t);
+  const uint32_t* const sorted = cta_sort(key, other, hist, hist + kHist, n, 32 - __clz(nb - 1));
+  int32_t* const staged = reinterpret_cast<int32_t*>(sorted == key ? other : key);  // (free now)
+  for (int b = t; b < nb; b += kThreads) f.rowid[b0 + b] = w;
+#pragma unroll 4
+  for (int j = t; j < n; j += kThreads) staged[j] = __ldg(a.col + e0 + j);
+  __syncthreads();
+  for (int j = t; j < n; j += kThreads) {
+    const uint32_t k = sorted[j], b = k >> kSortBits, e = k & (kSortEdges - 1);
+    if (j == 0 || sorted[j - 1] >> kSortBits != b) f.toff[b0 + b] = e0 + j;
+    const uint8_t id = ids[e];
+    sorted_ids[j] = id;
+    f.tile[e0 + j] = id;
+    f.s2x[(int64_t)(b0 + b) * a.W + id % (uint32_t)a.W] = staged[e];  // duplicates: the same value
+  }
+  zero_slots(a, f, b0 + nb, used, t, kThreads);
+  __syncthreads();
+  if (f.values) {
+#pragma unroll 4
+    for (int j = t; j < n; j += kThreads) staged[j] = __float_as_int(__ldg(f.values + e0 + j));
+    __syncthreads();
+    for (int j = t; j < n; j += kThreads)
+      f.tv[e0 + j] = __int_as_float(staged[sorted[j] & (kSortEdges - 1)]);
+    __threadfence_block();
+    __syncthreads();
+    if (dup && t / 32 < kMergeWarps)
+      merge_blocks(f, sorted_ids - e0, b0, nb, e0 + n, t / 32, kMergeWarps,
+                   reinterpret_cast<MergeScratch*>(hist)[t / 32], t & 31);
+    __syncthreads();
+  }
+}
+
 // One warp's window; false (nothing written) where a row's ranks do not ascend or the
-// window has too many blocks.
 __device__ __forceinline__ bool fill_warp(const Csr& a, const Fill& f, int32_t w, int32_t e0,
                                           int32_t n, uint8_t* sm, int lane) {
   const int32_t b0 = __ldg(f.rwo + w), nb = __ldg(f.rwo + w + 1) - b0;
@@ -858,170 +1099,150 @@ __device__ __forceinline__ bool fill_warp(const Csr& a, const Fill& f, int32_t w
   return true;
 }
 
-template <typename K>
-__device__ void fill_small(const Csr& a, const Fill& f, int32_t w, int32_t e0, int32_t n,
-                           uint8_t* sm, int t) {
-  constexpr int B = Cap<K>::kBits;
+// Blocks [p0, p1) of a window of any size in any order by one CTA: it reads all the window's
+// ranks, twice, a run of them per warp, and keeps the edges of its blocks, in order, which are
+// sorted by (block, edge). Where it keeps more than kPartSort, that many at a time go on from
+// each block's place so far. (16 loads under way per lane: 15 us for the ranks of 65,536 edges.)
+__device__ void fill_part(const Csr& a, const Fill& f, int32_t w, int32_t e0, int32_t n,
+                          int32_t p0, int32_t p1, uint8_t* sm) {
+  constexpr int V = kPartSort / 2 / kThreads, L = 16;
   uint32_t* key = reinterpret_cast<uint32_t*>(sm);
-  int32_t* part = reinterpret_cast<int32_t*>(sm + Cap<K>::kEdges * 4);
+  uint32_t* other = key + kPartSort;
+  int32_t* edge = reinterpret_cast<int32_t*>(other + kPartSort);  // kept edges
+  int32_t* cur = edge + kPartSort;                                // next place of each block
+  int32_t* hist = cur + kPartBlocks;
+  int32_t* part = hist + kHist;
+  __shared__ uint8_t ids[kPartSort];  // tile ids in sorted order, where it keeps them all
+  __shared__ uint8_t kept_ids[kPartSort];
+  __shared__ int32_t s_used, s_dup, s_before, s_kept[kThreads / 32];
+  const int t = threadIdx.x, lane = t & 31, np = p1 - p0;
+  const int64_t seg = ((int64_t)n / kThreads + 1) * 32;  // edges of a warp
+  const int64_t i0 = t / 32 * seg, i1 = min(i0 + seg, (int64_t)n);
   const int32_t b0 = __ldg(f.rwo + w), nb = __ldg(f.rwo + w + 1) - b0;
-  int n2 = 2;
-  while (n2 < n) n2 <<= 1;
-  int used = 0, dup = 0;
-  for (int i = t; i < n2; i += kGroup) {
-    uint32_t k = 0xffffffffu;
-    if (i < n) {
-      const int32_t rk = __ldg(f.e2c + e0 + i);
-      k = ((uint32_t)(a.block(rk)) << B) | (uint32_t)i;
-      used = max(used, rk + 1);
-      // ranks that do not ascend along a row: a repeated column is possible
-      if (i > 0 && __ldg(f.e2c + e0 + i - 1) >= rk &&
-          __ldg(f.e2r + e0 + i - 1) == __ldg(f.e2r + e0 + i))
-        dup = 1;
-    }
-    key[i] = k;
-  }
-  for (int b = t; b < nb; b += kGroup) f.rowid[b0 + b] = w;
+  if (t == 0) s_used = s_dup = s_before = 0;
+  for (int b = t; b < np; b += kThreads) cur[b] = 0;
   __syncthreads();
-  bitonic(key, n2, t);
-  for (int j = t; j < n; j += kGroup) {
-    const uint32_t k = key[j];
-    const int32_t b = b0 + (int32_t)(k >> B), e = e0 + (int32_t)(k & ((1u << B) - 1));
-    if (j == 0 || (key[j - 1] >> B) != (k >> B)) f.toff[b] = e0 + j;
-    const int32_t slot = a.slot(__ldg(f.e2c + e));
-    f.tile[e0 + j] = (uint8_t)((__ldg(f.e2r + e) - w * a.H) * a.W + slot);
-    f.s2x[(int64_t)b * a.W + slot] = __ldg(a.col + e);  // duplicates write the same value
-    if (f.values) f.tv[e0 + j] = __ldg(f.values + e);
-  }
-  // the most columns any thread saw, and whether any saw a possible duplicate
+  const int32_t rk0 = p0 * a.W, rk1 = p1 * a.W;  // ranks of the blocks
+  int used = 0, before = 0, kept = 0;
+  bool dup = false;
+  for (int64_t i = i0 + lane; i < i1; i += L * 32) {
+    int32_t rk[L];
 #pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    used = max(used, __shfl_xor_sync(0xffffffffu, used, o));
-    dup |= __shfl_xor_sync(0xffffffffu, dup, o);
-  }
-  if ((t & 31) == 0) part[t >> 5] = used * 2 + dup;
-  __syncthreads();
+    for (int v = 0; v < L; ++v) rk[v] = i + v * 32 < i1 ? __ldg(f.e2c + e0 + i + v * 32) : INT32_MAX;
 #pragma unroll
-  for (int i = 0; i < kGroup / 32; ++i) {
-    used = max(used, part[i] >> 1);
-    dup |= part[i] & 1;
-  }
-  zero_slots(a, f, b0 + nb, used, t, kGroup);
-  if (f.values && dup) {
-    __threadfence_block();
-    __syncthreads();
-    // block boundaries once more from the sorted keys
-    for (int j = t; j < n; j += kGroup)
-      if (j == 0 || (key[j - 1] >> B) != (key[j] >> B)) {
-        int j1 = j + 1;
-        while (j1 < n && (key[j1] >> B) == (key[j] >> B)) ++j1;
-        merge_block(f, e0 + j, e0 + j1);
+    for (int v = 0; v < L; ++v) {
+      before += rk[v] < rk0;
+      if (rk[v] >= rk0 && rk[v] < rk1) {
+        atomicAdd(cur + (a.block(rk[v]) - p0), 1);
+        ++kept;
+        used = max(used, rk[v] + 1);
+        if (f.values) dup |= repeats(f, e0, (int32_t)(e0 + i + v * 32), rk[v]);
       }
+    }
   }
-}
-
-__device__ void fill_large(const Csr& a, const Fill& f, int32_t w, int32_t e0, int32_t n,
-                           uint8_t* sm) {
-  int32_t* cur = reinterpret_cast<int32_t*>(sm);  // next place of each block of the sweep
-  int32_t* start = cur + kSweepBlocks;            // row starts (local), one past the last
-  int32_t* part = start + kMaxH + 1;
-  __shared__ int32_t s_used, s_dup;
-  __shared__ uint8_t s_mixed[kMaxH];              // rows whose ranks do not ascend
-  const int t = threadIdx.x;
-  const int64_t r0 = (int64_t)w * a.H;
-  const int rows = (int)min((int64_t)a.H, a.M - r0);
-  for (int r = t; r <= rows; r += kThreads) start[r] = __ldg(a.rowptr + r0 + r) - e0;
-  for (int r = t; r < rows; r += kThreads) s_mixed[r] = 0;
-  if (t == 0) s_used = s_dup = 0;
-  const int32_t b0 = __ldg(f.rwo + w), nb = __ldg(f.rwo + w + 1) - b0;
-  for (int b = t; b < nb; b += kThreads) f.rowid[b0 + b] = w;
-  int used = 0;
-  int32_t place = 0;  // edges in the blocks of the sweeps before
-  auto put = [&](int32_t i, int32_t rk, int32_t at, int row) {
-    const int32_t slot = a.slot(rk);
-    f.tile[e0 + at] = (uint8_t)(row * a.W + slot);
-    f.s2x[(int64_t)(b0 + a.block(rk)) * a.W + slot] = __ldg(a.col + e0 + i);
-    if (f.values) f.tv[e0 + at] = __ldg(f.values + e0 + i);
-  };
-  for (int32_t p0 = 0; p0 < nb; p0 += kSweepBlocks) {
-    const int32_t np = min(kSweepBlocks, nb - p0);
-    __syncthreads();
-    for (int b = t; b < np; b += kThreads) cur[b] = 0;
-    __syncthreads();
+  if (dup) s_dup = 1;
+  used = __reduce_max_sync(0xffffffffu, used);
+  before = __reduce_add_sync(0xffffffffu, before);
+  kept = __reduce_add_sync(0xffffffffu, kept);
+  if (lane == 0) {
+    atomicMax(&s_used, used);
+    atomicAdd(&s_before, before);
+    s_kept[t / 32] = kept;
+  }
+  __syncthreads();
+  const int per = (np + kThreads - 1) / kThreads, q0 = min(t * per, np), q1 = min(q0 + per, np);
+  int mine = 0;
+  for (int q = q0; q < q1; ++q) mine += cur[q];
+  int total;
+  int at = s_before + cta_scan(mine, part, &total);
+  for (int q = q0; q < q1; ++q) {
+    const int c = cur[q];
+    cur[q] = at;
+    f.toff[b0 + p0 + q] = e0 + at;
+    f.rowid[b0 + p0 + q] = w;
+    at += c;
+  }
+  __syncthreads();
+  auto flush = [&](int m) {
 #pragma unroll 4
-    for (int32_t i = t; i < n; i += kThreads) {
-      const int32_t rk = __ldg(f.e2c + e0 + i);
-      const uint32_t b = (uint32_t)(a.block(rk) - p0);
-      if (b < (uint32_t)np) atomicAdd(cur + b, 1);
-      if (p0 == 0) {
-        used = max(used, rk + 1);
-        if (i > 0) {
-          const int32_t before = __ldg(f.e2c + e0 + i - 1);
-          if (before >= rk) {
-            const int r = row_of(start, rows, i);
-            if (start[r] < i) {  // inside a row
-              s_dup = 1;
-              if (before > rk) s_mixed[r] = 1;
-            }
-          }
-        }
+    for (int j = t; j < m; j += kThreads) {
+      const int32_t rk = __ldg(f.e2c + edge[j]), row = __ldg(f.e2r + edge[j]) - w * a.H;
+      key[j] = (uint32_t)(a.block(rk) - p0) << kSortBits | (uint32_t)j;
+      kept_ids[j] = (uint8_t)(row * a.W + a.slot(rk));
+    }
+    __syncthreads();
+    const uint32_t* const sorted = cta_sort(key, other, hist, part, m, 32 - __clz(np - 1));
+    // the first kept edge of block b (from p0) among the m sorted ones
+    auto first_of = [&](uint32_t b) {
+      int lo = 0, hi = m;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (sorted[mid] >> kSortBits < b) lo = mid + 1; else hi = mid;
       }
-    }
-    if (p0 == 0) atomicMax(&s_used, used);
-    __syncthreads();
-    const int per = (np + kThreads - 1) / kThreads, q0 = min(t * per, np), q1 = min(q0 + per, np);
-    int mine = 0;
-    for (int q = q0; q < q1; ++q) mine += cur[q];
-    int total;
-    int at = place + cta_scan(mine, part, &total);
-    for (int q = q0; q < q1; ++q) {
-      const int c = cur[q];
-      cur[q] = at;
-      f.toff[b0 + p0 + q] = e0 + at;
-      at += c;
-    }
-    place += total;
-    __syncthreads();
-    for (int r = 0; r < rows; ++r) {
-      const int32_t i0 = start[r], i1 = start[r + 1];
-      if (!s_mixed[r]) {
-        // equal blocks are neighbours: an edge's place is its distance to the first of them
+      return lo;
+    };
 #pragma unroll 2
-        for (int32_t i = i0 + t; i < i1; i += kThreads) {
-          const int32_t rk = __ldg(f.e2c + e0 + i), blk = a.block(rk);
-          const uint32_t b = (uint32_t)(blk - p0);
-          if (b >= (uint32_t)np) continue;
-          int k = 0;
-          while (i - k > i0 && a.block(__ldg(f.e2c + e0 + i - k - 1)) == blk) ++k;
-          put(i, rk, cur[b] + k, r);
-        }
-        __syncthreads();
-        for (int32_t i = i0 + t; i < i1; i += kThreads) {
-          const uint32_t b = (uint32_t)(a.block(__ldg(f.e2c + e0 + i)) - p0);
-          if (b < (uint32_t)np) atomicAdd(cur + b, 1);
-        }
-      } else if (t < 32) {  // any order: 32 edges at a time, equal blocks by lane
-        for (int32_t i = i0; i < i1; i += 32) {
-          const int32_t rk = i + t < i1 ? __ldg(f.e2c + e0 + i + t) : -1;
-          const uint32_t b = rk < 0 ? 0xffffffffu : (uint32_t)(a.block(rk) - p0);
-          const bool in = b < (uint32_t)np;
-          const uint32_t same = __match_any_sync(0xffffffffu, in ? b : 0xffffffffu);
-          const int k = __popc(same & ((1u << t) - 1));
-          if (in) put(i + t, rk, cur[b] + k, r);
-          __syncwarp();
-          if (in && k == 0) cur[b] += __popc(same);
-          __syncwarp();
-        }
+    for (int j = t; j < m; j += kThreads) {
+      const uint32_t k = sorted[j], b = k >> kSortBits;
+      const int32_t e = edge[k & (kSortEdges - 1)], to = e0 + cur[b] + j - first_of(b);
+      const uint8_t id = kept_ids[k & (kSortEdges - 1)];
+      f.tile[to] = id;
+      if (total <= kPartSort) ids[to - e0 - s_before] = id;
+      f.s2x[(int64_t)(b0 + p0 + b) * a.W + id % (uint32_t)a.W] = __ldg(a.col + e);
+      if (f.values) f.tv[to] = __ldg(f.values + e);
+    }
+    __syncthreads();
+    for (int b = t; b < np; b += kThreads) cur[b] += first_of(b + 1) - first_of(b);
+    __syncthreads();
+  };
+  int m = 0;
+  if (total <= kPartSort) {
+    int to = 0;
+    for (int i = 0; i < t / 32; ++i) to += s_kept[i];
+    for (int64_t i = i0 + lane; i - lane < i1; i += L * 32) {
+      int32_t rk[L];
+#pragma unroll
+      for (int v = 0; v < L; ++v) rk[v] = i + v * 32 < i1 ? __ldg(f.e2c + e0 + i + v * 32) : -1;
+#pragma unroll
+      for (int v = 0; v < L; ++v) {
+        const bool keep = rk[v] >= rk0 && rk[v] < rk1;
+        const uint32_t mask = __ballot_sync(0xffffffffu, keep);
+        if (keep) edge[to + __popc(mask & ((1u << lane) - 1))] = (int32_t)(e0 + i + v * 32);
+        to += __popc(mask);
       }
-      __syncthreads();
+    }
+    m = total;
+    __syncthreads();
+  } else
+  for (int64_t i0 = 0; i0 < n; i0 += V * kThreads) {
+    int32_t keep = 0;  // of this thread's V edges, one after the other
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const int64_t i = i0 + t * V + v;
+      const int32_t b = i < n ? a.block(__ldg(f.e2c + e0 + i)) : -1;
+      keep |= (b >= p0 && b < p1) << v;
+    }
+    int add;
+    int to = m + cta_scan(__popc(keep), part, &add);
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+      if (keep >> v & 1) edge[to++] = (int32_t)(e0 + i0 + t * V + v);
+    m += add;
+    __syncthreads();
+    if (m > kPartSort - V * kThreads) {
+      flush(m);
+      m = 0;
     }
   }
-  zero_slots(a, f, b0 + nb, s_used, t, kThreads);
+  if (m) flush(m);
+  if (p1 == nb) zero_slots(a, f, b0 + nb, s_used, t, kThreads);
+  __shared__ int32_t s_end;
+  if (t == 0) s_end = cur[np - 1];  // (its place after the last block's edges)
   if (f.values && s_dup) {
     __threadfence_block();
     __syncthreads();
-    for (int b = t; b < nb; b += kThreads)
-      merge_block(f, f.toff[b0 + b], b + 1 < nb ? f.toff[b0 + b + 1] : e0 + n);
+    merge_blocks(f, total <= kPartSort ? ids - e0 - s_before : f.tile, b0 + p0, np, e0 + s_end,
+                 t / 32, kThreads / 32, reinterpret_cast<MergeScratch*>(sm)[t / 32], lane);
   }
   __syncthreads();
 }
@@ -1171,10 +1392,9 @@ __device__ __forceinline__ void fill_lane(const Csr& a, const Fill& f, int32_t w
 }
 
 // Matrices of few edges per window: as k_count_tiny.
-template <typename K>
-__global__ void __launch_bounds__(kGroup, 5) k_fill_tiny(const Csr a, const Fill f) {
-  __shared__ __align__(16) uint8_t sm[group_bytes<K>()];
-  __shared__ uint32_t redo[kGroup / 32];  // windows that one warp could not do
+__global__ void __launch_bounds__(kGroup, 5)
+    k_fill_tiny(const Csr a, const Fill f, int32_t* left, int32_t* __restrict__ left_list) {
+  __shared__ __align__(16) uint8_t sm[4 * kWarpBytes];
   const int t = threadIdx.x, lane = t & 31;
   const int64_t w = (int64_t)blockIdx.x * kGroup + t;
   int32_t e0 = 0, n = 0;
@@ -1182,33 +1402,24 @@ __global__ void __launch_bounds__(kGroup, 5) k_fill_tiny(const Csr a, const Fill
   if (w == 0) f.toff[f.T] = (int32_t)a.nnz;
   const int32_t most = __reduce_max_sync(0xffffffffu, n <= kLane ? n : 0);
   if (n > 0 && n <= kLane) fill_lane(a, f, (int32_t)w, e0, n, most);
-  uint32_t todo = 0;
   for (uint32_t m = __ballot_sync(0xffffffffu, n > kLane && n <= kWarpFill); m; m &= m - 1) {
     const int src = __ffs(m) - 1;
-    if (!fill_warp(a, f, (int32_t)(w - lane + src), __shfl_sync(0xffffffffu, e0, src),
-                   __shfl_sync(0xffffffffu, n, src), sm + (t / 32) * kWarpBytes, lane))
-      todo |= 1u << src;
+    const int32_t v = (int32_t)(w - lane + src);
+    if (!fill_warp(a, f, v, __shfl_sync(0xffffffffu, e0, src), __shfl_sync(0xffffffffu, n, src),
+                   sm + (t / 32) * kWarpBytes, lane) && lane == 0)
+      left_list[atomicAdd(left, 1)] = v;
   }
-  if (lane == 0) redo[t / 32] = todo;
-  __syncthreads();
-  for (int i = 0; i < kGroup / 32; ++i)
-    for (uint32_t m = redo[i]; m; m &= m - 1) {
-      const int32_t v = (int32_t)((int64_t)blockIdx.x * kGroup + 32 * i + __ffs(m) - 1);
-      window_edges(a, v, e0, n);
-      __syncthreads();
-      fill_small<K>(a, f, v, e0, n, sm, t);
-    }
 }
 
 // Warps first take the units of the listed windows (more than kWarpFill edges), then a
-// window each.
-template <typename K>
+// window each. Windows that they cannot do are left to k_fill_mixed.
 __global__ void __launch_bounds__(kGroup, 8)
     k_fill(const Csr a, const Fill f, const int32_t* __restrict__ units,
            const int2* __restrict__ unit_list, const uint8_t* __restrict__ mixed, int unit,
-           int64_t unit_room, int unit_ctas, int per) {
-  __shared__ __align__(16) uint8_t sm[group_bytes<K>()];
-  __shared__ int next, redo;  // windows that one warp could not do
+           int64_t unit_room, int unit_ctas, int per, int32_t* left,
+           int32_t* __restrict__ left_list) {
+  __shared__ __align__(16) uint8_t sm[4 * kWarpBytes];
+  __shared__ int next;
   const int t = threadIdx.x;
   if ((int)blockIdx.x < unit_ctas) {
     const int32_t many = (int32_t)min((int64_t)__ldg(units), unit_room);
@@ -1222,43 +1433,59 @@ __global__ void __launch_bounds__(kGroup, 8)
   int32_t e0, n;
   const int64_t w0 = (int64_t)(blockIdx.x - unit_ctas) * per;
   if (w0 == 0 && t == 0) f.toff[f.T] = (int32_t)a.nnz;
-  if (t == 0) {
-    next = kGroup / 32;
-    redo = 0;
-  }
+  if (t == 0) next = kGroup / 32;
   __syncthreads();
   for (int v = t / 32; v < per && w0 + v < a.nwin;) {
     window_edges(a, (int32_t)(w0 + v), e0, n);
     if (n > 0 && n <= kWarpFill &&
         !fill_warp(a, f, (int32_t)(w0 + v), e0, n, sm + (t / 32) * kWarpBytes, t & 31) &&
         (t & 31) == 0)
-      atomicOr(&redo, 1 << v);
+      left_list[atomicAdd(left, 1)] = (int32_t)(w0 + v);
     if ((t & 31) == 0) v = atomicAdd(&next, 1);
     v = __shfl_sync(0xffffffffu, v, 0);
   }
-  __syncthreads();
-  for (uint32_t todo = (uint32_t)redo; todo; todo &= todo - 1) {
-    const int32_t w = (int32_t)(w0 + __ffs(todo) - 1);
-    window_edges(a, w, e0, n);
-    __syncthreads();
-    fill_small<K>(a, f, w, e0, n, sm, t);
-  }
 }
 
+// Windows whose edges a sort has to place. Listed ones of more than kHuge edges (the list's
+// first) by parts, part p of the i-th by CTA (p + 91 i) % G; the other listed ones by a CTA
+// each; then those that k_fill left over, by a warp each.
 __global__ void __launch_bounds__(kThreads, 1)
     k_fill_mixed(const Csr a, const Fill f, const int32_t* __restrict__ count,
                  const int32_t* __restrict__ list, const uint8_t* __restrict__ mixed,
-                 int32_t room, const int32_t* __restrict__ any) {
+                 int32_t room, const int32_t* __restrict__ any, const int32_t* __restrict__ left,
+                 const int32_t* __restrict__ left_list) {
   extern __shared__ __align__(16) uint8_t dyn[];
-  if (!__ldg(any)) return;
-  const int32_t many = many_listed(count, room);
-  for (int32_t i = blockIdx.x; i < many; i += gridDim.x) {
-    const int32_t w = listed(count, list, room, i);
-    if (__ldg(mixed + w)) {
-      int32_t e0, n;
+  const int G = gridDim.x, c = blockIdx.x, t = threadIdx.x;
+  const int32_t rest = __ldg(left);
+  int32_t e0, n;
+  if (__ldg(any)) {
+    const int32_t many = many_listed(count, room), huge = min(__ldg(count), many);
+    for (int32_t i = 0; i < huge; ++i) {
+      const int32_t w = listed(count, list, room, i);
+      if (!__ldg(mixed + w)) continue;
       window_edges(a, w, e0, n);
-      fill_large(a, f, w, e0, n, dyn);
+      const int32_t nb = __ldg(f.rwo + w + 1) - __ldg(f.rwo + w);
+      const int parts = max(min((n + kPartEdges - 1) / kPartEdges, G), (nb + kPartBlocks - 1) / kPartBlocks);
+      int p = (int)((c - 91 * (int64_t)i) % G);
+      for (p = p < 0 ? p + G : p; p < parts; p += G)
+        fill_part(a, f, w, e0, n, (int32_t)((int64_t)nb * p / parts),
+                  (int32_t)((int64_t)nb * (p + 1) / parts), dyn);
     }
+    for (int32_t i = huge + c; i < many; i += G) {
+      const int32_t w = listed(count, list, room, i);
+      if (!__ldg(mixed + w)) continue;
+      window_edges(a, w, e0, n);
+      fill_cta(a, f, w, e0, n, dyn);
+    }
+    __syncthreads();
+  }
+  for (int32_t i = c * (kThreads / 32) + t / 32; i < rest; i += G * (kThreads / 32)) {
+    const int32_t w = __ldg(left_list + i);
+    window_edges(a, w, e0, n);
+    uint8_t* const sm = dyn + t / 32 * kLeftBytes;
+    if (n <= 128) fill_sorted<4>(a, f, w, e0, n, sm, t & 31);
+    else if (n <= 512) fill_sorted<16>(a, f, w, e0, n, sm, t & 31);
+    else fill_sorted<32>(a, f, w, e0, n, sm, t & 31);
   }
 }
 
@@ -1269,25 +1496,23 @@ Csr make_csr(const int32_t* col, const int32_t* rowptr, int32_t M, int32_t nwin,
 }
 
 struct Layout {
-  size_t head, list, mid, mixed, units, sums, total;  // head: see Head
+  size_t head, list, mid, mixed, units, sums, left, tall, sort, total;  // head: see Head
   int64_t room, mid_room, unit_room;                 // entries of the lists
   bool wide;
 };
 
 // Words of the workspace's head, zero at the start of a phase.
-enum Head { kCount = 0, kBad = 2, kOut = 3, kUnits = 5, kTicket = 6, kMid = 7, kAny = 8, kHead = 9 };
+enum Head { kCount = 0, kBad = 2, kOut = 3, kUnits = 5, kTicket = 6, kMid = 7, kAny = 8, kLeft = 9, kHead = 10 };
 
-// Blocks per unit of a large window (0: none, rows beyond the warp's arrays).
-int unit_blocks(int H) { return H > kUnitH ? 0 : 128; }
-static_assert(128 * 8 * 4 <= kCells, "a unit's masks fit");
+constexpr int kUnit = 128;  // blocks per unit of a large window
+static_assert(kUnit * 8 * 4 <= kCells, "a unit's masks fit");
 
 Layout layout(int32_t M, int64_t nnz, int32_t H) {
   Layout L{};
   L.wide = bits_for((uint64_t)(M > 0 ? M : 1)) + Cap<uint32_t>::kBits > 32;
   const size_t large = (size_t)nnz / (kWarpFill + 1) + 1;  // listed windows, at most
-  const int unit = unit_blocks(H);
   L.room = (int64_t)large;
-  L.unit_room = unit ? nnz / unit + (int64_t)large : 0;
+  L.unit_room = H > kUnitH ? 0 : nnz / kUnit + (int64_t)large;
   L.head = 0;
   L.list = 256;
   L.mid_room = nnz / (Cap<uint64_t>::kWarp + 1) + 1;
@@ -1295,12 +1520,26 @@ Layout layout(int32_t M, int64_t nnz, int32_t H) {
   L.mixed = align_up(L.mid + (size_t)L.mid_room * 4, 256);
   L.units = align_up(L.mixed + ((size_t)M + H - 1) / H, 256);
   L.sums = align_up(L.units + (size_t)L.unit_room * 8, 256);
-  L.total = align_up(L.sums + (((size_t)M + H - 1) / H / kScan + 1) * 4, 256);
+  L.left = align_up(L.sums + (((size_t)M + H - 1) / H / kScan + 1) * 4, 256);
+  L.tall = align_up(L.left + ((size_t)M + H - 1) / H * 4, 256);
+  L.sort = L.total = L.tall;
+  if (H > kUnitH) {
+    size_t bytes = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
+                                    (int32_t*)nullptr, (int32_t*)nullptr, nnz > 0 ? nnz : 1, 0, 32);
+    L.sort = align_up(L.tall + (size_t)nnz * 16, 256);
+    L.total = align_up(L.sort + bytes, 256);
+  }
   return L;
 }
 
-static_assert(kSweepBlocks * 4 + (kMaxH + 1) * 4 + 256 <= kLargeBytes, "fill_large fits");
-static_assert(kWarpFill <= Cap<uint64_t>::kEdges, "fill_small takes what a warp could not");
+static_assert(kHuge <= kSortEdges, "fill_sorted takes every window that is not huge");
+constexpr int kSortBytes =
+    kSortEdges * 9 + std::max(kHist * 4 + 256 + kSortEdges, kMergeWarps * (int)sizeof(MergeScratch));
+static_assert(kThreads / 32 * (int)sizeof(MergeScratch) <= kPartSort * 12 && kPartSort <= kSortEdges &&
+              kPartSort * 12 + kPartBlocks * 4 + kHist * 4 + 256 <= kSortBytes, "fill_part fits");
+static_assert(kThreads / 32 * kLeftBytes <= kSortBytes && sizeof(MergeScratch) <= kWarpFill * 4,
+              "fill_sorted, by every warp");
 
 // CTAs for the windows of more than `cap` edges: no more than there can be, one per SM.
 int large_ctas(int64_t nnz, int cap) {
@@ -1326,7 +1565,7 @@ dtc_status count_impl(const Csr& a, char* ws, const Layout& L, int32_t* e2c, int
   int32_t* mid_list = (int32_t*)(ws + L.mid);
   k_list<<<(a.nwin + 255) / 256, 256, 0, st>>>(a, Cap<K>::kEdges, Cap<K>::kWarp, count, list,
                                                mid_count, mid_list, (int32_t)L.mid_room, bad,
-                                               (int32_t)L.room, nullptr, 0, nullptr, nullptr, 0);
+                                               (int32_t)L.room, nullptr, 0, nullptr, nullptr, 0, nullptr);
   const int large = large_ctas(a.nnz, Cap<K>::kEdges);
   if (large) {
     DTC_CUDA(cudaFuncSetAttribute(k_count_large, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1348,44 +1587,86 @@ dtc_status count_impl(const Csr& a, char* ws, const Layout& L, int32_t* e2c, int
   return DTC_OK;
 }
 
-template <typename K>
+// Windows of more than kUnitH rows (block shapes of 64 x 4 and taller): all edges sorted by
+// block, with a global radix sort. A warp finds its part of a row by search; with that many
+// rows the searches cost more than the sort's passes.
+__global__ void k_tall_keys(const Csr a, const Fill f, uint32_t* __restrict__ key,
+                            int32_t* __restrict__ edge, int32_t* any) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= a.nnz) return;
+  const int32_t rk = __ldg(f.e2c + e);
+  key[e] = (uint32_t)(__ldg(f.rwo + __ldg(f.e2r + e) / a.H) + a.block(rk));
+  edge[e] = (int32_t)e;
+  if (repeats(f, 0, (int32_t)e, rk)) *any = 1;
+}
+__global__ void k_tall_emit(const Csr a, const Fill f, const uint32_t* __restrict__ key,
+                            const int32_t* __restrict__ edge) {
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= a.nnz) return;
+  const uint32_t b = __ldg(key + j);
+  const int32_t e = __ldg(edge + j), row = __ldg(f.e2r + e), w = row / a.H;
+  const int32_t slot = a.slot(__ldg(f.e2c + e));
+  if (j == 0) f.toff[f.T] = (int32_t)a.nnz;
+  if (j == 0 || __ldg(key + j - 1) != b) {
+    f.toff[b] = (int32_t)j;
+    f.rowid[b] = w;
+  }
+  f.tile[j] = (uint8_t)((row - w * a.H) * a.W + slot);
+  f.s2x[(int64_t)b * a.W + slot] = __ldg(a.col + e);
+  if (f.values) f.tv[j] = __ldg(f.values + e);
+}
+__global__ void __launch_bounds__(kGroup) k_tall_merge(const Csr a, const Fill f, const int32_t* any) {
+  __shared__ MergeScratch s[kGroup / 32];
+  if (*any)
+    merge_blocks(f, f.tile, 0, (int32_t)f.T, (int32_t)a.nnz, blockIdx.x * (kGroup / 32) + threadIdx.x / 32,
+                 gridDim.x * (kGroup / 32), s[threadIdx.x / 32], threadIdx.x & 31);
+}
+dtc_status fill_tall(const Csr& a, const Fill& f, char* ws, const Layout& L, cudaStream_t st) {
+  uint32_t *kin = (uint32_t*)(ws + L.tall), *kout = kin + a.nnz;
+  int32_t *ein = (int32_t*)(kout + a.nnz), *eout = ein + a.nnz;
+  int32_t* any = (int32_t*)(ws + L.head) + kAny;
+  const unsigned g = (unsigned)((a.nnz + 255) / 256);
+  DTC_CUDA(cudaMemsetAsync(f.s2x, 0, (size_t)f.T * a.W * 4, st));
+  k_tall_keys<<<g, 256, 0, st>>>(a, f, kin, ein, any);
+  size_t bytes = L.total - L.sort;
+  DTC_CUDA(cub::DeviceRadixSort::SortPairs(ws + L.sort, bytes, kin, kout, ein, eout, a.nnz, 0,
+                                           bits_for((uint64_t)f.T), st));
+  k_tall_emit<<<g, 256, 0, st>>>(a, f, kout, eout);
+  if (f.values) k_tall_merge<<<8 * num_sms(), kGroup, 0, st>>>(a, f, any);
+  return DTC_OK;
+}
+
 dtc_status fill_impl(const Csr& a, const Fill& f, char* ws, const Layout& L, cudaStream_t st) {
-  int32_t* count = (int32_t*)(ws + L.head) + kCount;
-  int32_t* list = (int32_t*)(ws + L.list);
-  const int large = large_ctas(a.nnz, kWarpFill);
-  int32_t* units = (int32_t*)(ws + L.head) + kUnits;
+  int32_t* head = (int32_t*)(ws + L.head);
+  int32_t *list = (int32_t*)(ws + L.list), *left_list = (int32_t*)(ws + L.left);
   int2* unit_list = (int2*)(ws + L.units);
   uint8_t* mixed = (uint8_t*)(ws + L.mixed);
-  const int unit = unit_blocks(a.H);
   int unit_ctas = 0;
-  if (large) {
-    k_list<<<(a.nwin + 255) / 256, 256, 0, st>>>(a, kWarpFill, INT32_MAX, count, list, nullptr,
-                                                 nullptr, 0, nullptr,
-                                                 (int32_t)L.room, f.rwo, unit, units, unit_list,
-                                                 L.unit_room);
-    int32_t* any = (int32_t*)(ws + L.head) + kAny;
-    DTC_CUDA(cudaMemsetAsync(mixed, unit ? 0 : 1, a.nwin, st));
-    if (!unit) DTC_CUDA(cudaMemsetAsync(any, 1, 4, st));
-    if (unit) {
-      k_mixed<<<(unsigned)((a.nnz + 2047) / 2048), 256, 0, st>>>(a, f.e2c, f.e2r, mixed,
-                                                                      any);
-      // a warp per unit up to eight CTAs per SM
-      const int64_t most = (L.unit_room + 3) / 4, want = 8 * (int64_t)num_sms();
-      unit_ctas = (int)(most < want ? most : want);
-    }
-    DTC_CUDA(cudaFuncSetAttribute(k_fill_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kLargeBytes));
-    k_fill_mixed<<<large, kThreads, kLargeBytes, st>>>(a, f, count, list, mixed,
-                                                       (int32_t)L.room, any);
+  if (a.nnz > kWarpFill) {
+    k_list<<<(a.nwin + 255) / 256, 256, 0, st>>>(a, kWarpFill, INT32_MAX, head + kCount, list, nullptr,
+                                                 nullptr, 0, nullptr, (int32_t)L.room, f.rwo, kUnit,
+                                                 head + kUnits, unit_list, L.unit_room, mixed);
+    k_mixed<<<(unsigned)((a.nnz + 2047) / 2048), 256, 0, st>>>(a, f.e2c, f.e2r, mixed, head + kAny);
+    // a warp per unit up to eight CTAs per SM
+    unit_ctas = (int)std::min<int64_t>((L.unit_room + 3) / 4, 8 * num_sms());
   }
   const int per = windows_per_cta(a.nwin);
   const bool tiny = tiny_windows(a.nnz, a.nwin);
   const int64_t ctas = tiny ? 0 : ((int64_t)a.nwin + per - 1) / per;
   if (unit_ctas + ctas)
-    k_fill<K><<<(unsigned)(unit_ctas + ctas), kGroup, 0, st>>>(
-        a, f, units, unit_list, mixed, unit, L.unit_room, unit_ctas, per);
+    k_fill<<<(unsigned)(unit_ctas + ctas), kGroup, 0, st>>>(a, f, head + kUnits, unit_list, mixed, kUnit,
+                                                          L.unit_room, unit_ctas, per, head + kLeft,
+                                                          left_list);
   if (tiny)
-    k_fill_tiny<K><<<(unsigned)(((int64_t)a.nwin + kGroup - 1) / kGroup), kGroup, 0, st>>>(a, f);
+    k_fill_tiny<<<(unsigned)(((int64_t)a.nwin + kGroup - 1) / kGroup), kGroup, 0, st>>>(
+        a, f, head + kLeft, left_list);
+  // a CTA per SM, fewer where there are not the edges
+  const int mixed_ctas = (int)std::min<int64_t>(a.nnz / 512 + 1, num_sms());
+  DTC_CUDA(cudaFuncSetAttribute(k_fill_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kSortBytes));
+  k_fill_mixed<<<mixed_ctas, kThreads, kSortBytes, st>>>(a, f, head + kCount, list, mixed,
+                                                         (int32_t)L.room, head + kAny, head + kLeft,
+                                                         left_list);
   return DTC_OK;
 }
 
@@ -1435,7 +1716,7 @@ extern "C" dtc_status dtc_convert_count(const int32_t* d_col, const int32_t* d_r
     if (s != DTC_OK) return s;
   } else {
     k_list<<<1, 32, 0, st>>>(a, 0, 0, nullptr, nullptr, nullptr, nullptr, 0, bad, 0,
-                             nullptr, 0, nullptr, nullptr, 0);
+                             nullptr, 0, nullptr, nullptr, 0, nullptr);
   }
   int32_t* out = (int32_t*)(ws + L.head) + kOut;
   const int32_t ctas = nwin ? (int32_t)(((int64_t)nwin + kScan - 1) / kScan) : 1;
@@ -1488,7 +1769,7 @@ extern "C" dtc_status dtc_convert_fill(const int32_t* d_col, const int32_t* d_ro
   const Fill f{d_edgeToColumn, d_edgeToRow, d_rowWindowOffset, d_values, d_tcblockRowid,
                d_tcblockOffset, d_sparseAToX, d_tileId, d_tcValues, num_blocks};
   DTC_CUDA(cudaMemsetAsync(ws + L.head, 0, kHead * 4, st));
-  s = L.wide ? fill_impl<uint64_t>(a, f, ws, L, st) : fill_impl<uint32_t>(a, f, ws, L, st);
+  s = block_h > kUnitH ? fill_tall(a, f, ws, L, st) : fill_impl(a, f, ws, L, st);
   if (s != DTC_OK) return s;
   DTC_CUDA(cudaGetLastError());
   return DTC_OK;

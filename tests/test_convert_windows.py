@@ -82,3 +82,24 @@ def test_few_edges_per_window(cuda, M, H, W, order):
     for k in ("RowWindowOffset", "TCblockRowid", "TCblocktileId", "TCblockoffset", "SparseAToX",
               "blockPartition", "edgeToColumn", "edgeToRow", "TCvalues"):
         np.testing.assert_array_equal(getattr(got, k).cpu().numpy(), exp[k], err_msg=k)
+
+
+@pytest.mark.parametrize("H,W", [(16, 8), (32, 8), (16, 16), (64, 4), (3, 64)])
+@pytest.mark.parametrize("n", [300, 1000, 9000, 40000, 200000])
+def test_unsorted_windows_with_hot_columns(cuda, n, H, W):
+    """Edges in any order, a few columns that most of them repeat (blocks of thousands of edges,
+    merged values) and many more that occur once."""
+    from dtc_b200 import metcf
+    M = 50000
+    rng = np.random.default_rng(n + H)
+    row = np.repeat([M // 2 // H * H, M // 2 // H * H + H - 1, M - 1], [n // 2, n // 4, n // 4])
+    col = np.where(rng.random(row.size) < 0.7, rng.integers(700, 703, row.size),
+                   rng.integers(0, M, row.size))
+    rowptr = np.searchsorted(row, np.arange(M + 1)).astype(np.int32)
+    col, val = col.astype(np.int32), rng.standard_normal(col.size).astype(np.float32)
+    got = metcf.convert(rowptr, col, M, H=H, W=W, values=val)
+    exp = O.metcf(rowptr, col, M, H=H, W=W, values=val)
+    assert got.T == exp["T"]
+    for k in ("RowWindowOffset", "TCblockRowid", "TCblocktileId", "TCblockoffset", "SparseAToX",
+              "blockPartition", "edgeToColumn", "edgeToRow", "TCvalues"):
+        np.testing.assert_array_equal(getattr(got, k).cpu().numpy(), exp[k], err_msg=k)
