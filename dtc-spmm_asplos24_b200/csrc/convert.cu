@@ -16,10 +16,11 @@
 // blocks, with the passes around them 3.8 ms for R-MAT 2^20, 32 M edges, of which the
 // edges' own bytes are 0.13 ms; here 1.0 ms: ranks 0.42, places 0.51). By window:
 //   ranks, up to 512 edges: one warp sorts packed (column, edge) keys in registers
-//     (bitonic, neighbours by shuffles) and reads the ranks off the order; up to 2048 (half
-//     of both where column and edge need more than 32 bits): the same by 128 threads
+//     (bitonic, neighbours by shuffles) and reads the ranks off the order (up to 256 where
+//     column and edge need more than 32 bits); up to 2048: the same by 128 threads
 //   ranks, larger: 1024 threads mark the columns in a bitmap (2^20 columns per sweep over
-//     the window) and count the bits before each (a whole CTA per SM, the longest first)
+//     the window) and count the bits before each (a whole CTA per SM, the longest first);
+//     where the columns take many sweeps they sort windows of up to 16384 edges instead
 //   places, up to 1024 edges: one warp marks the cells of every block and counts the marks
 //     before each; larger: a warp per 128 blocks does so, which finds its part of each row
 //     by binary search
@@ -27,8 +28,8 @@
 //     edges sorted by (block, edge), by one warp up to 1024, 1024 threads up to 16384, several
 //     such CTAs that share out the blocks beyond
 //   places in windows of more than 32 rows: a global radix sort
-// The lines lie where shared memory ends: a sort of 2048 keys beats clearing and counting a
-// bitmap of 2^20 columns (5 us) up to there.
+// The lines: a sort of 2048 keys beats clearing and counting a bitmap of 2^20 columns (5 us)
+// up to there; further ones beside the code.
 // Bound: instruction issue and the latency of dependent loads; DRAM is at a fifth.
 #include <algorithm>
 #include <cub/cub.cuh>
@@ -51,8 +52,8 @@ constexpr int kUnitH = 32;               // rows up to which a warp takes part o
 
 template <typename K>
 struct Cap {
-  static constexpr int kEdges = sizeof(K) == 4 ? 2048 : 1024;
-  static constexpr int kBits = sizeof(K) == 4 ? 11 : 10;
+  static constexpr int kEdges = 2048;  // ranks by 128 threads
+  static constexpr int kBits = 11;
   static constexpr int kWarp = sizeof(K) == 4 ? 512 : 256;  // ranks by one warp (registers)
 };
 // Bytes of a group: keys, 16-bit ranks and row starts of a middle window, or four
@@ -71,6 +72,7 @@ constexpr int kPer = 16;      // windows per CTA at most, by one warp each
 // warp / a lane per window: one row per window 33 / 1.9 ms, two 17 / 1.8, four 8.8 / 2.2.
 constexpr int kLane = 16;
 inline bool tiny_windows(int64_t nnz, int32_t nwin) { return nnz <= (int64_t)kLane * nwin; }
+// (count_sorted: its keys, ranks, rows)
 constexpr int kLargeBytes =
     kSweepCols / 8 + kSweepCols / 64 * 2 + kSweepCols / 32768 * 4 + (kMaxH + 1) * 4 + 256;
 
@@ -397,6 +399,59 @@ __device__ __forceinline__ void count_small(const Csr& a, int32_t w, int32_t e0,
   __syncthreads();
 }
 
+// A window of up to kThreads * E edges by a whole CTA: sorted by column, as count_small.
+template <int E>
+__device__ void count_sorted(const Csr& a, int32_t w, int32_t e0, int32_t n, uint8_t* sm,
+                             int32_t* e2c, int32_t* e2r, int32_t* bp, uint32_t* bad) {
+  constexpr int B = kSortBits;
+  uint64_t* key = reinterpret_cast<uint64_t*>(sm);
+  uint16_t* rank = reinterpret_cast<uint16_t*>(key + kSortEdges);
+  int32_t* start = reinterpret_cast<int32_t*>(rank + kSortEdges);
+  int32_t* part = start + kMaxH + 1;
+  const int t = threadIdx.x;
+  const int64_t r0 = (int64_t)w * a.H;
+  const int rows = (int)min((int64_t)a.H, a.M - r0);
+  for (int r = t; r < rows; r += kThreads) start[r] = __ldg(a.rowptr + r0 + r) - e0;
+  uint64_t x[E];
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    const int e = i * kThreads + t;
+    x[i] = ~0ull;
+    if (e < n) {
+      int32_t c = __ldg(a.col + e0 + e);
+      if (c < 0 || c >= a.M) {
+        atomicOr(bad, 8u);
+        c = 0;
+      }
+      x[i] = (uint64_t)(uint32_t)c << B | (uint32_t)e;
+    }
+  }
+  reg_bitonic<uint64_t, E, kThreads>(x, t, key);
+  __syncthreads();
+  key[t] = x[E - 1];  // the last key of each thread, for the next one
+  __syncthreads();
+  const uint64_t before = t ? key[t - 1] : 0;
+  uint32_t firsts = 0;
+#pragma unroll
+  for (int i = 0; i < E; ++i)
+    firsts |= (uint32_t)(t * E + i < n && ((i == 0 && t == 0) ||
+                                           (x[i] >> B) != ((i ? x[i ? i - 1 : 0] : before) >> B)))
+              << i;
+  int total;
+  const int r = cta_scan(__popc(firsts), part, &total) - 1;
+#pragma unroll
+  for (int i = 0; i < E; ++i)
+    if (t * E + i < n)
+      rank[(int)(x[i] & (kSortEdges - 1))] = (uint16_t)(r + __popc(firsts & ((2u << i) - 1)));
+  __syncthreads();
+  for (int i = t; i < n; i += kThreads) {
+    e2c[e0 + i] = rank[i];
+    e2r[e0 + i] = (int32_t)(r0 + row_of(start, rows, i));
+  }
+  if (t == 0) bp[w] = (total + a.W - 1) / a.W;
+  __syncthreads();
+}
+
 __device__ void count_large(const Csr& a, int32_t w, int32_t e0, int32_t n, uint8_t* sm,
                             int32_t* e2c, int32_t* e2r, int32_t* bp, uint32_t* bad) {
   uint32_t* bm = reinterpret_cast<uint32_t*>(sm);                     // kSweepCols bits
@@ -578,7 +633,7 @@ __global__ void __launch_bounds__(kGroup, 8)
       window_edges(a, w, e0, n);
       if (n <= 8 * kGroup)
         count_small<K, 8>(a, w, e0, n, sm, t, e2c, e2r, bp, bad);
-      else if constexpr (sizeof(K) == 4)
+      else
         count_small<K, 16>(a, w, e0, n, sm, t, e2c, e2r, bp, bad);
     }
     return;
@@ -616,7 +671,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     int32_t e0, n;
     const int32_t w = listed(count, list, room, i);
     window_edges(a, w, e0, n);
-    count_large(a, w, e0, n, dyn, e2c, e2r, bp, bad);
+    // (a sweep over the columns takes about 5 us of the SM, the sorts 18, 38 and 80 us)
+    const int sweeps = (int)(((int64_t)a.M + kSweepCols - 1) / kSweepCols);
+    if (n <= 4 * kThreads && sweeps > 3) count_sorted<4>(a, w, e0, n, dyn, e2c, e2r, bp, bad);
+    else if (n <= 8 * kThreads && sweeps > 7) count_sorted<8>(a, w, e0, n, dyn, e2c, e2r, bp, bad);
+    else if (n <= 16 * kThreads && sweeps > 15) count_sorted<16>(a, w, e0, n, dyn, e2c, e2r, bp, bad);
+    else count_large(a, w, e0, n, dyn, e2c, e2r, bp, bad);
     if (threadIdx.x == 0) next = gridDim.x + atomicAdd(ticket, 1);
     __syncthreads();
     i = next;

@@ -103,3 +103,28 @@ def test_unsorted_windows_with_hot_columns(cuda, n, H, W):
     for k in ("RowWindowOffset", "TCblockRowid", "TCblocktileId", "TCblockoffset", "SparseAToX",
               "blockPartition", "edgeToColumn", "edgeToRow", "TCvalues"):
         np.testing.assert_array_equal(getattr(got, k).cpu().numpy(), exp[k], err_msg=k)
+
+
+@pytest.mark.parametrize("M", [2 ** 20 + 1, 2 ** 22 + 3, 2 ** 23 + 5])
+@pytest.mark.parametrize("H", [1, 16, 64])
+def test_large_windows_of_many_columns(cuda, M, H):
+    """Matrices of more columns than one bitmap has bits: windows sorted by a CTA up to a size that
+    grows with the columns, beyond it ranked by several bitmaps."""
+    from dtc_b200 import metcf
+    rng = np.random.default_rng(M + H)
+    nwin = (M + H - 1) // H
+    counts = [1024, 1025, 2047, 2048, 2049, 4096, 4097, 8192, 8193, 16384, 16385, 30000]
+    row = np.concatenate([np.minimum((nwin - 1) * (i + 1) // len(counts) * H + rng.integers(0, H, n), M - 1)
+                          for i, n in enumerate(counts)])
+    col = rng.integers(0, M, row.size)
+    col[rng.random(row.size) < 0.1] = M - 1
+    o = np.lexsort((col, row))
+    row, col = row[o], col[o].astype(np.int32)
+    rowptr = np.searchsorted(row, np.arange(M + 1)).astype(np.int32)
+    val = rng.random(col.size).astype(np.float32)
+    got = metcf.convert(rowptr, col, M, H=H, W=4, values=val)
+    exp = O.metcf(rowptr, col, M, H=H, W=4, values=val)
+    assert got.T == exp["T"]
+    for k in ("RowWindowOffset", "TCblockRowid", "TCblocktileId", "TCblockoffset", "SparseAToX",
+              "blockPartition", "edgeToColumn", "edgeToRow", "TCvalues"):
+        np.testing.assert_array_equal(getattr(got, k).cpu().numpy(), exp[k], err_msg=k)
