@@ -74,12 +74,9 @@ float* slot_region(void* ws, size_t bytes, size_t offset, int64_t T, int32_t N, 
   offset += (size_t)(-((intptr_t)ws + (intptr_t)offset) & 15);
   if (offset >= bytes) return nullptr;
   char* q = (char*)ws + offset;
-  // fewer slots than chunks: as many chunks as there are slots (spmm_run), from one per SM
-  // on. R-MAT 2^20, N = 128, a workspace for 32 tiles per SM: 1.5 ms, 8.7 without slots (the
-  // CTA of a long window's first piece runs all the others).
   const int64_t fit = (int64_t)((bytes - offset) / ((size_t)H * N * sizeof(float)));
   const int64_t want = direct_chunks(T);
-  if (fit < want && fit < num_sms()) return nullptr;
+  if (fit == 0) return nullptr;
   *n = fit < want ? fit : want;
   return (float*)q;
 }

@@ -14,7 +14,7 @@ struct Epilogue {
 
 // C = act(A B + bias) on ME-TCF arrays of block shape H x W. `slots`: workspace for
 // the pieces of windows that chunk boundaries cut, H x N floats for each of
-// `nslots` chunks, or null (one CTA then runs such a window's pieces in turn).
+// `nslots` chunks, or null (clusters of CTAs then add the pieces up, with the same bits).
 dtc_status spmm_run(const int32_t* rwo, const uint8_t* tile, const int32_t* toff,
                     const int32_t* s2x, const float* vals, int32_t M, int32_t nwin, int64_t T,
                     int bformat, const void* b0, const void* b1, int32_t N, int precision, float* C,
@@ -26,8 +26,8 @@ size_t direct_slots_bytes(int64_t T, int32_t N, int H);
 // The tiles of a required region of `n` of them from its first 16-byte boundary on (the widths
 // that are multiples of 4 are written 8 and 16 bytes at a time): one less off that boundary.
 float* aligned_tiles(void* region, int32_t N, int64_t* n);
-// The slots at byte `offset` of a caller workspace: `n` of them, a slot per chunk or, from
-// one per SM on, as many as fit; null when those do not fit.
+// The slots at byte `offset` of a caller workspace: `n` of them, a slot per chunk or as many
+// as fit; null when none does.
 float* slot_region(void* ws, size_t bytes, size_t offset, int64_t T, int32_t N, int H, int64_t* n);
 // Tiles of the partials region that strict balance requires for `grid` chunks
 // (0 = 16 per SM), and its bytes.

@@ -70,7 +70,9 @@ extern "C" dtc_status dtc_spmm_balance_noalloc(const int32_t* d_tcblockRowid,
   int grid = num_sms();
   if ((int64_t)grid > num_blocks) grid = (int)(num_blocks > 0 ? num_blocks : 1);
   const size_t rwo_bytes = align_up((size_t)(nwin + 1) * 4, 256);
-  const size_t part_bytes = (N % 4 == 0) ? (size_t)2 * grid * 16 * (size_t)N * 4 : 0;
+  // (other widths run without the tiles where they do not fit)
+  size_t part_bytes = (size_t)2 * grid * 16 * (size_t)N * 4;
+  if (N % 4 != 0 && rwo_bytes + part_bytes > kScratchBytes) part_bytes = 0;
   if (rwo_bytes + part_bytes > kScratchBytes) {
     set_error("dtc_spmm_balance_noalloc: needs " + std::to_string(rwo_bytes + part_bytes) +
               " bytes of scratch (4*(ceil(num_nodes/16)+1) rounded to 256, plus 128*N per SM) "

@@ -137,13 +137,6 @@ dtc_status spmm_run(const int32_t* rwo, const uint8_t* tile, const int32_t* toff
     return DTC_OK;
   }
   if (N % 4 == 0) DTC_REQUIRE(((uintptr_t)C & 15) == 0, "C must be 16-byte aligned");
-  const Chunks c = chunks_of(T);
-  const bool limited = slots && c.g > nslots;
-  p.slots = slots;
-  p.G = (int)(limited ? nslots : c.g);
-  p.G1 = limited ? 0 : (int)c.g1;
-  p.lmax = (int32_t)(p.G1 ? T * 3 / 4 / p.G1 + 1 : (T + p.G - 1) / p.G);
-  const bool four = precision == DTC_PREC_SPLIT4;
   // tcgen05 (spmm_umma.cuh) beyond 128 features, where an instruction fills its 128
   // rows twice per gathered block, and from 65 on where the mma.sync kernel needs twice
   // the instructions per block (32-row windows; the two planes of BF16X2). ms, mma.sync /
@@ -151,6 +144,18 @@ dtc_status spmm_run(const int32_t* rwo, const uint8_t* tile, const int32_t* toff
   // 0.84 / 0.91; 32 x 8: fp32 1.25 / 0.90, BF16X2 1.63 / 1.03, BF16 1.27 / 0.96; stencil
   // 100^3 N = 256, 16 x 8: fp32 1.45 / 1.19, BF16X2 1.60 / 1.24, BF16 1.22 / 1.03.
   const bool umma = N > 128 || (N > 64 && (H == 32 || bformat == DTC_B_BF16X2));
+  // Fewer slots than chunks: as many chunks as there are slots. So few that the product leaves SMs
+  // idle are left alone: R-MAT 2^18, 2 per SM / none, ms: fp32 N = 128 0.56 / 0.68; on tcgen05 (a
+  // pipeline per CTA) N = 256 1.96 / 0.98, BF16X2 N = 128 1.26 / 0.67. R-MAT 2^20, fp32 N = 128, 32
+  // per SM 1.5 / 2.4.
+  const Chunks c = chunks_of(T);
+  if (slots && c.g > nslots && nslots < (umma ? 8 : 2) * num_sms()) slots = nullptr;
+  const bool limited = slots && c.g > nslots;
+  p.slots = slots;
+  p.G = (int)(limited ? nslots : c.g);
+  p.G1 = limited ? 0 : (int)c.g1;
+  p.lmax = (int32_t)(p.G1 ? T * 3 / 4 / p.G1 + 1 : (T + p.G - 1) / p.G);
+  const bool four = precision == DTC_PREC_SPLIT4;
   switch (bformat) {
     case DTC_B_F32:
       if (N % 4) return direct_f32_odd(p, W, st);

@@ -42,8 +42,7 @@
 // its piece, sets a flag, the warp to its left adds its own). A window cut by a chunk
 // boundary leaves its first piece in C and each later chunk's piece in that chunk's
 // slot of the workspace; k_add_slots adds them in chunk order. Without a workspace
-// the CTA of the first piece runs the following chunks of that window too and adds
-// them in the same order, so the bits are the same.
+// (SEQ) clusters of kTeam CTAs take the chunks: see kTeam.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -158,6 +157,107 @@ __device__ __forceinline__ void chunk_cuts(const DirectParams& p, int32_t k, int
   } else {
     b1 = cut_at(p, x1, i.y, p.lmax);
   }
+}
+
+// Chunks without a workspace. A cluster of kTeam CTAs runs kTeam chunks in a row, one each, and
+// keeps their pieces of cut windows in shared memory, where the cluster adds them to the first
+// piece (in C), in chunk order: the same sums and bits as k_add_slots. A cut window belongs to
+// the cluster whose chunks hold its start. Where it goes on beyond the cluster's last chunk the
+// cluster runs its pieces of the next kTeam chunks, round after round, up to its end; those
+// chunks' own clusters leave these pieces out. (One CTA for all chunks of windows that follow
+// each other without an uncut boundary: R-MAT 2^20, N = 128, fp32 8.7 ms, this 2.4; with a
+// workspace 1.44.)
+constexpr int kTeam = 8;
+// The boundaries base .. base + kTeam of chunks, by all warps of a CTA.
+__device__ __forceinline__ void team_cuts(const DirectParams& p, int32_t base, Cut* s, int warp,
+                                          int warps, int lane) {
+  for (int i = 2 * warp; i <= kTeam; i += 2 * warps) {
+    const int32_t x0 = base + i < p.G ? chunk_start(p, base + i) : p.T;
+    const int32_t x1 = base + i + 1 < p.G ? chunk_start(p, base + i + 1) : p.T;
+    const int2 a = search2(p.rwo, 0, p.nwin, min(x0, p.T - 1) + 1, 0, p.nwin, min(x1, p.T - 1) + 1, lane);
+    if (lane == 0) {
+      s[i] = x0 < p.T ? cut_at(p, x0, a.x, p.lmax) : Cut{p.T, max(a.x - 1, 0), false};
+      if (i < kTeam) s[i + 1] = x1 < p.T ? cut_at(p, x1, a.y, p.lmax) : Cut{p.T, max(a.y - 1, 0), false};
+    }
+  }
+}
+// A round of a cluster: the first one (of its own chunks), or of window `only`'s next chunks.
+struct Round {
+  int32_t only, foreign;  // -1: none; foreign: the window that an earlier cluster adds up
+  __device__ __forceinline__ Round(const Cut* cut, int32_t only_)
+      : only(only_), foreign(only_ < 0 && cut[0].open ? cut[0].win : -1) {}
+  // whether a piece that starts at boundary c is one of the round's
+  __device__ __forceinline__ bool has(const Cut& c) const {
+    return c.open && (only >= 0 ? c.win == only : c.win != foreign);
+  }
+  // member `rank`'s part of chunk k: the windows from c0 on, up to block hi
+  __device__ __forceinline__ void part(const DirectParams& p, const Cut* cut, int rank, int32_t k,
+                                       int lane, Cut& c0, int32_t& hi) const {
+    c0 = cut[rank];
+    hi = cut[rank + 1].pos;
+    if (only >= 0) {
+      hi = has(c0) ? min(hi, min(max(__ldg(p.rwo + only + 1), 0), p.T)) : c0.pos;
+    } else if (c0.open && c0.win == foreign) {  // what comes after it
+      const int32_t at = min(max(__ldg(p.rwo + c0.win + 1), 0), p.T - 1);
+      const int2 i = search2(p.rwo, 0, p.nwin, at + 1, 0, 0, 0, lane);
+      c0 = Cut{min(max(__ldg(p.rwo + c0.win + 1), 0), p.T), max(i.x - 1, 0), false};
+    }
+  }
+  __device__ __forceinline__ int32_t next(const Cut* cut) const {  // the next round's window
+    return has(cut[kTeam]) ? cut[kTeam].win : -1;
+  }
+  __device__ __forceinline__ uint32_t pieces(const Cut* cut) const {  // members that have one
+    uint32_t m = 0;
+    for (int r = 0; r < kTeam; ++r) m |= (uint32_t)has(cut[r]) << r;
+    return m;
+  }
+};
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float ld_peer(uint32_t addr, int rank) {  // a peer's shared memory
+  uint32_t a;
+  float v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+// The end of a round: adds up its pieces, H x width floats each at `tile` of the members' shared
+// memory, columns from col0 on. Returns the next round's window, -1: the CTA is done (a member
+// without a piece need not wait for the others then). Called by all threads.
+__device__ __forceinline__ int32_t end_round(const DirectParams& p, const Cut* cut, const Round& round,
+                                             const float* tile, int width, int col0, int rank, int t,
+                                             int threads) {
+  const uint32_t at = smem_u32(tile), pieces = round.pieces(cut);
+  const int32_t next = round.next(cut);
+  if (pieces == 0 || (next < 0 && !(pieces >> rank & 1))) return next;
+  const uint32_t who = next < 0 ? pieces : (1u << kTeam) - 1;  // members that add
+  cluster_sync();  // every member's pieces are there
+  t += __popc(who & ((1u << rank) - 1)) * threads;
+  threads *= __popc(who);
+  for (int r = 0; r < kTeam;) {
+    if (!round.has(cut[r])) {
+      ++r;
+      continue;
+    }
+    const int32_t w = cut[r].win;
+    int e = r + 1;  // pieces r .. e - 1 are of one window
+    while (e < kTeam && cut[e].open && cut[e].win == w) ++e;
+    const bool ends = !(cut[e].open && cut[e].win == w);
+    const int64_t row0 = (int64_t)w * p.H;
+    const int rows = (int)min((int64_t)p.H, p.M - row0);
+    for (int x = t; x < rows * width; x += threads) {
+      const int f = col0 + x % width;
+      if (f >= p.N) continue;
+      float* const c = p.C + (row0 + x / width) * p.N + f;
+      float acc = *c;
+      for (int q = r; q < e; ++q) acc += ld_peer(at + x * 4, q);
+      *c = ends ? finish(p, acc, f) : acc;
+    }
+    r = e;
+  }
+  cluster_sync();  // the pieces are read, and what they were added to is written
+  return next;
 }
 
 // Adds the pieces of every window that chunk boundaries cut to the first piece (in C), in
@@ -304,14 +404,13 @@ struct Shape {
   static constexpr int kWarp = P * kStep + kA;
   static constexpr int kAcc = kQ * kJ * MH * 4;     // accumulators per lane
   static constexpr int kSmem = NW * kWarp;
-  static constexpr int kSmemChain = NW * kAcc * 128;  // pieces in shared memory (no workspace)
   static constexpr int PB = P / SUB;                // blocks per group
   static_assert(P == 4 && P % SUB == 0, "four phases");
 };
 
 constexpr int kPre = 4;  // tile ids / values per lane loaded one group ahead (128 entries)
 
-template <int FORM, bool FOUR, int NF, int MH, int SUB, int NW, int P, int CTAS>
+template <int FORM, bool FOUR, int NF, int MH, int SUB, int NW, int P, int CTAS, bool SEQ>
 __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParams p) {
   using S = Shape<FORM, NF, MH, SUB, NW, P>;
   constexpr int BW = 8 * SUB, PB = S::PB, Q = S::kQ, J = S::kJ;
@@ -323,7 +422,6 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
   const int wr = warp / p.wf, nranges = NW / p.wf;
   const int col0 = (blockIdx.y * p.wf + warp % p.wf) * NF;
   const bool full = col0 + NF <= p.N;  // every feature of the slice exists
-  const bool seq = p.slots == nullptr;  // no workspace: pieces of a cut window in sequence
   if (threadIdx.x < NW) flags[threadIdx.x] = 0;
   __syncthreads();
 
@@ -332,7 +430,9 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
   uint8_t* const abuf = ringp + P * S::kStep;
   auto lds16 = [](const uint8_t* a) { return *reinterpret_cast<const uint4*>(a); };
   auto lds8 = [](const uint8_t* a) { return *reinterpret_cast<const uint2*>(a); };
-  float* chain = reinterpret_cast<float*>(smem + S::kSmem) + warp * S::kAcc * 32;
+  const int32_t cta_col0 = blockIdx.y * p.wf * NF;
+  float* const piece = reinterpret_cast<float*>(smem + S::kSmem);  // (SEQ) H x tw floats
+  const int tw = p.wf * NF;
   float acc[Q][J][MH][4];
   // Copies: 8 lanes read one row's 128 (64) consecutive bytes, lane l chunk l % 8 of rows
   // 2 (l / 8) and the next. Places of chunk c, chosen so that neither the copies nor the
@@ -426,37 +526,39 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
             fn(h * 16 + hh * 8 + gr, col0 + q * 64 + j * 8 + 2 * gc, acc[q][j][h][2 * hh],
                acc[q][j][h][2 * hh + 1]);
   };
-  // acc += the tile at `t` (rows of N floats, `rows` of them valid)
-  auto add_tile = [&](const float* t, int rows) {
+  // acc += the tile at `t` (rows of N floats, `rows` of them valid); `slot`: a piece's place
+  auto add_tile = [&](const float* t, int rows, bool slot) {
+    const size_t ld = SEQ && slot ? tw : p.N;
     if constexpr (FORM == kF32Odd) {
       each1([&](int r, int f, float& x) {
-        if (r < rows && f < p.N) x += t[(size_t)r * p.N + f];
+        if (r < rows && f < p.N) x += t[r * ld + f];
       });
     } else if constexpr (S::kLdsm) {
       each2([&](int r, int f, float& x, float& y) {
         if (r < rows && f < p.N) {
-          const float2 v = *reinterpret_cast<const float2*>(t + (size_t)r * p.N + f);
+          const float2 v = *reinterpret_cast<const float2*>(t + r * ld + f);
           x += v.x; y += v.y;
         }
       });
     } else {
       each4([&](int r, int f, float& x, float& y, float& z, float& w) {
         if (r < rows && f < p.N) {
-          const float4 v = *reinterpret_cast<const float4*>(t + (size_t)r * p.N + f);
+          const float4 v = *reinterpret_cast<const float4*>(t + r * ld + f);
           x += v.x; y += v.y; z += v.z; w += v.w;
         }
       });
     }
   };
-  auto store_tile = [&](float* t, int rows, bool epi) {
+  auto store_tile = [&](float* t, int rows, bool epi, bool slot) {
+    const size_t ld = SEQ && slot ? tw : p.N;
     if constexpr (FORM == kF32Odd) {
       each1([&](int r, int f, float& x) {
-        if (r < rows && f < p.N) t[(size_t)r * p.N + f] = epi ? finish(p, x, f) : x;
+        if (r < rows && f < p.N) t[r * ld + f] = epi ? finish(p, x, f) : x;
       });
     } else if constexpr (S::kLdsm) {
       each2([&](int r, int f, float& x, float& y) {
         if (r < rows && f < p.N)
-          *reinterpret_cast<float2*>(t + (size_t)r * p.N + f) =
+          *reinterpret_cast<float2*>(t + r * ld + f) =
               epi && (p.bias || p.relu) ? make_float2(finish(p, x, f), finish(p, y, f + 1))
                                         : make_float2(x, y);
       });
@@ -467,7 +569,7 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
           if (epi && (p.bias || p.relu))
             v = make_float4(finish(p, x, f), finish(p, y, f + 1), finish(p, z, f + 2),
                             finish(p, w, f + 3));
-          *reinterpret_cast<float4*>(t + (size_t)r * p.N + f) = v;
+          *reinterpret_cast<float4*>(t + r * ld + f) = v;
         }
       });
     }
@@ -484,13 +586,24 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
       for (int r = 0; r < rows; ++r) c_rows(w)[(size_t)r * p.N + f] = finish(p, 0.0f, f);
   };
 
-  for (int32_t k = blockIdx.x;; ++k) {
-    Cut c0, c1;
-    chunk_cuts(p, k, lane, c0, c1);
-    if (seq && k == (int32_t)blockIdx.x && c0.open) break;  // an earlier CTA runs this piece
-    const uint32_t mark = (uint32_t)(k - (int32_t)blockIdx.x) + 1;
+  __shared__ Cut cuts[SEQ ? kTeam + 1 : 1];
+  const int rank = SEQ ? blockIdx.x % kTeam : 0;
+  int32_t k = blockIdx.x, only = -1;
+  for (uint32_t mark = 1;; ++mark) {  // (SEQ: rounds)
+    Cut c0, c1, from;
+    int32_t hi = 0;
+    if constexpr (SEQ) {
+      team_cuts(p, k - rank, cuts, warp, NW, lane);
+      __syncthreads();
+      c0 = cuts[rank];
+      c1 = cuts[rank + 1];
+      Round(cuts, only).part(p, cuts, rank, k, lane, from, hi);
+    } else {
+      chunk_cuts(p, k, lane, c0, c1);
+    }
     // (c1.win < c0.win: only with invalid window ids)
     const int32_t len = c1.win < c0.win ? 0 : c1.pos - c0.pos;
+    float* const slot = SEQ ? piece - cta_col0 : p.slots + (size_t)k * H * p.N;
     const int nr = min(nranges, max(1, len >> 2));  // ranges of at least 4 blocks
     if (len > 0 && wr < nr && col0 < p.N) {
       // this warp's range
@@ -499,8 +612,12 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
       const int32_t most = max(len / nr / 2, 1);
       const int32_t wtop = min(c1.win + 1, p.nwin);
       const int2 si = search2(p.rwo, c0.win, wtop, x0 + 1, c0.win, wtop, min(x1, p.T - 1) + 1, lane);
-      const Cut r0 = wr == 0 ? c0 : cut_at(p, x0, si.x, most);
-      const Cut r1 = wr == nr - 1 ? c1 : cut_at(p, x1, si.y, most);
+      Cut r0 = wr == 0 ? c0 : cut_at(p, x0, si.x, most);
+      Cut r1 = wr == nr - 1 ? c1 : cut_at(p, x1, si.y, most);
+      if constexpr (SEQ) {  // (the ranges of the whole chunk: the same sums)
+        if (r0.pos < from.pos) r0 = from;
+        if (r1.pos > hi) r1 = Cut{hi, 0, false};
+      }
       const int32_t nblk = r1.pos - r0.pos;
       if (nblk > 0) {
         const int32_t nst = nblk * SUB;
@@ -858,27 +975,16 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
             const int rows = rows_of(w);
             float* out = c_rows(w);
             if (head) {
+              const bool cut = wr == 0 || w == cutw;
+              store_tile(cut ? slot : out, cut ? H : rows, false, cut);
               if (wr > 0) {  // the left neighbour adds its piece
-                if (seq) {
-#pragma unroll
-                  for (int z = 0; z < S::kAcc; ++z)
-                    chain[z * 32 + lane] = (&acc[0][0][0][0])[z];
-                } else {
-                  const bool cut = w == cutw;
-                  store_tile(cut ? p.slots + (size_t)k * H * p.N : out, cut ? H : rows, false);
-                }
                 __threadfence_block();
                 __syncwarp();
                 if (lane == 0) flags[warp] = mark;
-              } else if (seq) {
-                add_tile(out, rows);
-                store_tile(out, rows, true);
-              } else {
-                store_tile(p.slots + (size_t)k * H * p.N, H, false);
               }
               head = false;
             } else {
-              store_tile(out, rows, true);
+              store_tile(out, rows, true, false);
             }
             if (wend >= nblk) {
               if (r1.pos == p.T)  // windows without blocks at the very end
@@ -922,33 +1028,18 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
             }
             __syncwarp();
             __threadfence_block();
-            if (seq) {
-              const float* from = chain + p.wf * S::kAcc * 32;
-#pragma unroll
-              for (int z = 0; z < S::kAcc; ++z) (&acc[0][0][0][0])[z] += from[z * 32 + lane];
-            } else {
-              add_tile(cut ? p.slots + (size_t)k * H * p.N : out, cut ? H : rows);
-            }
+            add_tile(cut ? slot : out, cut ? H : rows, cut);
           }
           // does the window end inside the chunk?
           const bool ends_here = wend + r0.pos <= c1.pos;
-          if (head && wr > 0) {
-            if (seq) {
-#pragma unroll
-              for (int z = 0; z < S::kAcc; ++z) chain[z * 32 + lane] = (&acc[0][0][0][0])[z];
-            } else {
-              store_tile(cut ? p.slots + (size_t)k * H * p.N : out, cut ? H : rows, false);
-            }
+          if (head) {
+            const bool own = wr == 0 || cut;
+            store_tile(own ? slot : out, own ? H : rows, false, own);
             __threadfence_block();
             __syncwarp();
-            if (lane == 0) flags[warp] = mark;
-          } else if (head && !seq) {
-            store_tile(p.slots + (size_t)k * H * p.N, H, false);
-          } else if (head) {
-            add_tile(out, rows);
-            store_tile(out, rows, ends_here);
+            if (wr > 0 && lane == 0) flags[warp] = mark;
           } else {
-            store_tile(out, rows, ends_here);
+            store_tile(out, rows, ends_here, false);
           }
         }
       }
@@ -957,8 +1048,14 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
       __syncwarp();
       if (lane == 0) flags[warp] = mark;
     }
-    if (!seq || !c1.open) break;
-    __syncthreads();  // the next piece adds to what this one wrote
+    if constexpr (!SEQ) {
+      break;
+    } else {
+      only = end_round(p, cuts, Round(cuts, only), piece, tw, cta_col0, rank, threadIdx.x, NW * 32);
+      if (only < 0) break;
+      __syncthreads();  // (the next round's cuts)
+      k += kTeam;
+    }
   }
   if (p.stamps) {
     __syncthreads();
@@ -977,25 +1074,60 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
 
 constexpr int kP = 4;
 
-template <int FORM, bool FOUR, int NF, int MH, int SUB, int CTAS>
-dtc_status launch(DirectParams& p, cudaStream_t st) {
-  using S = Shape<FORM, NF, MH, SUB, kNW, kP>;
-  auto* fn = k_spmm_direct<FORM, FOUR, NF, MH, SUB, kNW, kP, CTAS>;
-  const int smem = S::kSmem + (p.slots ? 0 : S::kSmemChain);
-  static_assert(S::kSmem + S::kSmemChain <= 232448, "dynamic shared memory per CTA");
-  static bool attr_set[64] = {};
+// A kernel on clusters of kTeam CTAs along x (SEQ), or on single ones.
+template <bool SEQ>
+dtc_status launch_ctas(void (*fn)(DirectParams), const DirectParams& p, unsigned slices, int threads,
+                       int smem, int most, cudaStream_t st, bool (&attr_set)[64]) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev & 63]) {
-    DTC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  S::kSmem + S::kSmemChain));
+    DTC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     attr_set[dev & 63] = true;
   }
-  const int slices = (p.N + NF - 1) / NF;
-  p.wf = slices >= 4 ? 4 : slices >= 2 ? 2 : 1;
-  const dim3 grid((unsigned)p.G, (unsigned)((slices + p.wf - 1) / p.wf));
-  fn<<<grid, kNW * 32, smem, st>>>(p);
+  if constexpr (SEQ) {
+    cudaLaunchConfig_t c = {};
+    cudaLaunchAttribute a;
+    a.id = cudaLaunchAttributeClusterDimension;
+    a.val.clusterDim.x = kTeam;
+    a.val.clusterDim.y = a.val.clusterDim.z = 1;
+    c.gridDim = dim3((unsigned)((p.G + kTeam - 1) / kTeam * kTeam), slices);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    DTC_CUDA(cudaLaunchKernelEx(&c, fn, p));
+  } else {
+    fn<<<dim3((unsigned)p.G, slices), threads, smem, st>>>(p);
+  }
   DTC_CUDA(cudaGetLastError());
+  return DTC_OK;
+}
+
+// `slices`: feature slices of the form with a workspace, which set the ranges per chunk.
+template <int FORM, bool FOUR, int NF, int MH, int SUB, int CTAS, bool SEQ>
+dtc_status launch_form(DirectParams& p, int slices, cudaStream_t st) {
+  using S = Shape<FORM, NF, MH, SUB, kNW, kP>;
+  constexpr int kPiece = 16 * MH * NF * 4;  // per slice of features
+  static_assert(S::kSmem + 4 * kPiece <= 232448 - 2048, "shared memory per CTA");
+  static bool attr_set[64] = {};
+  p.wf = slices >= 4 ? 4 : slices >= 2 ? 2 : 1;
+  slices = (p.N + NF - 1) / NF;
+  return launch_ctas<SEQ>(k_spmm_direct<FORM, FOUR, NF, MH, SUB, kNW, kP, CTAS, SEQ>, p,
+                          (unsigned)((slices + p.wf - 1) / p.wf), kNW * 32,
+                          S::kSmem + (SEQ ? p.wf * kPiece : 0), S::kSmem + (SEQ ? 4 * kPiece : 0), st,
+                          attr_set);
+}
+
+template <int FORM, bool FOUR, int NF, int MH, int SUB, int CTAS>
+dtc_status launch(DirectParams& p, cudaStream_t st) {
+  // (SEQ: the pieces' place in shared memory would leave room for two CTAs of 128 features)
+  const int slices = (p.N + NF - 1) / NF;
+  const dtc_status s =
+      p.slots ? launch_form<FORM, FOUR, NF, MH, SUB, CTAS, false>(p, slices, st)
+              : launch_form<FORM, FOUR, NF == 128 ? 64 : NF, MH, SUB, NF == 128 ? 4 : CTAS, true>(
+                    p, slices, st);
+  if (s != DTC_OK) return s;
   if (p.slots && p.G > 1) {
     k_add_slots<<<add_ctas(p), kAddThreads, 0, st>>>(p);
     DTC_CUDA(cudaGetLastError());

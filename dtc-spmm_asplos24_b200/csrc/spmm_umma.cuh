@@ -93,7 +93,7 @@ struct WindowWalk {
   }
 };
 
-template <int FORM, bool FOUR, int NT, int WH, int SUB, int R, int CTAS>
+template <int FORM, bool FOUR, int NT, int WH, int SUB, int R, int CTAS, bool SEQ>
 __global__ void __launch_bounds__(kUmmaThreads, CTAS)
     k_spmm_umma(const __grid_constant__ DirectParams p) {
   using S = UShape<FORM, NT, WH, SUB, R>;
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kUmmaThreads, CTAS)
   volatile uint32_t* const abort_flag = tmem_slot + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col0 = blockIdx.y * NT * 128;
-  const bool seq = p.slots == nullptr;
+  float* const piece = reinterpret_cast<float*>(smem + S::kSmem - 1024);  // (SEQ) WH x NT * 128 floats
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < R; ++i) mbar_init(full + i, 32 + 1);  // 32 lanes' copies, the A values
@@ -143,10 +143,23 @@ __global__ void __launch_bounds__(kUmmaThreads, CTAS)
   uint32_t n = 0;    // stages of the CTA so far (over its chunks)
   uint32_t acq = 0;  // windows with blocks so far
   bool ok = true;
-  for (int32_t k = blockIdx.x; ok; ++k) {
+  __shared__ Cut cuts[SEQ ? kTeam + 1 : 1];
+  const int rank = SEQ ? blockIdx.x % kTeam : 0;
+  // (SEQ: rounds. Without them one pass; for 32-row windows a loop all the same, that is left
+  // after it: the compiler's order of the body is better then, R-MAT 2^20, N = 128, BF16X2 1.90 ms,
+  // 2.03 without; for 16-row windows it is worse, 1.90 and 1.85.)
+  constexpr bool kLoop = !SEQ && WH == 32;
+  int32_t only = -1;
+  for (int32_t k = blockIdx.x; !kLoop || ok; k += kLoop ? 1 : 0) {
     Cut c0, c1;
-    chunk_cuts(p, k, lane, c0, c1);
-    if (seq && k == (int32_t)blockIdx.x && c0.open) break;  // an earlier CTA runs this piece
+    if constexpr (SEQ) {
+      team_cuts(p, k - rank, cuts, warp, kUmmaThreads / 32, lane);
+      __syncthreads();
+      Round(cuts, only).part(p, cuts, rank, k, lane, c0, c1.pos);
+      if (!ok) c1.pos = c0.pos;
+    } else {
+      chunk_cuts(p, k, lane, c0, c1);
+    }
     const int32_t nblk = c1.pos - c0.pos;
     if (nblk > 0) {
       if (warp >= kLoad0 && warp < kTile0) {
@@ -389,10 +402,12 @@ __global__ void __launch_bounds__(kUmmaThreads, CTAS)
             break;
           }
           tc_fence_after();
-          // a piece of a cut window: to the chunk's slot, or (no workspace) onto C; the first
-          // piece, and a whole window, to C
-          const bool raw = win.end > nblk, slot = head && !seq;
-          float* const out = slot ? p.slots + (int64_t)k * tile : p.C + (int64_t)win.w * tile;
+          // a piece of a cut window: to the chunk's slot; the first piece, and a whole window, to C
+          const bool raw = win.end > nblk, slot = head;
+          float* const out = !slot ? p.C + (int64_t)win.w * tile
+                             : SEQ ? piece - col0
+                                   : p.slots + (int64_t)k * tile;
+          const int32_t ld = SEQ && slot ? NT * 128 : p.N;
           const int rows = slot ? WH : (int)min((int64_t)WH, p.M - (int64_t)win.w * WH);
 #pragma unroll 1
           for (int t = 0; t < NT; ++t) {
@@ -422,9 +437,8 @@ __global__ void __launch_bounds__(kUmmaThreads, CTAS)
 #pragma unroll
                 for (int r = 0; r < 16; ++r) {
                   if (h * 16 + r < rows) {
-                    float* const o = out + (int64_t)(h * 16 + r) * p.N + f;
-                    float x = __uint_as_float(v[r]);
-                    if (head && seq) x = *o + x;
+                    float* const o = out + (int64_t)(h * 16 + r) * ld + f;
+                    const float x = __uint_as_float(v[r]);
                     *o = slot || raw ? x : finish(p, x, f);
                   }
                 }
@@ -443,9 +457,17 @@ __global__ void __launch_bounds__(kUmmaThreads, CTAS)
       }
       n += (uint32_t)((nblk + PB - 1) / PB);
     }
-    if (!seq || !c1.open) break;
-    __syncthreads();  // the next piece adds to what this one wrote
-    ok = ok && !*abort_flag;
+    if constexpr (!SEQ) {
+      if (!kLoop || p.slots) break;
+    } else {
+      __syncthreads();
+      only = end_round(p, cuts, Round(cuts, only), piece, NT * 128, col0, rank, threadIdx.x,
+                       kUmmaThreads);
+      if (only < 0) break;
+      __syncthreads();  // (the next round's cuts)
+      k += kTeam;
+      ok = ok && !*abort_flag;
+    }
   }
   if (warp == kIssuer && lane == 0) {  // every MMA has finished before the TMEM is freed
     tc_commit(drain);
@@ -471,21 +493,22 @@ __global__ void __launch_bounds__(kUmmaThreads, CTAS)
   }
 }
 
+template <int FORM, bool FOUR, int NT, int WH, int SUB, int R, int CTAS, bool SEQ>
+dtc_status launch_umma_form(DirectParams& p, cudaStream_t st) {
+  using S = UShape<FORM, NT, WH, SUB, R>;
+  constexpr int smem = S::kSmem + (SEQ ? WH * NT * 128 * 4 : 0);
+  static_assert(smem <= 232448 - 1024 && S::kTmem * CTAS <= 512, "per-SM budget");
+  static bool attr_set[64] = {};
+  return launch_ctas<SEQ>(k_spmm_umma<FORM, FOUR, NT, WH, SUB, R, CTAS, SEQ>, p,
+                          (unsigned)((p.N + NT * 128 - 1) / (NT * 128)), kUmmaThreads, smem, smem, st,
+                          attr_set);
+}
+
 template <int FORM, bool FOUR, int NT, int WH, int SUB, int R, int CTAS>
 dtc_status launch_umma(DirectParams& p, cudaStream_t st) {
-  using S = UShape<FORM, NT, WH, SUB, R>;
-  auto* fn = k_spmm_umma<FORM, FOUR, NT, WH, SUB, R, CTAS>;
-  static_assert(S::kSmem <= 232448 && S::kTmem * CTAS <= 512, "per-SM budget");
-  static bool attr_set[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!attr_set[dev & 63]) {
-    DTC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem));
-    attr_set[dev & 63] = true;
-  }
-  const dim3 grid((unsigned)p.G, (unsigned)((p.N + NT * 128 - 1) / (NT * 128)));
-  fn<<<grid, kUmmaThreads, S::kSmem, st>>>(p);
-  DTC_CUDA(cudaGetLastError());
+  const dtc_status s = p.slots ? launch_umma_form<FORM, FOUR, NT, WH, SUB, R, CTAS, false>(p, st)
+                               : launch_umma_form<FORM, FOUR, NT, WH, SUB, 3, CTAS, true>(p, st);  // (room for the pieces)
+  if (s != DTC_OK) return s;
   if (p.slots && p.G > 1) {
     k_add_slots<<<add_ctas(p), kAddThreads, 0, st>>>(p);
     DTC_CUDA(cudaGetLastError());
