@@ -62,24 +62,31 @@ dtc_status rowid_to_rwo(const int32_t* rowid, int64_t T, int32_t nwin, int32_t* 
   return DTC_OK;
 }
 
-// Chunks of the TC-block range when no workspace limits them, from the blocks per warp of
-// a CTA (q): three chunks per SM, one wave, until a chunk has kNW * 80 blocks, then that
-// size until there are 15 per SM, then up to kNW * 192 blocks. The last quarter of the
-// blocks is cut four times finer, so that the last CTAs to start are short (R-MAT 2^19,
-// N = 128 on tcgen05: 1.10 -> 0.87 ms), except in the smallest products. A chunk costs its
-// pipeline's start and, where it cuts a window, a piece in the workspace; too few leave SMs
-// idle. us with 15 alike per SM / this: 27-point stencil 40^3, BF16, 32-row windows 117 /
-// 69, uniform 23438 x 47 116 / 89 (16-row windows 116 / 75), R-MAT 2^15 133 / 94; R-MAT
-// 2^18 with the 15 per SM that it keeps 502, with 3 580.
+// Chunks of the TC-block range when no workspace limits them.
+//   up to 1024 blocks: chunks of 8; then 128 of them until they have 32
+//   chunks of 32 blocks up to three per SM (one wave), then these until they have 64
+//   the first three quarters of the blocks in three chunks per SM until these have kNW * 80
+//   blocks, then in that size until there are 15 per SM, then in up to kNW * 192 blocks; the last
+//   quarter in chunks a quarter as long, so that the last CTAs to start are short (R-MAT 2^19,
+//   N = 128 on tcgen05: 1.10 -> 0.87 ms)
+// A chunk costs its pipeline's start and, where it cuts a window, a piece in the workspace; too few
+// leave SMs idle. us, before / with the line in question: 302 blocks, fp32 N = 256 20.7 (chunks of 32)
+// / 13.1; 24,059 blocks, fp32 N = 256 57 (3.1 per SM: a second wave) / 40; 27-point stencil 40^3,
+// BF16, 32-row windows 117 (15 alike per SM) / 69, R-MAT 2^15 133 / 94; R-MAT 2^18 with the 15 per SM
+// 502, with 3 580.
+// kMaxChunks bounds the workspace (a tile of H x N floats each), not the speed: beyond 7 M blocks
+// there are more than 60 per SM all the same.
+constexpr int64_t kMaxChunks = 16384;
 struct Chunks {
   int64_t g, g1;  // all chunks; those of the first three quarters (0: all alike)
 };
 Chunks chunks_of(int64_t T) {
-  const int64_t sms = num_sms();
-  int64_t q = std::max(std::min<int64_t>(T / (sms * 12), 80), T / (sms * 60));
-  q = q < 8 ? 8 : q > 192 ? 192 : q;
+  const int64_t sms = num_sms(), wave = 3 * sms;
+  if (T / (wave * kNW) < 16)
+    return {std::max<int64_t>({1, std::min<int64_t>(T / 8, 128), std::min(T / 32, wave)}), 0};
+  int64_t q = std::max(std::min<int64_t>(T / (wave * kNW), 80), T / (5 * wave * kNW));
+  q = std::max(std::min<int64_t>(q, 192), T / (kMaxChunks * 4 / 7 * kNW) + 1);
   const int64_t g = T / (q * kNW);
-  if (q < 16) return {g < 1 ? 1 : g, 0};
   return {g * 3 / 4 + g, g * 3 / 4};
 }
 int direct_chunks(int64_t T) { return (int)chunks_of(T).g; }
@@ -154,7 +161,11 @@ dtc_status spmm_run(const int32_t* rwo, const uint8_t* tile, const int32_t* toff
   p.slots = slots;
   p.G = (int)(limited ? nslots : c.g);
   p.G1 = limited ? 0 : (int)c.g1;
-  p.lmax = (int32_t)(p.G1 ? T * 3 / 4 / p.G1 + 1 : (T + p.G - 1) / p.G);
+  // Windows of more blocks are cut at chunk boundaries: of more than a chunk has, and than a common
+  // window of small graphs (4096 rows of 8 edges, 32-row windows of about 32 blocks, N = 512 fp32: half
+  // of them cut 44 us, none 27).
+  p.lmax = (int32_t)(p.G1 ? T * 3 / 4 / p.G1 + 1
+                          : std::max<int64_t>((T + p.G - 1) / p.G, H == 32 ? 48 : 32));
   const bool four = precision == DTC_PREC_SPLIT4;
   switch (bformat) {
     case DTC_B_F32:

@@ -167,10 +167,8 @@ def spmm_ex_launches(m: METCF, mode=0, grid=0, queue=True):
     chunk, the sum of the cut windows' pieces."""
     if m.T == 0:
         return 0
-    sms = torch.cuda.get_device_properties(m.RowWindowOffset.device).multi_processor_count
-    # blocks per range, 4 ranges per chunk (chunks_of in spmm_direct.cu)
-    q = min(max(min(m.T // (sms * 12), 80), m.T // (sms * 60), 8), 192)
-    return 1 + (1 if (queue or mode == 1) and m.T // (4 * q) > 1 else 0)
+    chunks = spmm_ex_workspace_bytes(m, 64) // (m.H * 64 * 4)  # (a slot each)
+    return 1 + (1 if (queue or mode == 1) and chunks > 1 else 0)
 
 
 def spmm_ex(m: METCF, planes, fmt, N, precision, mode=0, grid=0, use_values=True, out=None,
