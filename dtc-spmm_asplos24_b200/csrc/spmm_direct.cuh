@@ -1049,9 +1049,12 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
       if (lane == 0) flags[warp] = mark;
     }
     if constexpr (!SEQ) {
-      // (always; the odd widths in a loop all the same, which the compiler orders better: R-MAT
-      // 2^17, N = 41 311 us, 319 without)
-      if (FORM != kF32Odd || p.slots) break;
+      // (Always, as there are slots; written as the end of a loop where the compiler orders the body
+      // better with one. us, without / with: R-MAT 2^17, fp32 N = 41 319 / 311; R-MAT 2^18, FP8 N = 128
+      // 16 x 16 4 % less with, BF16 32 x 8 N = 64 6 %, fp32 N = 128 16 x 8 3 %; fp32 N = 32 2 % more,
+      // SPLIT24 32 x 8 5 % more.)
+      constexpr bool kLoop = FORM == kF32Odd || ((NF == 128 || MH == 2) && FORM != kSplit24);
+      if (!kLoop || p.slots) break;
     } else {
       only = end_round(p, cuts, Round(cuts, only), piece, tw, cta_col0, rank, threadIdx.x, NW * 32);
       if (only < 0) break;
