@@ -7,17 +7,15 @@
 //   mode   0 = window-scheduled, 1 = strict balance
 //   waves  the workspace's partial tiles, waves x SMs (balance mode stops at 16)
 //   ntile  128-feature tiles per CTA
-// The kernels cut the blocks into chunks of their own (spmm_run): with the whole
-// workspace the candidates run alike and differ by noise; with balance mode's
-// required bytes alone, `waves` bounds the chunks.
-// Each candidate runs once untimed and `reps` times between CUDA events on the
-// caller's stream; the mean is its time. Candidates change neither the B form
-// nor the product precision, only how fp32 partial sums are grouped; each
-// candidate's result is bitwise reproducible (the pieces of a cut window are
-// added in a fixed order).
+// The kernels cut the blocks into chunks of their own (spmm_run), and the workspace that
+// dtc_autotune asks for has a slot for each: all candidates are the same launch there.
+// It runs once untimed and `reps` times between CUDA events on the caller's stream, and
+// its mean is the time of every candidate; the first one is named the fastest. What
+// does change a product's time, the block shape and the B form, are the caller's arrays
+// (tune.tune_forms, costmodel.Scheduler search over them).
+#include <algorithm>
 #include <vector>
 #include "impl.h"
-
 
 using namespace dtc;
 
@@ -128,36 +126,30 @@ dtc_status dtc_autotune(const int32_t* d_rowWindowOffset, const uint8_t* d_tileI
   DTC_CUDA(cudaEventCreate(&ev.a));
   DTC_CUDA(cudaEventCreate(&ev.b));
   const int sms = num_sms();
-  int best_i = -1;
-  for (int i = 0; i < ncand; ++i) {
-    dtc_schedule& c = cand[i];
-    int64_t g = (int64_t)c.waves * sms;
-    if (g > num_blocks) g = num_blocks > 0 ? num_blocks : 1;
-    c.grid = (int32_t)g;
-    auto run = [&]() {
-      return dtc_spmm_ex(d_rowWindowOffset, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues,
-                         num_nodes, num_windows, num_blocks, block_h, block_w, bformat, d_Bplane0,
-                         d_Bplane1, N, precision, d_C, c.mode, c.grid, c.ntile, d_workspace,
-                         workspace_bytes, stream);
-    };
-    s = run();  // warm-up
+  auto run = [&]() {
+    return dtc_spmm_ex(d_rowWindowOffset, d_tileId, d_tcblockOffset, d_sparseAToX, d_tcValues,
+                       num_nodes, num_windows, num_blocks, block_h, block_w, bformat, d_Bplane0,
+                       d_Bplane1, N, precision, d_C, 0, 0, 0, d_workspace, workspace_bytes, stream);
+  };
+  s = run();  // warm-up
+  if (s != DTC_OK) return s;
+  DTC_CUDA(cudaEventRecord(ev.a, st));
+  for (int r = 0; r < reps; ++r) {
+    s = run();
     if (s != DTC_OK) return s;
-    DTC_CUDA(cudaEventRecord(ev.a, st));
-    for (int r = 0; r < reps; ++r) {
-      s = run();
-      if (s != DTC_OK) return s;
-    }
-    DTC_CUDA(cudaEventRecord(ev.b, st));
-    DTC_CUDA(cudaEventSynchronize(ev.b));
-    float ms = 0.0f;
-    DTC_CUDA(cudaEventElapsedTime(&ms, ev.a, ev.b));
+  }
+  DTC_CUDA(cudaEventRecord(ev.b, st));
+  DTC_CUDA(cudaEventSynchronize(ev.b));
+  float ms = 0.0f;
+  DTC_CUDA(cudaEventElapsedTime(&ms, ev.a, ev.b));
+  for (dtc_schedule& c : cand) {
+    c.grid = (int32_t)std::max<int64_t>(std::min<int64_t>((int64_t)c.waves * sms, num_blocks), 1);
     c.ms = ms / reps;
-    if (best_i < 0 || c.ms < cand[best_i].ms) best_i = i;
   }
   if (results)
     for (int i = 0; i < ncand && i < max_results; ++i) results[i] = cand[i];
   if (num_results) *num_results = ncand;
-  *best = best_i;
+  *best = 0;
   return DTC_OK;
 }
 

@@ -60,6 +60,10 @@ def feasible(N):
     return np.array([c["ntile"] <= auto_ntile(N, c["H"], c["W"]) for c in CLASSES], np.uint8)
 
 
+# What a reorder has to gain over the caller's own order before it is chosen: it renumbers the
+# rows and takes longer than hundreds of products (three products per class differ by 1 to 2 %).
+REORDER_GAIN = 1.03
+
 _INDEX = {(c["mode"], c["waves"], c["ntile"], c["form"], c["reorder"], c["H"], c["W"]): i
           for i, c in enumerate(CLASSES)}
 
@@ -420,9 +424,10 @@ class Scheduler:
 
     def plan(self, rowptr, col, m: metcf.METCF, N, exhaustive=False, B=None, reps=3,
              verify_top=0):
-        """The class to run. With verify_top = k > 1 the model's k cheapest
-        predicted classes are timed on the caller's data and the fastest wins
-        (model-guided search: k measurements instead of all K classes)."""
+        """The class to run. With verify_top = k > 1 the launches of the model's k
+        cheapest predicted classes are timed on the caller's data and the fastest
+        wins. Classes that differ in mode, waves or N-tile alone are one launch: all
+        K classes are twelve, so that verify_top = K is the exhaustive choice."""
         if self.net is not None and not exhaustive:
             f = features(rowptr, col, m, N).reshape(1, -1)
             if verify_top > 1:
@@ -444,16 +449,22 @@ class Scheduler:
 
     @staticmethod
     def _fastest(rowptr, col, m, N, B, reps, classes):
-        """Times the given classes on this matrix (CUDA events) and returns the fastest."""
+        """Times the launches that the given classes name (block shape, B form, reorder; the
+        kernels cut their own chunks) on this matrix (CUDA events), each once, and returns the
+        first class of the fastest."""
         dev = m.RowWindowOffset.device
         if B is None:
             B = torch.randn((m.M, N), device=dev)
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
         mets, perms, best, best_c = {}, {}, None, None
         out = torch.empty((m.M, N), dtype=torch.float32, device=dev)
+        seen = set()
         for c in classes:
             k = CLASSES[c]
             key = (k["reorder"], k["H"], k["W"])
+            if key + (k["form"],) in seen:
+                continue
+            seen.add(key + (k["form"],))
             if key not in mets:
                 if k["reorder"]:
                     if "p" not in perms:
@@ -476,7 +487,7 @@ class Scheduler:
                 tune.run(mm, planes, fmt, N, prec, sched, out=out, workspace=ws)
             e1.record()
             torch.cuda.synchronize()
-            ms = e0.elapsed_time(e1) / reps
+            ms = e0.elapsed_time(e1) / reps * (REORDER_GAIN if k["reorder"] else 1.0)
             if best is None or ms < best:
                 best, best_c = ms, c
         return best_c
@@ -501,8 +512,9 @@ class Scheduler:
                     ok = feasible(N)
                     for sc in scheds:  # the fastest schedule inside the class space
                         key = (sc.mode, sc.waves, sc.ntile, fo, ro, h, w)
-                        if key in _INDEX and ok[_INDEX[key]] and (best is None or sc.ms < best):
-                            best, best_c = sc.ms, _INDEX[key]
+                        ms = sc.ms * (REORDER_GAIN if ro else 1.0)
+                        if key in _INDEX and ok[_INDEX[key]] and (best is None or ms < best):
+                            best, best_c = ms, _INDEX[key]
         return best_c
 
 
