@@ -91,9 +91,12 @@ def measured_traffic(workload, kernel):
     p = os.path.join(ROOT, "profiles", f) if f else None
     if not p or not os.path.exists(p):
         return None
+    # the launch is the form, the block shape and the reorder (mode, waves and N-tile are not)
+    launch = lambda k: (k.split("_mode")[0], k.endswith("_tca"))  # noqa: E731
     for line in open(p):
         cells = [x.strip().strip("`") for x in line.strip().strip("|").split("|")]
-        if len(cells) >= 2 and cells[0] == kernel and cells[1].replace(",", "").isdigit():
+        if len(cells) >= 2 and "_mode" in cells[0] and launch(cells[0]) == launch(kernel) and \
+                cells[1].replace(",", "").isdigit():
             return int(cells[1].replace(",", ""))
     return None
 
@@ -475,23 +478,19 @@ def run_balance_report(args):
             grid = min(16 * sms, m.T)
             full = metcf.spmm_ex_workspace_bytes(m, N, mode, grid)
             for queue in (True, False):
-                wsb = full if queue else max(full - _queue_bytes(m, grid), 0)
+                # (without slots: the bytes that the mode requires)
+                wsb = full if queue else full - metcf.spmm_ex_workspace_bytes(m, N, 0, grid)
                 ws = torch.empty(max(wsb, 1), dtype=torch.uint8, device=dev)
                 fn = lambda: metcf.spmm_ex(m, planes, fmt, N, prec, mode=mode, grid=grid,
-                                           out=out, workspace=ws if wsb else None)
+                                           out=out, workspace=ws)
                 for _ in range(3):
                     fn()
-                r = balance.cta_report(fn, capacity=max(grid, sms, m.T // 400) + 8, device=dev)
+                # every chunk and feature slice has a record (at most 16384 chunks and a cluster)
+                r = balance.cta_report(fn, capacity=16400 * ((N + 31) // 32), device=dev)
                 rows[f"{form}_h32_mode{mode}_{'slots' if queue else 'no-slots'}"] = r
     line = {"metric": "per-CTA busy time of one SpMM launch (us)", "workload": name,
             "nnz": A.nnz, "T": m.T, "chunks": min(16 * sms, m.T), "schedules": rows}
     print(json.dumps(line), flush=True)
-
-
-def _queue_bytes(m, grid):
-    """Bytes of the chunk slots spmm_ex_workspace_bytes includes."""
-    from dtc_b200 import metcf
-    return metcf.spmm_ex_workspace_bytes(m, 128, 0, grid)
 
 
 # ------------------------------------------------------------------ our arm
@@ -610,8 +609,8 @@ def main():
         results[k] = {"ms": ms, "gflops": flops / (ms * 1e-3) / 1e9,
                       "hbm_frac": nbytes / (float(np.mean(per)) * 1e-3) / 1e9 / peaks["hbm_gbs"],
                       "bytes_per_B_elem": eb}
-    # autotuned schedules: every (mode, chunks, N-tile) at block shapes 16 x 8, 32 x 8 and
-    # 16 x 16 for the plain TF32 drop-in and for the two B forms within 1e-5 (dtc_autotune)
+    # dtc_autotune at block shapes 16 x 8, 32 x 8 and 16 x 16 for the plain TF32 drop-in and
+    # for the B forms within 1e-5
     from dtc_b200 import tune, costmodel, reorder as reorder_mod
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     mets = {(16, 8): m,
@@ -631,13 +630,12 @@ def main():
     shape_name = lambda hw: f"h{hw[0]}w{hw[1]}"
     exh_key = min((k for k in tuned_tbl if k[0] != "tf32"), key=lambda k: tuned_tbl[k].ms)
 
-    # the learned scheduler's choice (features -> MLP on the GPU, its 8 cheapest
-    # predicted classes timed on this matrix); the exhaustive autotuner is its
-    # fallback when no weights match the class space
+    # the scheduler's choice: every launch that its classes name (block shape, B form
+    # within 1e-5, TCA reorder or not) timed on this matrix
     t0 = time.perf_counter()
     plan = costmodel.Scheduler(device=dev).plan(torch.from_numpy(A.rowptr).to(dev),
                                                 torch.from_numpy(A.col).to(dev), m, N, B=B,
-                                                verify_top=8)
+                                                verify_top=costmodel.K)
     plan_s = time.perf_counter() - t0
     perm = None
     At = A
@@ -719,7 +717,8 @@ def main():
                 "metcf_bytes": S, "compulsory_bytes": S + A.K * N * eb_t + A.M * N * 4,
                 "kernel": tuned, "kernel_ms": kern_ms,
                 "note": "achieved = algorithmic bytes (ME-TCF + distinct gathered B rows + C) / "
-                        "mean step time; dram_frac = measured DRAM bytes / the same time"}
+                        "mean step time: gathered rows that L2 holds count too, so frac may pass "
+                        "1; dram_frac = measured DRAM bytes / the same time"}
 
     # end to end through the public API with host buffers: pinned fp32 B ->
     # device (row gather when reordered) -> storage-form pack -> SpMM -> pinned
