@@ -102,8 +102,8 @@ const float* values_ptr(const c10::optional<torch::Tensor>& values, int64_t nnz)
   return v.data_ptr<float>();
 }
 
-// Plans the reference accepts (DTCSpMM_kernel.cu:840-930); all run the
-// tcgen05 kernel here (vector width / N split are not parameters of it).
+// Plans the reference accepts (DTCSpMM_kernel.cu:840-930); all run the same
+// kernels here (vector width / N split are not parameters of them).
 // "mma_sync" selects the legacy-ISA kernel.
 bool legacy_plan(const std::string& plan) {
   static const char* ok[] = {"float_nonsplit", "float2_nonsplit", "float2_split",

@@ -65,10 +65,10 @@ dtc_status rowid_to_rwo(const int32_t* rowid, int64_t T, int32_t nwin, int32_t* 
 // Chunks of the TC-block range when no workspace limits them.
 //   up to 1024 blocks: chunks of 8; then 128 of them until they have 32
 //   chunks of 32 blocks up to three per SM (one wave), then these until they have 64
-//   the first three quarters of the blocks in three chunks per SM until these have kNW * 80
-//   blocks, then in that size until there are 15 per SM, then in up to kNW * 192 blocks; the last
-//   quarter in chunks a quarter as long, so that the last CTAs to start are short (R-MAT 2^19,
-//   N = 128 on tcgen05: 1.10 -> 0.87 ms)
+//   beyond, chunks of a third of an SM's share until that is kNW * 80 blocks, of that size until
+//   it is a fifteenth of a share, then up to kNW * 192 blocks; the last quarter of the blocks in
+//   chunks a quarter as long, so that the last CTAs to start are short (R-MAT 2^19, N = 128 on
+//   tcgen05: 1.10 -> 0.87 ms): 5.25 and 26 chunks per SM in all
 // A chunk costs its pipeline's start and, where it cuts a window, a piece in the workspace; too few
 // leave SMs idle. us, before / with the line in question: 302 blocks, fp32 N = 256 20.7 (chunks of 32)
 // / 13.1; 24,059 blocks, fp32 N = 256 57 (3.1 per SM: a second wave) / 40; 27-point stencil 40^3,

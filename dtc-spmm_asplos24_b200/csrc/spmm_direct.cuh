@@ -908,7 +908,7 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
                 for (int j = 0; j < 8; ++j) {
                   const uint32_t sel = j & 1 ? 0x7632 : 0x5410;
                   bh[j] = __byte_perm(xh[j >> 1], yh[j >> 1], sel);
-                  if constexpr (FORM == kBF16 || FORM == kFP8) {  // lo = 0
+                  if constexpr (FORM == kFP8) {  // lo = 0
 #pragma unroll
                     for (int h = 0; h < MH; ++h)
                       mma_bf16_k16(acc[q][j][h], ah[h][0], ah[h][1], al[h][0], al[h][1], bh[j],
@@ -925,7 +925,7 @@ __global__ void __launch_bounds__(NW * 32, CTAS) k_spmm_direct(const DirectParam
                     }
                   }
                 }
-                if constexpr ((FORM == kBF16X2 || FORM == kSplit24) && !FOUR) {
+                if constexpr (FORM == kSplit24 && !FOUR) {
 #pragma unroll
                   for (int j = 0; j < 8; ++j)
 #pragma unroll
@@ -1142,7 +1142,8 @@ dtc_status launch(DirectParams& p, cudaStream_t st) {
 
 template <int FORM, bool FOUR, int MH, int SUB>
 dtc_status by_width(DirectParams& p, cudaStream_t st) {
-  // (32 features of acc at 5 CTAs, 64 at 4 and 128 at 3: what the registers allow)
+  // (32 features of acc at 5 CTAs, 64 at 4 and 128 at 3: what the registers allow, but for 4 to
+  // 28 bytes that a dozen of the instances spill)
   if constexpr (FORM == kF32 || FORM == kF32Odd) {
     if (p.N <= 32) return launch<FORM, FOUR, 32, MH, SUB, MH == 2 ? 4 : 5>(p, st);
   }

@@ -1,8 +1,8 @@
 // Legacy-ISA TC-block SpMM: mma.sync.m16n8k8 TF32 with B gathered straight
 // into registers, one CTA per row window -- the instruction family and
 // schedule of the reference kernels (DTC-SpMM/DTCSpMM_kernel.cu:2663-2866),
-// written for any N >= 1 with full bounds checks. Used for shapes the TMA
-// path cannot take (N % 4 != 0) and as the recompiled-legacy comparison point.
+// written for any N >= 1 with full bounds checks: the recompiled-legacy
+// comparison point (plan "mma_sync", dtc_spmm_mma_sync).
 #include "common.cuh"
 
 namespace dtc {

@@ -8,8 +8,8 @@ with its own dense operand: the batch's TC blocks are cut into chunks
 (contiguous block ranges, cut inside a row window only where one is longer
 than a chunk), one CTA each, handed out by the hardware block scheduler.
 The pieces of cut windows go to the workspace and a small kernel adds them
-(queue=False leaves that workspace out: the CTA of a window's first piece runs
-its other pieces too; the bits are the same). Both launches can be captured in
+(queue=False leaves that workspace out: clusters of CTAs add their pieces up in
+shared memory; the bits are the same). Both launches can be captured in
 a CUDA graph and replayed.
 
 There is no counterpart in the reference, which multiplies one matrix per

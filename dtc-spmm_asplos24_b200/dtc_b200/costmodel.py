@@ -9,17 +9,20 @@ The reference fixes its schedule by hand per dataset and N
 with TC blocks of 16 x 8, 32 x 8 or 16 x 16 (window height x compaction width;
 the reference's blockSize_h x blockSize_w), mode 0 (window-scheduled) or 1
 (strict balance), waves in {1,2,4,8,16,32,64} in window mode and {1,2,4,8,16}
-in balance mode (chunks = waves x SMs, so the split threshold is ceil(T /
-chunks) blocks), N-tiles per CTA in {1,2,4}, two B forms within 1e-5
+in balance mode, N-tiles per CTA in {1,2,4}, two B forms within 1e-5
 relative error (SPLIT24, 3 bytes per element rebuilt on chip, and BF16X2, 4
 bytes per element used as stored; both with 3-term products) and TCA reorder off or
 on. The network predicts, for every class, log(t_class / t_best) of the SpMM
 kernel; it is trained on timings the library measures itself on seeded
 synthetic matrices (``collect``), entirely with the library's own CUDA kernels
 (forward, backward, Adam). The model changes only which schedule runs: every
-class computes the same product within its form's error bound. The exhaustive
-autotuner (``tune.autotune`` over every class) is its fallback and the
-reference point of its regret.
+class computes the same product within its form's error bound.
+
+The committed dataset and weights are of kernels for which mode, waves and
+N-tiles were launches of their own. The present kernels cut their chunks
+themselves, so that the classes are twelve launches (block shape, B form, reorder):
+the network orders them for a plan without measurement, and
+``plan(verify_top=K)`` times each of the twelve once, which is the exhaustive choice.
 """
 import ctypes as C
 import math
@@ -414,8 +417,7 @@ class Plan:
 
 class Scheduler:
     """Picks a class for (matrix, N): the trained model when its weights are
-    present and match the class space, else the exhaustive autotuner over every
-    class."""
+    present and match the class space, else the fastest launch."""
 
     def __init__(self, weights=WEIGHTS_PATH, device="cuda"):
         self.net = MLP.load(weights, device) if weights and os.path.exists(weights) else None

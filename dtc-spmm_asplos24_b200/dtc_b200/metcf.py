@@ -154,8 +154,8 @@ def pack_b_into(B: torch.Tensor, fmt: int, planes):
 
 def spmm_ex_workspace_bytes(m: METCF, N, mode=0, grid=0):
     """Workspace bytes of spmm_ex for this schedule: the partial tiles of balance
-    mode (required) and a slot per chunk after them (optional: without them fewer
-    CTAs share a row window of many blocks)."""
+    mode (required) and a slot per chunk after them (optional: without them
+    clusters of CTAs add up the pieces of a row window of many blocks)."""
     wsb = C.c_size_t()
     call("dtc_spmm_ex_workspace_bytes", m.M, m.T, N, m.H, mode, grid, C.byref(wsb))
     return wsb.value

@@ -1,12 +1,11 @@
-"""Schedule autotuning over the C ABI's exhaustive tuner (dtc_autotune).
+"""Schedule autotuning over the C ABI's tuner (dtc_autotune).
 
 The reference chooses balance / vector width / N split from a fixed table
-per dataset (scripts/DTCSpMM/run_DTC_SpMM.py:10-30). Here every schedule the
-kernels support is timed on the caller's own ME-TCF and B (``autotune``), and
-``tune_forms`` extends the search over the B storage forms that meet an error
-budget. A schedule changes neither the B form nor the product precision:
-schedules of one form differ only in how fp32 partial sums are grouped (all
-within the form's error bound), and each schedule is bitwise reproducible.
+per dataset (scripts/DTCSpMM/run_DTC_SpMM.py:10-30). Here the product is timed
+on the caller's own ME-TCF and B (``autotune``: with its workspace all schedules
+of a form are one launch), and ``tune_forms`` searches over the B storage forms
+that meet an error budget. A schedule changes neither the B form nor the product
+precision, and each is bitwise reproducible.
 """
 import ctypes as C
 from dataclasses import dataclass
@@ -33,7 +32,7 @@ FORMS = {
 
 
 def candidates(N, H=16, split=False):
-    """Every (mode, waves, ntile) schedule the kernels support for width N at
+    """Every (mode, waves, ntile) schedule that a call can name for width N at
     window height H (split: the split-precision kernels)."""
     L = _lib.lib()
     n = L.dtc_schedule_candidates_ex(N, H, 1 if split else 0, None, 0)
@@ -50,7 +49,7 @@ def workspace_for(m: METCF, N, device):
 
 def autotune(m: METCF, planes, fmt, N, precision, reps=3, use_values=True, out=None,
              workspace=None):
-    """Times every candidate schedule; returns (list of measured Schedules, best)."""
+    """Times the product; returns (list of Schedules with their time, best)."""
     dev = planes[0].device
     C_ = out if out is not None else torch.empty((m.M, N), dtype=torch.float32, device=dev)
     ws = workspace if workspace is not None else workspace_for(m, N, dev)
@@ -85,10 +84,9 @@ def eligible_forms(max_rel_err):
 
 
 def tune_forms(m: METCF, B: torch.Tensor, max_rel_err=1e-5, reps=3, forms=None):
-    """Exhaustive search over (form within the error budget) x schedule.
+    """Search over the forms within the error budget.
 
-    Returns (best Choice, {form: [measured Schedules]}) -- the table the
-    learned cost model is trained on and evaluated against.
+    Returns (best Choice, {form: [measured Schedules]}).
     """
     N = B.shape[1]
     forms = forms if forms is not None else eligible_forms(max_rel_err)

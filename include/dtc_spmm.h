@@ -12,9 +12,10 @@
  *
  * Workspaces of the SpMM entry points hold pieces of row windows that are cut
  * between CTAs: the partial tiles of strict balance (required) and, after them,
- * a slot for every chunk of TC blocks (optional: without it fewer CTAs share a
- * window of many blocks). The *_workspace_bytes queries return the size with
- * both (workspace base 256-byte aligned).
+ * a slot for every chunk of TC blocks (optional, at most 16384 of them). Without
+ * slots clusters of CTAs add the pieces up in shared memory: the same bits, up to
+ * two thirds slower on matrices with windows of many blocks. The *_workspace_bytes
+ * queries return the size with both. The base needs 4-byte alignment.
  *
  * Each entry point names the reference interface it replaces (paths relative
  * to the reference project root, HPMLL/DTC-SpMM_ASPLOS24).
@@ -203,8 +204,8 @@ dtc_status dtc_pack_b(int fmt, const float* d_B, int64_t rows, int32_t N, void* 
 
 /* Window-scheduled SpMM. Replaces run_DTCSpMM / spmm_forward_ptx_uint8_improved
  * (DTC-SpMM/DTCSpMM.cpp:117-131 -> DTCSpMM_kernel.cu:811-944) and DTCSpMM_gcn
- * (DTCSpMM.cpp:147-161 -> DTCSpMM_kernel.cu:1033-1116): one launch, each row
- * window is owned by one CTA, no workspace. d_tcValues == NULL reproduces the
+ * (DTCSpMM.cpp:147-161 -> DTCSpMM_kernel.cu:1033-1116): one launch, no
+ * workspace (see the top of this header). d_tcValues == NULL reproduces the
  * reference's implicit A = 1 (DTCSpMM_kernel.cu:837-838). C rows of empty
  * windows are written as zeros (the reference zero-fills, :823). */
 dtc_status dtc_spmm(const int32_t* d_rowWindowOffset, const uint8_t* d_tileId,
@@ -213,8 +214,7 @@ dtc_status dtc_spmm(const int32_t* d_rowWindowOffset, const uint8_t* d_tileId,
                     int64_t num_blocks, const float* d_B, int32_t N, float* d_C,
                     dtc_stream_t stream);
 
-/* dtc_spmm with a workspace: a window of more blocks than one CTA's share is
- * then multiplied by several CTAs (same bits as without). Any N. */
+/* dtc_spmm with a workspace of slots (same bits as without). Any N. */
 dtc_status dtc_spmm_workspace_bytes(int32_t num_nodes, int64_t num_blocks, int32_t N,
                                     size_t* bytes);
 dtc_status dtc_spmm_ws(const int32_t* d_rowWindowOffset, const uint8_t* d_tileId,
@@ -225,11 +225,13 @@ dtc_status dtc_spmm_ws(const int32_t* d_rowWindowOffset, const uint8_t* d_tileId
 
 /* Strict-balance SpMM. Replaces run_DTCSpMM_balance /
  * spmm_balance_forward_ptx_uint8_prefetch (DTC-SpMM/DTCSpMM.cpp:163-178 ->
- * DTCSpMM_kernel.cu:1118-1199, kernels :4730-4901, :5085-5362). Every CTA gets
- * an equal contiguous range of TC blocks (windows split across CTAs); partial
- * tiles go to the workspace and are reduced in fixed CTA order by a second
- * kernel, so results are bitwise reproducible (the reference uses fp32
- * atomicAdd). Needs only d_tcblockRowid, like the reference. */
+ * DTCSpMM_kernel.cu:1118-1199, kernels :4730-4901, :5085-5362). The TC blocks
+ * are cut into contiguous chunks, inside a row window where one has more blocks
+ * than a chunk; the pieces of cut windows go to the workspace and are added in
+ * chunk order by a second kernel, so results are bitwise reproducible (the
+ * reference uses fp32 atomicAdd). Needs only d_tcblockRowid, like the
+ * reference. Window ids that are out of range or descend set bit 1 of
+ * dtc_device_status; C then has no meaning. */
 dtc_status dtc_spmm_balance_workspace_bytes(int32_t num_nodes, int64_t num_blocks, int32_t N,
                                             size_t* bytes);
 dtc_status dtc_spmm_balance(const int32_t* d_tcblockRowid, const uint8_t* d_tileId,
@@ -245,8 +247,9 @@ dtc_status dtc_spmm_balance(const int32_t* d_tcblockRowid, const uint8_t* d_tile
  * partial tiles live in a fixed 16 MiB array compiled into the library, held
  * in the memory of every GPU that loads it until the process exits.
  * Limit: 4*(ceil(num_nodes/16)+1) bytes (rounded up to 256) + 128*N bytes per
- * SM (one CTA per SM) must fit in dtc_noalloc_scratch_capacity() bytes; larger
- * problems get DTC_ERR_WORKSPACE_TOO_SMALL. The first call on a device looks
+ * SM must fit in dtc_noalloc_scratch_capacity() bytes; larger problems get
+ * DTC_ERR_WORKSPACE_TOO_SMALL (widths that are no multiple of 4 do without the
+ * tiles instead). The first call on a device looks
  * up the array's device address with that device current -- make it before
  * any stream capture. All calls share the array: calls that overlap on the
  * GPU race and must be serialised by the caller. Same results semantics as
@@ -267,9 +270,9 @@ size_t dtc_noalloc_scratch_capacity(void);
  * range that the required workspace has partial tiles for (0 = 16 per SM); the
  * kernels cut the range themselves, into fewer chunks than they would like only
  * where the workspace has fewer slots. ntile is checked and has no effect (the
- * kernels pick their feature slices). d_rowWindowOffset is required (build it from TCblockRowid with
- * dtc_rowid_to_window_offset). Workspace: required in mode 1 (partial tiles),
- * optional slots after it (see the top of this header). */
+ * kernels pick their feature slices). d_rowWindowOffset is required (build it
+ * from TCblockRowid with dtc_rowid_to_window_offset). Workspace: required in
+ * mode 1 (partial tiles), optional slots after it (see the top of this header). */
 dtc_status dtc_spmm_ex(const int32_t* d_rowWindowOffset, const uint8_t* d_tileId,
                        const int32_t* d_tcblockOffset, const int32_t* d_sparseAToX,
                        const float* d_tcValues, int32_t num_nodes, int32_t num_windows,
@@ -299,18 +302,17 @@ dtc_status dtc_spmm_fused(const int32_t* d_rowWindowOffset, const uint8_t* d_til
 /* N split chosen per dataset and N) by measurement on the caller's data.     */
 /* ------------------------------------------------------------------------- */
 typedef struct {
-  int32_t mode;   /* 0 = window-scheduled (no window split), 1 = strict balance */
-  int32_t waves;  /* chunks = waves x SMs, capped at T: the split threshold is  */
-                  /* ceil(T / chunks) TC blocks (one CTA per SM pulls chunks)  */
+  int32_t mode;   /* 0 = window-scheduled, 1 = strict balance                   */
+  int32_t waves;  /* grid = waves x SMs, capped at T                            */
   int32_t ntile;  /* 128-feature tiles per CTA (1, 2 or 4)                      */
-  int32_t grid;   /* chunk count the measurement used (output)                  */
+  int32_t grid;   /* partial tiles of mode 1's workspace (output)               */
   float ms;       /* mean kernel time over the timed repetitions (output)       */
 } dtc_schedule;
 
-/* Fills out[0..min(count, max_out)) with every schedule the kernels support for
+/* Fills out[0..min(count, max_out)) with every schedule that a call can name for
  * N and returns the count (out may be NULL to query it): waves 1, 2, 4, 8, 16,
- * 32 and 64 in window mode, 1 to 16 in balance mode (whose cut windows keep
- * partial tiles per chunk), times the N-tiles the kernels hold for N. */
+ * 32 and 64 in window mode, 1 to 16 in balance mode, times the N-tiles. With a
+ * workspace of all slots they are one launch. */
 int dtc_schedule_candidates(int32_t N, dtc_schedule* out, int max_out);
 /* The same for a given window height and kernel family (split = 1 for the
  * split-precision forms, whose N-tiles per CTA are capped at 2 at height 32). */
@@ -321,12 +323,12 @@ int dtc_schedule_candidates_ex(int32_t N, int32_t block_h, int split, dtc_schedu
 dtc_status dtc_autotune_workspace_bytes(int32_t num_nodes, int64_t num_blocks, int32_t N,
                                         int32_t block_h, size_t* bytes);
 
-/* Times every candidate (one untimed run + `reps` runs between CUDA events on
- * `stream`; synchronises it; split forms at block width 16 skip N-tile counts
- * above 2, which those kernels cap) on the given ME-TCF arrays and B form, writes the
- * measured schedules to results[0..max_results), their count to *num_results
- * and the index of the fastest to *best. d_C receives the last candidate's
- * product. Arguments as in dtc_spmm_ex. */
+/* Times the product (one untimed run + `reps` runs between CUDA events on
+ * `stream`; synchronises it) on the given ME-TCF arrays and B form and writes
+ * every candidate with that time to results[0..max_results) (split forms at
+ * block width 16 without N-tile counts above 2), their count to *num_results and
+ * the index of the fastest, the first one, to *best. d_C receives the product.
+ * Arguments as in dtc_spmm_ex. */
 dtc_status dtc_autotune(const int32_t* d_rowWindowOffset, const uint8_t* d_tileId,
                         const int32_t* d_tcblockOffset, const int32_t* d_sparseAToX,
                         const float* d_tcValues, int32_t num_nodes, int32_t num_windows,
@@ -395,7 +397,7 @@ dtc_status dtc_mlp_argmin(const float* d_Y, const uint8_t* d_feasible, int feasi
  * writes, for each of its CTAs c < capacity (c = blockIdx.x + gridDim.x *
  * blockIdx.y), four uint64 values to d_records[4c .. 4c+3]: the %globaltimer
  * (ns) at kernel entry and at exit, the SM id, and the number of TC-block
- * chunks the CTA processed. capacity = 0 turns it off. No reference
+ * chunks the CTA processed (1). capacity = 0 turns it off. No reference
  * counterpart (the reference's per-SM clock kernels,
  * DTC-SpMM/DTCSpMM_kernel.cu:62-79, are a separate instrumented build). */
 dtc_status dtc_set_cta_timer(uint64_t* d_records, int32_t capacity);
