@@ -40,11 +40,11 @@ namespace {
 
 constexpr int kGroup = 128;              // threads of a CTA: four windows, or one middle window
 constexpr int kWarpFill = 1024;          // windows up to here: places by one warp
-constexpr int kLeftBytes = kWarpFill * 5;  // of a warp that sorts such a window: keys, tile ids
+constexpr int kLeftBytes = kWarpFill * 5;  // a warp that sorts such a window: keys, tile ids
 constexpr int kThreads = 1024;           // threads of a large window
 constexpr int kSweepCols = 1 << 20;      // columns per sweep of a large window's bitmap
 constexpr int kSortBits = 14, kSortEdges = 1 << kSortBits;  // edges that a large CTA sorts
-constexpr int kMergeWarps = 16;          // of a large CTA that merge
+constexpr int kMergeWarps = 16;          // warps of it that merge repeated entries
 constexpr int kPartBlocks = 8192;        // blocks of a part of a huge window, at most
 constexpr int kPartSort = 8192, kPartEdges = 6144;  // edges of a part: sorted at a time, on average
 constexpr int kMaxH = 256;               // rows of a window (block_h * block_w <= 256)
@@ -171,12 +171,15 @@ __global__ void k_mixed(const Csr a, const int32_t* __restrict__ e2c,
     r[v] = in ? __ldg(e2r + e - 1) : 0;
     q[v] = in ? __ldg(e2r + e) : 1;
   }
+  bool found = false;
 #pragma unroll
   for (int v = 0; v < 8; ++v)
     if (c[v] >= d[v] && r[v] == q[v]) {
       mixed[q[v] / a.H] = 1;
-      *any = 1;
+      found = true;
     }
+  // (a store per CTA: one per edge waits for the word in L2)
+  if (__syncthreads_or(found) && threadIdx.x == 0) *any = 1;
 }
 
 // ------------------------------------------------------------- group helpers
@@ -1593,7 +1596,7 @@ Layout layout(int32_t M, int64_t nnz, int32_t H) {
   return L;
 }
 
-static_assert(kHuge <= kSortEdges, "fill_sorted takes every window that is not huge");
+static_assert(kHuge <= kSortEdges, "fill_cta takes every window that is not huge");
 constexpr int kSortBytes =
     kSortEdges * 9 + std::max(kHist * 4 + 256 + kSortEdges, kMergeWarps * (int)sizeof(MergeScratch));
 static_assert(kThreads / 32 * (int)sizeof(MergeScratch) <= kPartSort * 12 && kPartSort <= kSortEdges &&
@@ -1613,7 +1616,6 @@ int windows_per_cta(int32_t nwin) {
   const int64_t p = nwin / (8 * (int64_t)num_sms());
   return p < 4 ? 4 : p > kPer ? kPer : (int)p;
 }
-static_assert(kPer <= 32, "a bit per window");
 
 template <typename K>
 dtc_status count_impl(const Csr& a, char* ws, const Layout& L, int32_t* e2c, int32_t* e2r,
@@ -1653,11 +1655,14 @@ dtc_status count_impl(const Csr& a, char* ws, const Layout& L, int32_t* e2c, int
 __global__ void k_tall_keys(const Csr a, const Fill f, uint32_t* __restrict__ key,
                             int32_t* __restrict__ edge, int32_t* any) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= a.nnz) return;
-  const int32_t rk = __ldg(f.e2c + e);
-  key[e] = (uint32_t)(__ldg(f.rwo + __ldg(f.e2r + e) / a.H) + a.block(rk));
-  edge[e] = (int32_t)e;
-  if (repeats(f, 0, (int32_t)e, rk)) *any = 1;
+  bool found = false;
+  if (e < a.nnz) {
+    const int32_t rk = __ldg(f.e2c + e);
+    key[e] = (uint32_t)(__ldg(f.rwo + __ldg(f.e2r + e) / a.H) + a.block(rk));
+    edge[e] = (int32_t)e;
+    found = repeats(f, 0, (int32_t)e, rk);
+  }
+  if (__syncthreads_or(found) && threadIdx.x == 0) *any = 1;
 }
 __global__ void k_tall_emit(const Csr a, const Fill f, const uint32_t* __restrict__ key,
                             const int32_t* __restrict__ edge) {
