@@ -86,12 +86,21 @@ class BatchedSpMM:
         self.m = _m.convert(rowptr, col, self.layout.total_rows, values=val, device=self.device)
         self.B = torch.zeros((self.layout.total_rows, N), dtype=torch.float32, device=self.device)
         self.C = torch.empty((self.layout.total_rows, N), dtype=torch.float32, device=self.device)
-        self._parts = [self.B[int(o):int(o) + int(r)]  # each matrix's rows of the operand
-                       for o, r in zip(self.layout.offsets, self.layout.rows)]
         self.planes = None
         self.queue = queue
         self._alloc_ws()
         self.graph: Optional[torch.cuda.CUDAGraph] = None
+
+    @property
+    def B(self):
+        """The stacked operand; another tensor may be put in its place."""
+        return self._B
+
+    @B.setter
+    def B(self, B):
+        self._B = B
+        self._parts = [B[int(o):int(o) + int(r)]  # each matrix's rows of it
+                       for o, r in zip(self.layout.offsets, self.layout.rows)]
 
     def _alloc_ws(self):
         """Workspace of the current schedule: partial tiles (balance mode) and,

@@ -34,3 +34,20 @@ def test_load_forms(cuda, form):
     with torch.no_grad():
         plan.load(b for b in Bs)
     np.testing.assert_array_equal(plan.B.detach().cpu().numpy(), want.cpu().numpy())
+
+
+def test_load_fills_the_operand_that_the_plan_has(cuda):
+    """A caller may put another tensor in place of the stacked operand."""
+    import torch
+    from dtc_b200 import gen
+    from dtc_b200.batched import BatchedSpMM
+    mats = [gen.uniform(n, mean=4.0, seed=n) for n in (33, 70, 16)]
+    plan = BatchedSpMM(mats, 32)
+    Bs = [torch.randn(m.M, 32, device="cuda") for m in mats]
+    plan.load(Bs)
+    old, want = plan.B, plan.B.clone()
+    C = plan.run().clone()
+    plan.B = torch.zeros_like(old)
+    old.fill_(float("nan"))
+    plan.load(Bs)
+    assert torch.equal(plan.B, want) and torch.equal(plan.run(), C)
